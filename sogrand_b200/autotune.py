@@ -3,9 +3,9 @@
 Every variant of the plain decoder computes bit-identical results; they
 differ only in speed, which depends on the codeword mix.  The dimensions:
 warps per codeword CTA (8 to 16); the channel cube in shared memory (staged
-by a bulk copy) or read from global memory; error patterns per lane per step
-(G = 1, 2 or 4); lines per warp (1: 32 lanes per line; 2: 16 lanes per
-line, the "-l2-" variants).  autotune() decodes one seeded batch of
+by a bulk copy) or read from global memory; lines per warp (1: 32 lanes per
+line; 2: 16 lanes per line and 2 or 4 patterns per lane, the "-l2-"
+variants).  One-line variants with and without "-g2" are the same kernel.  autotune() decodes one seeded batch of
 the caller's workload with each variant, timed with CUDA events, and selects
 the fastest for the process.
 """

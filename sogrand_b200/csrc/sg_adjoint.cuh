@@ -38,7 +38,7 @@ __device__ __forceinline__ double sg_sum16(double v, int lane)
 
 /* Gradient with respect to the line input x (lanes 0..15) of g . L_APP,
  * g the upstream gradient of L_APP (lanes 0..15). */
-__device__ __forceinline__ double sg_line_vjp(double x, double g, const SgAdjOut& a, const double* etab, int lane)
+__device__ __forceinline__ double sg_line_vjp(double x, double g, const SgAdjOut& a, SgTab etab, int lane)
 {
     const bool act = lane < 16;
     if (a.curl == 0)
@@ -105,13 +105,16 @@ struct SgBackwardArgs {
     int32_t loss_mode;           /* 0: BCE of the final APP; 1: summed over all phases' APPs */
     double thres;
     double alpha[SG_MAX_PHASES];
+    SgK k; /* constants of exp and log */
+    sg_order_meta meta;
 };
 
 template <int NW>
 struct SgBackSmem {
     double gle[SG_CUBE]; /* d loss / d L_E of the phase being processed */
-    alignas(16) double etab[SG_EXP_TAB_LEN];
+    SgEtab<false> etab;
     alignas(16) double ltab[SG_LOG_TAB_LEN];
+    SgExpK ek;
     SgWarpScratch ws[NW];
     double ga;   /* d loss / d alpha of the phase */
     double lsum; /* loss of the codeword */
@@ -124,14 +127,17 @@ __global__ void __launch_bounds__(NW * 32, 3) sg_backward_kernel(const __grid_co
     constexpr int NT = NW * 32;
     SgBackSmem<NW>& S = *reinterpret_cast<SgBackSmem<NW>*>(sg_smem_raw);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    for (int i = tid; i < SG_EXP_TAB_LEN; i += NT)
-        S.etab[i] = g_etab[i];
+    sg_etab_fill<false, false>(S.etab, g_etab, tid, NT);
     for (int i = tid; i < SG_LOG_TAB_LEN; i += NT)
         S.ltab[i] = g_ltab[i];
     SgLineParams lp;
     lp.L = args.L;
-    lp.tmax = 0xffffffffu;
+    lp.meta = &args.meta;
+    lp.ek = &S.ek;
+    if (tid == 0)
+        S.ek = sg_exp_k();
     lp.thres = args.thres;
+    const SgTab etab = sg_etab_of<false, false>(S.etab, args.k.v), ltab{S.ltab, args.k.v};
     __syncthreads();
     for (unsigned long long cw = blockIdx.x; cw < args.n_cw; cw += gridDim.x) {
         const int P = args.stats[cw].phases;
@@ -166,7 +172,7 @@ __global__ void __launch_bounds__(NW * 32, 3) sg_backward_kernel(const __grid_co
                 const double lep = lane < 16 ? ck[pos] : 0.0;
                 const double x = lane < 16 ? __dadd_rn(g[pos], __dmul_rn(alpha, lep)) : 1.0;
                 SgAdjOut a;
-                const SgLineResult r = sg_decode_line<1, true>(x, lp, args.enum_tabs, S.etab, S.ltab, &S.ws[warp], &a);
+                const SgLineResult r = sg_decode_line<true, false, false>(x, lp, args.enum_tabs, etab, ltab, &S.ws[warp], &a);
                 const double gE = lane < 16 ? S.gle[pos] : 0.0;
                 double gL = 0.0, lossv = 0.0;
                 const bool scored = p == P - 1 || args.loss_mode == 1;
@@ -176,7 +182,7 @@ __global__ void __launch_bounds__(NW * 32, 3) sg_backward_kernel(const __grid_co
                     lossv = z > 0.0 ? z + log1p(exp(-z)) : log1p(exp(z)); /* softplus */
                     gL = s / (1.0 + exp(-z));                              /* s * sigmoid(z) */
                 }
-                const double gx = sg_line_vjp(x, gL + gE, a, S.etab, lane) - gE;
+                const double gx = sg_line_vjp(x, gL + gE, a, etab, lane) - gE;
                 if (lane < 16) {
                     S.gle[pos] = alpha * gx;
                     if (args.grad_llr)

@@ -1,17 +1,7 @@
-/* sg_api.cu -- B200 SOGRAND cubic decoder: kernels and C ABI.
- *
- * Kernels
- *   sg_decode_kernel   the whole iterative decode of a codeword per CTA
- *                      (SOGRAND_C/cubic_decoder_final.c:119-289): the 32 KB
- *                      channel cube arrives in shared memory by one bulk
- *                      asynchronous copy (cp.async.bulk, completion on an
- *                      mbarrier) and stays there with the 32 KB extrinsic
- *                      cube for all iterations; 8 warps take the 256 lines
- *                      of a phase from a shared counter and decode one line
- *                      each (sg_line.cuh); after every phase one warp runs the
- *                      early-termination test on the 256 hard-decision words.
- *   sg_bitso_kernel    SOGRAND_bitSO on independent lines, one warp per line.
- *   sg_gen_kernel      seeded source + encoder + AWGN channel (sg_gen.h).
+/* sg_api.cu -- B200 SOGRAND cubic decoder: C ABI, and the kernels of the
+ * table-driven math (sg_kernels.cuh; sg_cr.cu holds the correctly rounded
+ * ones), the generator (sg_gen_kernel: seeded source, encoder, AWGN channel)
+ * and the adjoint.
  *
  * Built with -fmad=false: no floating-point contraction anywhere, as in the
  * reference's plain gcc build; the exp/log routines use explicit FMAs.
@@ -25,6 +15,7 @@
 #include <stdlib.h>
 #include <string.h>
 
+#include <algorithm>
 #include <atomic>
 #include <chrono>
 #include <condition_variable>
@@ -35,403 +26,19 @@
 #include <vector>
 
 #include "../../include/sogrand_b200.h"
-#include "sg_code.h"
-#include "sg_enum.h"
+#include "sg_cr.h"
 #include "sg_gen.h"
-#include "sg_line.cuh"
-#include "sg_line16.cuh"
-#include "sg_math.h"
-
-#define SG_THREADS 256
-#define SG_WARPS (SG_THREADS / 32)
-/* Bounded device-side waits.  The limit of a wait that can give up (the
- * bulk-copy wait here, the persistent decoder's idle rounds) is a launch
- * argument, SG_WAIT_LIMIT_DEFAULT unless sg_set_wait_limit() changed it.
- * After a bulk-copy wait gave up, the copy may still be writing into the
- * CTA's shared memory: the CTA waits for it again, up to SG_DRAIN_LIMIT
- * polls, before it releases that memory. */
-#define SG_WAIT_LIMIT_DEFAULT (1ll << 22)
-#define SG_DRAIN_LIMIT (1ll << 26)
-
-__device__ const double g_etab[SG_EXP_TAB_LEN] = SG_EXP_TAB_INIT;
-__device__ const double g_ltab[SG_LOG_TAB_LEN] = SG_LOG_TAB_INIT;
-
-/* ------------------------------------------------------------ device -- */
-
-struct SgDecodeArgs {
-    const double* llr;
-    uint8_t* bits;
-    double* lapp;
-    sg_cw_stats* stats;
-    const uint32_t* enum_tabs;
-    unsigned int* err;
-    double* ckpt; /* nullable: [n_cw][3*imax][4096], L_E entering each phase */
-    unsigned long long n_cw;
-    long long wait_limit; /* polls or idle rounds before a bounded wait gives up */
-    int32_t L;
-    int32_t imax;
-    uint32_t tmax;
-    int32_t use_bulk;
-    double thres;
-    double alpha[SG_MAX_PHASES];
-};
-
-/* Poll the mbarrier for phase `parity` at most `limit` times; 1 when it
- * completed. */
-__device__ __forceinline__ uint32_t sg_mbar_wait(uint32_t mbar, uint32_t parity, long long limit)
-{
-    uint32_t ok = 0;
-    for (long long it = 0; it < limit && !ok; it++) {
-        asm volatile(
-            "{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
-            : "=r"(ok)
-            : "r"(mbar), "r"(parity)
-            : "memory");
-    }
-    return ok;
-}
-
-/* Outputs of a codeword that is not decoded: zero bits and statistics with
- * the given converged code (-1 non-finite input, -2 a wait gave up).
- * Called by the whole CTA. */
-__device__ __forceinline__ void sg_cw_not_decoded(const SgDecodeArgs& args, unsigned long long cw, int code)
-{
-    if (threadIdx.x < SG_INFO_BYTES)
-        args.bits[cw * SG_INFO_BYTES + threadIdx.x] = 0;
-    if (threadIdx.x == 0 && args.stats) {
-        sg_cw_stats st;
-        st.iterations = 0;
-        st.ng = 0;
-        st.ng_p = 0;
-        st.converged = code;
-        st.phases = 0;
-        args.stats[cw] = st;
-    }
-}
-
-/* Shared memory of a decode CTA.  With LCH_SMEM the channel cube is staged
- * here by one bulk copy; otherwise each line reads its 16 channel LLRs from
- * global memory (L2-resident) once per phase. */
-template <int NW, bool LCH_SMEM, int LPW = 1> /* LPW: lines decoded per warp at a time */
-struct SgCwSmem {
-    alignas(16) double lch[LCH_SMEM ? SG_CUBE : 2]; /* bulk-copy destination */
-    double le[SG_CUBE];
-    alignas(16) double etab[SG_EXP_TAB_LEN]; /* read as double2 by the exp routines */
-    alignas(16) double ltab[SG_LOG_TAB_LEN];
-    SgWarpScratch ws[NW * LPW];
-    uint16_t hdw[256];
-    unsigned long long mbar;
-    unsigned long long ng;
-    unsigned int ngmax;
-    int line_next;
-    int conv;
-    int bad;
-};
-
-/* Cube index of bit `i` of line `l` in phase `axis` (lines of the reference's
- * column phase run along the stride-1 index, rows along stride 16, slices
- * along stride 256; cubic_decoder_final.c:157-247). */
-__device__ __forceinline__ int sg_pos(int axis, int l, int i)
-{
-    const int a = l >> 4, b = l & 15;
-    if (axis == 0)
-        return a * 256 + b * 16 + i;
-    if (axis == 1)
-        return a * 256 + i * 16 + b;
-    return i * 256 + a * 16 + b;
-}
-
-/* Early termination (cubic_decoder_final.c:317-391) on the 256 line words
- * of the phase just run: the hard decisions form a product codeword iff
- * every word is a component codeword and the words satisfy the component
- * parity equations along both other axes (bitwise).  Warp-wide. */
-__device__ __forceinline__ bool sg_is_codeword(const uint16_t* hdw, int lane)
-{
-    bool bad = false;
-    for (int q = lane; q < 256; q += 32) {
-        const uint32_t x = hdw[q];
-        bad |= ((x >> 8) & 0xffu) != c_ptab[x & 0xffu];
-    }
-    for (int q = lane; q < 128; q += 32) {
-        const int a = q >> 3, j = q & 7;
-        uint32_t acc = 0;
-#pragma unroll
-        for (int b = 0; b < 8; b++)
-            if ((c_prow[b] >> j) & 1u)
-                acc ^= hdw[a * 16 + b];
-        bad |= acc != hdw[a * 16 + 8 + j];
-    }
-    for (int q = lane; q < 128; q += 32) {
-        const int b = q >> 3, j = q & 7;
-        uint32_t acc = 0;
-#pragma unroll
-        for (int a = 0; a < 8; a++)
-            if ((c_prow[a] >> j) & 1u)
-                acc ^= hdw[a * 16 + b];
-        bad |= acc != hdw[(8 + j) * 16 + b];
-    }
-    return !__any_sync(SG_FULL, bad);
-}
-
-__device__ __forceinline__ uint32_t sg_smem_u32(const void* p)
-{
-    return (uint32_t)__cvta_generic_to_shared(p);
-}
-
-extern __shared__ __align__(128) unsigned char sg_smem_raw[];
-
-template <int NW, bool LCH_SMEM, int MINB, int G, bool CR, int LPW = 1>
-__global__ void __launch_bounds__(NW * 32, MINB) sg_decode_kernel(const __grid_constant__ SgDecodeArgs args)
-{
-    constexpr int NT = NW * 32;
-    SgCwSmem<NW, LCH_SMEM, LPW>& S = *reinterpret_cast<SgCwSmem<NW, LCH_SMEM, LPW>*>(sg_smem_raw);
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const bool use_bulk = LCH_SMEM && args.use_bulk;
-    for (int i = tid; i < SG_EXP_TAB_LEN; i += NT)
-        S.etab[i] = g_etab[i];
-    for (int i = tid; i < SG_LOG_TAB_LEN; i += NT)
-        S.ltab[i] = g_ltab[i];
-    const uint32_t mbar = sg_smem_u32(&S.mbar);
-    if (tid == 0 && use_bulk) {
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(mbar) : "memory");
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    __syncthreads();
-    uint32_t phase_bit = 0;
-    SgLineParams lp;
-    lp.L = args.L;
-    lp.tmax = args.tmax;
-    lp.thres = args.thres;
-
-    for (unsigned long long cw = blockIdx.x; cw < args.n_cw; cw += gridDim.x) {
-        const double* g = args.llr + cw * SG_CUBE;
-        if (use_bulk) {
-            if (tid == 0) {
-                /* order earlier generic-proxy reads of lch before the async write */
-                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(mbar),
-                             "r"((uint32_t)(SG_CUBE * 8))
-                             : "memory");
-                asm volatile(
-                    "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                        sg_smem_u32(S.lch)),
-                    "l"(g), "r"((uint32_t)(SG_CUBE * 8)), "r"(mbar)
-                    : "memory");
-            }
-        } else if (LCH_SMEM) {
-            for (int i = tid; i < SG_CUBE; i += NT)
-                S.lch[i] = g[i];
-        }
-        for (int i = tid; i < SG_CUBE; i += NT)
-            S.le[i] = 0.0;
-        if (tid == 0) {
-            S.ng = 0;
-            S.conv = 0;
-            S.bad = 0;
-        }
-        if (use_bulk && tid == 0) {
-            if (!sg_mbar_wait(mbar, phase_bit, args.wait_limit)) {
-                /* gave up: report it, then let the copy land before this
-                 * CTA's shared memory is reused or released */
-                atomicOr(args.err, 1u);
-                if (!sg_mbar_wait(mbar, phase_bit, SG_DRAIN_LIMIT))
-                    atomicOr(args.err, 2u);
-                S.bad = 2;
-            }
-        }
-        phase_bit ^= 1u;
-        __syncthreads();
-        if (S.bad == 2) {
-            /* this codeword and the CTA's later ones are reported as not
-             * decoded (converged = -2) */
-            for (unsigned long long c = cw; c < args.n_cw; c += gridDim.x)
-                sg_cw_not_decoded(args, c, -2);
-            return;
-        }
-        bool nonfinite = false;
-        for (int i = tid; i < SG_CUBE; i += NT)
-            nonfinite |= !isfinite(LCH_SMEM ? S.lch[i] : __ldg(g + i));
-        if (__syncthreads_or(nonfinite)) {
-            sg_cw_not_decoded(args, cw, -1);
-            __syncthreads();
-            continue;
-        }
-
-        int phases = 0;
-        unsigned long long ng_p = 0;
-        int axis_last = 0;
-        bool conv = false;
-        for (int iter = 1; iter <= args.imax && !conv; iter++) {
-            for (int axis = 0; axis < 3 && !conv; axis++) {
-                const double alpha = args.alpha[3 * (iter - 1) + axis];
-                if (tid == 0) {
-                    S.line_next = 0;
-                    S.ngmax = 0;
-                }
-                __syncthreads();
-                if constexpr (LPW == 2) {
-                    /* the warp takes two lines at a time, one per half, and
-                     * decodes them in lockstep (sg_line16.cuh) */
-                    const int hb = lane & 16, sl = lane & 15;
-                    SgWarpScratch* wsl = &S.ws[2 * warp + (hb >> 4)];
-                    for (;;) {
-                        int l = 0;
-                        if (lane == 0)
-                            l = atomicAdd(&S.line_next, 2);
-                        l = __shfl_sync(SG_FULL, l, 0) + (hb >> 4);
-                        if (l >= 256) /* 256 lines: both halves leave together */
-                            break;
-                        const int pos = sg_pos(axis, l, sl);
-                        const double le0 = S.le[pos];
-                        const double v = __dadd_rn(LCH_SMEM ? S.lch[pos] : __ldg(g + pos), __dmul_rn(alpha, le0));
-                        if (args.ckpt)
-                            args.ckpt[(cw * (3ull * args.imax) + 3 * (iter - 1) + axis) * SG_CUBE + pos] = le0;
-                        const SgLineResult r = sg_decode_line16<G, CR>(v, lp, args.enum_tabs, S.etab, S.ltab, wsl);
-                        S.le[pos] = r.le;
-                        if (args.lapp)
-                            args.lapp[cw * SG_CUBE + pos] = r.lapp;
-                        if (sl == 0) {
-                            S.hdw[l] = (uint16_t)r.hdword;
-                            atomicAdd(&S.ng, (unsigned long long)r.T);
-                            atomicMax(&S.ngmax, r.T);
-                        }
-                    }
-                } else {
-                    for (;;) {
-                        int l = 0;
-                        if (lane == 0)
-                            l = atomicAdd(&S.line_next, 1);
-                        l = __shfl_sync(SG_FULL, l, 0);
-                        if (l >= 256)
-                            break;
-                        const int pos = sg_pos(axis, l, lane & 15);
-                        double v = 1.0;
-                        if (lane < 16) { /* L_ch + (alpha*L_E) */
-                            v = __dadd_rn(LCH_SMEM ? S.lch[pos] : __ldg(g + pos), __dmul_rn(alpha, S.le[pos]));
-                            if (args.ckpt)
-                                args.ckpt[(cw * (3ull * args.imax) + 3 * (iter - 1) + axis) * SG_CUBE + pos] = S.le[pos];
-                        }
-                        const SgLineResult r =
-                            sg_decode_line<G, false, CR>(v, lp, args.enum_tabs, S.etab, S.ltab, &S.ws[warp]);
-                        if (lane < 16) {
-                            S.le[pos] = r.le;
-                            if (args.lapp)
-                                args.lapp[cw * SG_CUBE + pos] = r.lapp;
-                        }
-                        if (lane == 0) {
-                            S.hdw[l] = (uint16_t)r.hdword;
-                            atomicAdd(&S.ng, (unsigned long long)r.T);
-                            atomicMax(&S.ngmax, r.T);
-                        }
-                    }
-                }
-                __syncthreads();
-                phases++;
-                axis_last = axis;
-                ng_p += S.ngmax;
-                if (warp == 0) {
-                    const bool c = sg_is_codeword(S.hdw, lane);
-                    if (lane == 0)
-                        S.conv = c;
-                }
-                __syncthreads();
-                conv = S.conv != 0;
-            }
-        }
-
-        /* hard_decision (:393-415): info bit b = s*64 + r*8 + c is the sign of
-         * L_APP at cube index s*256 + r*16 + c; packed MSB first (:272-280) */
-        if (tid < SG_INFO_BYTES) {
-            uint32_t byte = 0;
-            for (int q = 0; q < 8; q++) {
-                const int b = tid * 8 + q;
-                const int p = (b >> 6) * 256 + ((b >> 3) & 7) * 16 + (b & 7);
-                int l, bit;
-                if (axis_last == 0) {
-                    l = (p >> 8) * 16 + ((p >> 4) & 15);
-                    bit = p & 15;
-                } else if (axis_last == 1) {
-                    l = (p >> 8) * 16 + (p & 15);
-                    bit = (p >> 4) & 15;
-                } else {
-                    l = ((p >> 4) & 15) * 16 + (p & 15);
-                    bit = p >> 8;
-                }
-                byte = (byte << 1) | ((S.hdw[l] >> bit) & 1u);
-            }
-            args.bits[cw * SG_INFO_BYTES + tid] = (uint8_t)byte;
-        }
-        if (tid == 0 && args.stats) {
-            sg_cw_stats st;
-            st.iterations = 0.5 * phases;
-            st.ng = S.ng;
-            st.ng_p = ng_p;
-            st.converged = conv ? 1 : 0;
-            st.phases = phases;
-            args.stats[cw] = st;
-        }
-        __syncthreads();
-    }
-}
-
-#include "sg_persist.cuh"
+#include "sg_kernels.cuh"
 #include "sg_adjoint.cuh"
-
-struct SgLineSmem {
-    alignas(16) double etab[SG_EXP_TAB_LEN];
-    alignas(16) double ltab[SG_LOG_TAB_LEN];
-    SgWarpScratch ws[SG_WARPS];
-};
-
-template <bool CR>
-__global__ void __launch_bounds__(SG_THREADS) sg_bitso_kernel(const double* __restrict__ llr,
-                                                               unsigned long long n_lines,
-                                                               SgLineParams lp, double* lapp, double* le,
-                                                               int32_t* nguess, int32_t* ncw,
-                                                               const uint32_t* enum_tabs)
-{
-    __shared__ SgLineSmem S;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    for (int i = tid; i < SG_EXP_TAB_LEN; i += SG_THREADS)
-        S.etab[i] = g_etab[i];
-    for (int i = tid; i < SG_LOG_TAB_LEN; i += SG_THREADS)
-        S.ltab[i] = g_ltab[i];
-    __syncthreads();
-    for (unsigned long long l = (unsigned long long)blockIdx.x * SG_WARPS + warp; l < n_lines;
-         l += (unsigned long long)gridDim.x * SG_WARPS) {
-        const double v = lane < 16 ? llr[l * 16 + lane] : 1.0;
-        if (__any_sync(SG_FULL, !isfinite(v))) { /* not decoded: NaN out, N_guess -1 */
-            if (lane < 16) {
-                lapp[l * 16 + lane] = __longlong_as_double(0x7ff8000000000000ll);
-                le[l * 16 + lane] = __longlong_as_double(0x7ff8000000000000ll);
-            }
-            if (lane == 0) {
-                nguess[l] = -1;
-                if (ncw)
-                    ncw[l] = 0;
-            }
-            continue;
-        }
-        const SgLineResult r = sg_decode_line<1, false, CR>(v, lp, enum_tabs, S.etab, S.ltab, &S.ws[warp]);
-        if (lane < 16) {
-            lapp[l * 16 + lane] = r.lapp;
-            le[l * 16 + lane] = r.le;
-        }
-        if (lane == 0) {
-            nguess[l] = (int32_t)r.T;
-            if (ncw)
-                ncw[l] = r.ncw;
-        }
-    }
-}
 
 __global__ void __launch_bounds__(SG_THREADS) sg_gen_kernel(uint64_t seed, uint64_t cw0,
                                                              unsigned long long n_cw, double sigma,
                                                              double lo, double hi, uint8_t* info,
-                                                             double* llr)
+                                                             double* llr, const __grid_constant__ SgK k)
 {
-    __shared__ alignas(16) double etab[SG_EXP_TAB_LEN];
-    __shared__ alignas(16) double ltab[SG_LOG_TAB_LEN];
+    __shared__ alignas(16) double etab_s[SG_EXP_TAB_LEN];
+    __shared__ alignas(16) double ltab_s[SG_LOG_TAB_LEN];
+    const SgTab etab{etab_s, k.v}, ltab{ltab_s, k.v};
     __shared__ uint16_t W[256];
     __shared__ alignas(16) double stage[SG_CUBE]; /* the codeword's LLRs, stored coalesced */
     __shared__ uint8_t ib[SG_INFO_BYTES];
@@ -439,9 +46,9 @@ __global__ void __launch_bounds__(SG_THREADS) sg_gen_kernel(uint64_t seed, uint6
     __shared__ uint8_t ptab[256];
     const int tid = threadIdx.x;
     for (int i = tid; i < SG_EXP_TAB_LEN; i += SG_THREADS)
-        etab[i] = g_etab[i];
+        etab_s[i] = g_etab[i];
     for (int i = tid; i < SG_LOG_TAB_LEN; i += SG_THREADS)
-        ltab[i] = g_ltab[i];
+        ltab_s[i] = g_ltab[i];
     if (tid < 8)
         prow[tid] = c_prow[tid];
     ptab[tid] = c_ptab[tid];
@@ -493,10 +100,10 @@ __global__ void __launch_bounds__(SG_THREADS) sg_gen_kernel(uint64_t seed, uint6
          * unluckiest lane.  Each position keeps its first accepted attempt
          * (after SG_POLAR_TRIES rejections, 0), as sg_normal does; the LLRs
          * are staged in shared memory and stored coalesced. */
-        int k = 0;
+        int q = 0;
         uint64_t att = 0;
-        while (k < SG_CUBE / SG_THREADS) {
-            const uint32_t p = (uint32_t)(tid + SG_THREADS * k);
+        while (q < SG_CUBE / SG_THREADS) {
+            const uint32_t p = (uint32_t)(tid + SG_THREADS * q);
             const uint64_t ctr = gc * 4096u + p;
             const double u = sg_sym_unit(sg_rand(seed, 1 + 2 * att, ctr));
             const double v = sg_sym_unit(sg_rand(seed, 2 + 2 * att, ctr));
@@ -509,12 +116,12 @@ __global__ void __launch_bounds__(SG_THREADS) sg_gen_kernel(uint64_t seed, uint6
                 if (ok) {
                     const double l = sg_log(ss, ltab);
                     const double m = -2.0 * l;
-                    const double q = m / ss;
-                    z = u * __dsqrt_rn(q);
+                    const double ms = m / ss;
+                    z = u * __dsqrt_rn(ms);
                 }
                 const int bit = (W[p >> 4] >> (p & 15)) & 1;
                 stage[p] = sg_llr_of(bit, s, z);
-                k++;
+                q++;
                 att = 0;
             } else {
                 att++;
@@ -595,66 +202,6 @@ __global__ void __launch_bounds__(256) sg_summary_kernel(const sg_cw_stats* __re
     }
 }
 
-/* Decoder kernel configurations: warps per codeword CTA, channel cube in
- * shared memory (bulk copy) or read from global memory, minimum resident
- * CTAs per SM for the register budget, error patterns per lane per step,
- * and lines per warp (1: 32 lanes per line, sg_line.cuh; 2: 16 lanes per
- * line, sg_line16.cuh). */
-struct SgVariant {
-    const char* name;
-    int nw;
-    bool lch_smem;
-    size_t smem;
-    const void* fn;    /* table-driven exp/log */
-    const void* fn_cr; /* correctly rounded exp/log (the reference-exact mode) */
-};
-
-#define SG_VARIANT(NW, L, M, G, NAME)                                                               \
-    { NAME, NW, L, sizeof(SgCwSmem<NW, L>), (const void*)sg_decode_kernel<NW, L, M, G, false>, \
-      (const void*)sg_decode_kernel<NW, L, M, G, true> }
-#define SG_VARIANT_L2(NW, M, G, NAME)                                                                          \
-    { NAME, NW, false, sizeof(SgCwSmem<NW, false, 2>), (const void*)sg_decode_kernel<NW, false, M, G, false, 2>, \
-      (const void*)sg_decode_kernel<NW, false, M, G, true, 2> }
-static const SgVariant g_variants[] = {
-    SG_VARIANT(8, false, 3, 1, "w8-gmem"),
-    SG_VARIANT(8, true, 2, 1, "w8-smem"),
-    SG_VARIANT(12, true, 2, 1, "w12-smem"),
-    SG_VARIANT(16, false, 2, 1, "w16-gmem"),
-    SG_VARIANT(16, false, 2, 2, "w16-gmem-g2"),
-    SG_VARIANT(8, false, 3, 2, "w8-gmem-g2"),
-    SG_VARIANT(12, true, 2, 2, "w12-smem-g2"),
-    SG_VARIANT_L2(8, 2, 2, "w8-l2-g2"),
-    SG_VARIANT_L2(8, 2, 4, "w8-l2-g4"),
-    SG_VARIANT_L2(10, 2, 2, "w10-l2-g2"),
-    SG_VARIANT_L2(16, 1, 2, "w16-l2-g2"),
-};
-#define SG_NVARIANTS ((int)(sizeof(g_variants) / sizeof(g_variants[0])))
-
-/* Batched persistent decoder configurations: warps per CTA (one CTA per
- * SM), codeword slots per CTA. */
-struct SgPVariant {
-    const char* name;
-    int nw;
-    int slots;
-    size_t smem;
-    const void* fn;    /* table-driven exp/log */
-    const void* fn_cr; /* correctly rounded exp/log (the reference-exact mode) */
-};
-#define SG_PVARIANT(NW, C, G, NAME)                                                                \
-    { NAME, NW, C, sizeof(SgPersistSmem<NW, C>), (const void*)sg_persist_kernel<NW, C, G, false>, \
-      (const void*)sg_persist_kernel<NW, C, G, true> }
-static const SgPVariant g_pvariants[] = {
-    SG_PVARIANT(24, 3, 1, "p24x3"),
-    SG_PVARIANT(28, 3, 1, "p28x3"),
-    SG_PVARIANT(16, 3, 1, "p16x3"),
-    SG_PVARIANT(20, 4, 1, "p20x4"),
-    SG_PVARIANT(32, 3, 1, "p32x3"),
-    SG_PVARIANT(32, 3, 2, "p32x3-g2"),
-    SG_PVARIANT(24, 3, 2, "p24x3-g2"),
-    SG_PVARIANT(28, 3, 2, "p28x3-g2"),
-};
-#define SG_NPVARIANTS ((int)(sizeof(g_pvariants) / sizeof(g_pvariants[0])))
-
 /* 16-byte alignment of the shared tables (double2 loads) and of the bulk
  * copy destination, for every configuration built. */
 template <class T>
@@ -682,10 +229,10 @@ static_assert(sizeof(SgPersistSmem<32, 3>) <= 227 * 1024 && sizeof(SgPersistSmem
                   sizeof(SgCwSmem<16, false>) <= 227 * 1024 && sizeof(SgCwSmem<12, true>) <= 227 * 1024 &&
                   sizeof(SgCwSmem<16, false, 2>) <= 227 * 1024,
               "shared memory per CTA");
-/* the two-lines-per-warp configurations built for two CTAs per SM fit them
- * (228 KB per SM, 1 KB of it reserved per CTA) */
+/* the configurations built for two CTAs per SM fit them (228 KB per SM, 1 KB
+ * of it reserved per CTA) */
 static_assert(2 * (sizeof(SgCwSmem<8, false, 2>) + 1024) <= 228 * 1024 &&
-                  2 * (sizeof(SgCwSmem<10, false, 2>) + 1024) <= 228 * 1024,
+                  2 * (sizeof(SgCwSmem<16, false>) + 1024) <= 228 * 1024,
               "two CTAs per SM");
 
 /* Static device memory of the allocation-free entry point: the error flag
@@ -715,14 +262,16 @@ __global__ void sg_enum_build_kernel(uint32_t* out, unsigned int* ok)
  * reference's per-guess arithmetic can reach.  CR: the correctly rounded
  * exp; otherwise the table-driven sg_exp_neg. */
 template <bool CR>
-__global__ void __launch_bounds__(256) sg_guess_ceiling_kernel(unsigned long long iters, double* sink)
+__global__ void __launch_bounds__(256) sg_guess_ceiling_kernel(unsigned long long iters, double* sink,
+                                                               const __grid_constant__ SgK k)
 {
-    __shared__ alignas(16) double etab[SG_EXP_TAB_LEN];
+    __shared__ alignas(16) double etab_s[SG_EXP_TAB_LEN];
+    const SgTab etab{etab_s, k.v};
     for (int i = threadIdx.x; i < SG_EXP_TAB_LEN; i += 256)
-        etab[i] = g_etab[i];
+        etab_s[i] = g_etab[i];
     __syncthreads();
     double pm0 = 1e-3 * (threadIdx.x + 1), pm1 = pm0 + 0.37, acc0 = 1.0, acc1 = 1.0;
-    for (unsigned long long k = 0; k < iters; k++) {
+    for (unsigned long long it = 0; it < iters; it++) {
         pm0 = __dadd_rn(pm0, 1.1e-5);
         pm1 = __dadd_rn(pm1, 1.3e-5);
         acc0 = __dsub_rn(acc0, CR ? sg_exp_cr_neg(-pm0, etab) : sg_exp_neg(-pm0, etab));
@@ -768,10 +317,9 @@ std::mutex g_mu;
 std::atomic<long long> g_wait_limit{SG_WAIT_LIMIT_DEFAULT};
 std::atomic<int> g_math_mode{0}; /* 0: table-driven exp/log, 1: correctly rounded */
 /* Selected kernel variants, one per math mode (sogrand_b200.autotune
- * measures them): on B200 at 2 dB the table math is fastest with two error
- * patterns per lane (p32x3-g2, w16-gmem-g2), the correctly rounded math,
- * whose larger exp leaves no registers for the second pattern, with one
- * (p32x3, w16-gmem). */
+ * measures them).  B200, 12 000 codewords at 2 dB, table math: p32x3 122.0
+ * ms, p28x3 124.2, p24x3 127.1; w16-gmem 124.8, w8-gmem 139.1, w12-smem
+ * 140.7, w8-smem 169.1. */
 int g_pvariant_by_mode[2] = {5, 4};
 int g_variant_by_mode[2] = {4, 3};
 #define g_pvariant (g_pvariant_by_mode[g_math_mode.load()])
@@ -783,6 +331,12 @@ bool g_host_ready = false;
 
 const double k_etab_host[SG_EXP_TAB_LEN] = SG_EXP_TAB_INIT;
 const double k_ltab_host[SG_LOG_TAB_LEN] = SG_LOG_TAB_INIT;
+const SgK k_consts = SG_K_INIT;
+const SgTab k_etab_tab{k_etab_host, k_consts.v}, k_ltab_tab{k_ltab_host, k_consts.v};
+
+/* Kernel of a configuration, by math mode. */
+const void* decode_fn(int v, bool cr) { return cr ? sg_cr_decode_fn(v) : k_variants[v].fn; }
+const void* persist_fn(int v, bool cr) { return cr ? sg_cr_persist_fn(v) : k_pvariants[v].fn; }
 
 sg_status host_init_locked()
 {
@@ -815,20 +369,19 @@ sg_status get_ctx(DevCtx** out)
         SG_CUDA(cudaMalloc(&c.err, sizeof(unsigned int)));
         SG_CUDA(cudaMalloc(&c.err_sink, 148 * 64 * sizeof(double)));
         SG_CUDA(cudaMemset(c.err, 0, sizeof(unsigned int)));
-        SG_CUDA(cudaMemcpyToSymbol(c_hcol, g_code.hcol, sizeof g_code.hcol));
-        SG_CUDA(cudaMemcpyToSymbol(c_prow, g_code.prow, sizeof g_code.prow));
-        SG_CUDA(cudaMemcpyToSymbol(c_ptab, g_code.ptab, sizeof g_code.ptab));
+        SG_CUDA(sg_load_code(g_code));
+        SG_CUDA(sg_cr_load_code(g_code));
         for (int v = 0; v < SG_NVARIANTS; v++) {
-            SG_CUDA(cudaFuncSetAttribute(g_variants[v].fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)g_variants[v].smem));
-            SG_CUDA(cudaFuncSetAttribute(g_variants[v].fn_cr, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)g_variants[v].smem));
+            SG_CUDA(cudaFuncSetAttribute(decode_fn(v, false), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)k_variants[v].smem));
+            SG_CUDA(cudaFuncSetAttribute(decode_fn(v, true), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)k_variants[v].smem));
         }
         for (int v = 0; v < SG_NPVARIANTS; v++) {
-            SG_CUDA(cudaFuncSetAttribute(g_pvariants[v].fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)g_pvariants[v].smem));
-            SG_CUDA(cudaFuncSetAttribute(g_pvariants[v].fn_cr, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)g_pvariants[v].smem));
+            SG_CUDA(cudaFuncSetAttribute(persist_fn(v, false), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)k_pvariants[v].smem));
+            SG_CUDA(cudaFuncSetAttribute(persist_fn(v, true), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)k_pvariants[v].smem));
         }
         SG_CUDA(cudaFuncSetAttribute(sg_backward_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)sizeof(SgBackSmem<8>)));
@@ -860,6 +413,37 @@ uint32_t tmax_eff(uint64_t tmax)
     if (tmax == 0)
         return 0x7fffffffu; /* if (Tmax==0) Tmax=Inf, :607 */
     return tmax > 0xffffffffull ? 0xffffffffu : (uint32_t)tmax;
+}
+
+/* Starts of the logistic weights of every IC's pattern order, counted once. */
+struct OrderStarts {
+    std::vector<uint32_t> start[SG_ENUM_NTAB];
+    uint32_t h3[SG_ENUM_NTAB];
+    OrderStarts()
+    {
+        uint32_t cnt[17][137];
+        sg_enum_counts(cnt);
+        for (int ic = 0; ic < SG_ENUM_NTAB; ic++) {
+            start[ic].resize(16 * ic + 136);
+            start[ic].resize(sg_enum_starts(ic, cnt, start[ic].data(), &h3[ic]));
+        }
+    }
+};
+
+/* sg_order_meta for a Tmax as tmax_eff() gives it: the first weight that
+ * starts at or after Tmax ends the decode. */
+void order_meta(uint32_t tmax, sg_order_meta* m)
+{
+    static const OrderStarts o;
+    for (int ic = 0; ic < SG_ENUM_NTAB; ic++) {
+        m->h3[ic] = o.h3[ic];
+        m->lim[ic] = SG_ENUM_LEN;
+        if (tmax < SG_ENUM_LEN) {
+            const auto it = std::lower_bound(o.start[ic].begin(), o.start[ic].end(), tmax);
+            if (it != o.start[ic].end())
+                m->lim[ic] = *it;
+        }
+    }
 }
 
 int grid_for(unsigned long long n, int cap)
@@ -919,14 +503,16 @@ sg_status sg_decode_device(const double* d_llr, size_t n_cw, const sg_params* p,
     a.wait_limit = g_wait_limit.load();
     a.L = p->L;
     a.imax = p->Imax;
-    a.tmax = tmax_eff(p->Tmax);
+    order_meta(tmax_eff(p->Tmax), &a.meta);
     a.use_bulk = ((uintptr_t)d_llr & 15u) == 0;
     a.thres = p->thres;
     memcpy(a.alpha, p->alpha, sizeof a.alpha);
-    const SgVariant& v = g_variants[g_variant];
+    a.k = k_consts;
+    const int mode = g_math_mode.load(), vi = g_variant_by_mode[mode];
+    const SgVariant& v = k_variants[vi];
     const int grid = grid_for(n_cw, 1 << 30);
     void* kargs[] = {(void*)&a};
-    SG_CUDA(cudaLaunchKernel(g_math_mode.load() ? v.fn_cr : v.fn, dim3(grid), dim3(v.nw * 32), kargs, v.smem,
+    SG_CUDA(cudaLaunchKernel(decode_fn(vi, mode == 1), dim3(grid), dim3(v.nw * 32), kargs, v.smem,
                              (cudaStream_t)stream));
     return SG_OK;
 }
@@ -944,18 +530,15 @@ sg_status sg_bitso_device(const double* d_llr, size_t n_lines, int32_t L, uint64
     sg_status s = get_ctx(&c);
     if (s != SG_OK)
         return s;
-    SgLineParams lp;
-    lp.L = L;
-    lp.tmax = tmax_eff(Tmax);
-    lp.thres = thres;
+    sg_order_meta meta;
+    order_meta(tmax_eff(Tmax), &meta);
     const unsigned long long blocks = (n_lines + SG_WARPS - 1) / SG_WARPS;
-    if (g_math_mode.load())
-        sg_bitso_kernel<true><<<grid_for(blocks, 148 * 64), SG_THREADS, 0, (cudaStream_t)stream>>>(
-            d_llr, n_lines, lp, d_lapp, d_le, d_nguess, d_ncw, c->enum_tabs);
-    else
-        sg_bitso_kernel<false><<<grid_for(blocks, 148 * 64), SG_THREADS, 0, (cudaStream_t)stream>>>(
-            d_llr, n_lines, lp, d_lapp, d_le, d_nguess, d_ncw, c->enum_tabs);
-    SG_CUDA(cudaGetLastError());
+    const uint32_t* tabs = c->enum_tabs;
+    SgK k = k_consts;
+    unsigned long long n = n_lines;
+    void* kargs[] = {&d_llr, &n, &L, &thres, &d_lapp, &d_le, &d_nguess, &d_ncw, &tabs, &k, &meta};
+    SG_CUDA(cudaLaunchKernel(g_math_mode.load() ? sg_cr_bitso_fn() : (const void*)sg_bitso_kernel<false>,
+                             dim3(grid_for(blocks, 148 * 64)), dim3(SG_THREADS), kargs, 0, (cudaStream_t)stream));
     return SG_OK;
 }
 
@@ -1097,10 +680,10 @@ sg_status sg_gen_llr_host(uint64_t seed, uint64_t cw0, size_t n_cw, double sigma
         if (info)
             memcpy(info + c * SG_INFO_BYTES, ib, SG_INFO_BYTES);
         sg_encode_words(ib, g_code.prow, g_code.ptab, W);
-        const double s = sigma > 0.0 ? sigma : sg_sigma_draw(seed, gc, ebn0_lo_db, ebn0_hi_db, k_etab_host);
+        const double s = sigma > 0.0 ? sigma : sg_sigma_draw(seed, gc, ebn0_lo_db, ebn0_hi_db, k_etab_tab);
         for (int p = 0; p < SG_CUBE; p++) {
             const int bit = (W[p >> 4] >> (p & 15)) & 1;
-            llr[c * SG_CUBE + p] = sg_llr_of(bit, s, sg_normal(seed, gc, (uint32_t)p, k_ltab_host));
+            llr[c * SG_CUBE + p] = sg_llr_of(bit, s, sg_normal(seed, gc, (uint32_t)p, k_ltab_tab));
         }
     }
     return SG_OK;
@@ -1120,7 +703,7 @@ sg_status sg_gen_llr_device(uint64_t seed, uint64_t cw0, size_t n_cw, double sig
     if (s != SG_OK)
         return s;
     sg_gen_kernel<<<grid_for(n_cw, 148 * 16), SG_THREADS, 0, (cudaStream_t)stream>>>(
-        seed, cw0, n_cw, sigma, ebn0_lo_db, ebn0_hi_db, d_info, d_llr);
+        seed, cw0, n_cw, sigma, ebn0_lo_db, ebn0_hi_db, d_info, d_llr, k_consts);
     SG_CUDA(cudaGetLastError());
     return SG_OK;
 }
@@ -1132,8 +715,13 @@ size_t sg_pattern_order(int32_t ic, uint32_t* out, size_t cap)
     std::vector<uint32_t> t(SG_ENUM_LEN);
     const size_t n = sg_enum_build_impl(ic, t.data());
     const size_t m = n < cap ? n : cap;
-    for (size_t i = 0; i < m; i++)
-        out[i] = sg_ent_pattern(t[i]) | (t[i] & SG_ENUM_GS);
+    int32_t prev = 0;
+    for (size_t i = 0; i < m; i++) {
+        const uint32_t pat = sg_ent_pattern(t[i]);
+        const int32_t wt = sg_enum_weight(ic, pat);
+        out[i] = pat | (i && wt != prev ? SG_ENUM_GS : 0u);
+        prev = wt;
+    }
     return m;
 }
 
@@ -1215,14 +803,13 @@ sg_status noalloc_setup(NoAllocCtx** out)
         sg_code_build(&code);
         SG_CUDA(cudaGetSymbolAddress((void**)&c.scratch, g_noalloc_scratch));
         SG_CUDA(cudaGetSymbolAddress((void**)&c.enum_tabs, g_noalloc_enum));
-        SG_CUDA(cudaMemcpyToSymbol(c_hcol, code.hcol, sizeof code.hcol));
-        SG_CUDA(cudaMemcpyToSymbol(c_prow, code.prow, sizeof code.prow));
-        SG_CUDA(cudaMemcpyToSymbol(c_ptab, code.ptab, sizeof code.ptab));
+        SG_CUDA(sg_load_code(code));
+        SG_CUDA(sg_cr_load_code(code));
         for (int v = 0; v < SG_NVARIANTS; v++) {
-            SG_CUDA(cudaFuncSetAttribute(g_variants[v].fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)g_variants[v].smem));
-            SG_CUDA(cudaFuncSetAttribute(g_variants[v].fn_cr, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)g_variants[v].smem));
+            SG_CUDA(cudaFuncSetAttribute(decode_fn(v, false), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)k_variants[v].smem));
+            SG_CUDA(cudaFuncSetAttribute(decode_fn(v, true), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)k_variants[v].smem));
         }
         /* the completion flags of the build borrow the scratch array */
         unsigned int* ok = reinterpret_cast<unsigned int*>(c.scratch);
@@ -1286,14 +873,16 @@ sg_status sg_decode_summary_device_noalloc(const double* d_llr, size_t n_cw, con
     a.wait_limit = g_wait_limit.load();
     a.L = p->L;
     a.imax = p->Imax;
-    a.tmax = tmax_eff(p->Tmax);
+    order_meta(tmax_eff(p->Tmax), &a.meta);
     a.use_bulk = ((uintptr_t)d_llr & 15u) == 0;
     a.thres = p->thres;
     memcpy(a.alpha, p->alpha, sizeof a.alpha);
-    const SgVariant& v = g_variants[g_variant];
+    a.k = k_consts;
+    const int mode = g_math_mode.load(), vi = g_variant_by_mode[mode];
+    const SgVariant& v = k_variants[vi];
     void* kargs[] = {(void*)&a};
-    SG_CUDA(cudaLaunchKernel(g_math_mode.load() ? v.fn_cr : v.fn, dim3(grid_for(n_cw, 1 << 30)),
-                             dim3(v.nw * 32), kargs, v.smem, st));
+    SG_CUDA(cudaLaunchKernel(decode_fn(vi, mode == 1), dim3(grid_for(n_cw, 1 << 30)), dim3(v.nw * 32), kargs, v.smem,
+                             st));
     sg_summary_kernel<<<grid_for((n_cw + 255) / 256, 148 * 8), 256, 0, st>>>(stats, bits, d_ref_info, n_cw, err,
                                                                               d_summary);
     SG_CUDA(cudaGetLastError());
@@ -1344,16 +933,17 @@ sg_status batch_enqueue(sg_batch b, const double* d_llr, size_t n_cw, const sg_p
     a.wait_limit = g_wait_limit.load();
     a.L = p->L;
     a.imax = p->Imax;
-    a.tmax = tmax_eff(p->Tmax);
+    order_meta(tmax_eff(p->Tmax), &a.meta);
     a.use_bulk = 0;
     a.thres = p->thres;
     memcpy(a.alpha, p->alpha, sizeof a.alpha);
-    const SgPVariant& v = g_pvariants[g_pvariant];
+    a.k = k_consts;
+    const int mode = g_math_mode.load(), vi = g_pvariant_by_mode[mode];
+    const SgPVariant& v = k_pvariants[vi];
     SgQueue* q = b->q;
     void* kargs[] = {(void*)&a, (void*)&q};
     const int grid = (int)(n_cw < (size_t)c->sms ? n_cw : (size_t)c->sms);
-    SG_CUDA(cudaLaunchKernel(g_math_mode.load() ? v.fn_cr : v.fn, dim3(grid), dim3(v.nw * 32), kargs, v.smem,
-                             st));
+    SG_CUDA(cudaLaunchKernel(persist_fn(vi, mode == 1), dim3(grid), dim3(v.nw * 32), kargs, v.smem, st));
     return SG_OK;
 }
 
@@ -1777,7 +1367,7 @@ sg_status sg_batch_check(sg_batch b)
 
 int sg_batch_variant_count(void) { return SG_NPVARIANTS; }
 
-const char* sg_batch_variant_name(int v) { return (v >= 0 && v < SG_NPVARIANTS) ? g_pvariants[v].name : ""; }
+const char* sg_batch_variant_name(int v) { return (v >= 0 && v < SG_NPVARIANTS) ? k_pvariants[v].name : ""; }
 
 sg_status sg_batch_set_variant(int v)
 {
@@ -1793,7 +1383,7 @@ sg_status sg_guess_ceiling(unsigned long long iters, int32_t mode, double* guess
 {
     if (!guesses_per_second || iters == 0 || (mode != 0 && mode != 1))
         return fail(SG_ERR_ARG, "need iters > 0, mode 0 or 1 and an output pointer");
-    void (*kern)(unsigned long long, double*) =
+    void (*kern)(unsigned long long, double*, SgK) =
         mode == 1 ? sg_guess_ceiling_kernel<true> : sg_guess_ceiling_kernel<false>;
     DevCtx* c = nullptr;
     sg_status s = get_ctx(&c);
@@ -1803,9 +1393,9 @@ sg_status sg_guess_ceiling(unsigned long long iters, int32_t mode, double* guess
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     SG_CUDA(cudaEventCreate(&e0));
     SG_CUDA(cudaEventCreate(&e1));
-    kern<<<blocks, 256>>>(iters / 8 + 1, c->err_sink); /* warm-up */
+    kern<<<blocks, 256>>>(iters / 8 + 1, c->err_sink, k_consts); /* warm-up */
     SG_CUDA(cudaEventRecord(e0));
-    kern<<<blocks, 256>>>(iters, c->err_sink);
+    kern<<<blocks, 256>>>(iters, c->err_sink, k_consts);
     SG_CUDA(cudaEventRecord(e1));
     SG_CUDA(cudaEventSynchronize(e1));
     float ms = 0;
@@ -1845,11 +1435,12 @@ sg_status sg_forward_device(const double* d_llr, size_t n_cw, const sg_params* p
     a.wait_limit = g_wait_limit.load();
     a.L = p->L;
     a.imax = p->Imax;
-    a.tmax = tmax_eff(p->Tmax);
+    order_meta(tmax_eff(p->Tmax), &a.meta);
     a.use_bulk = ((uintptr_t)d_llr & 15u) == 0;
     a.thres = p->thres;
     memcpy(a.alpha, p->alpha, sizeof a.alpha);
-    const SgVariant& v = g_variants[g_variant];
+    a.k = k_consts;
+    const SgVariant& v = k_variants[g_variant];
     void* kargs[] = {(void*)&a};
     SG_CUDA(cudaLaunchKernel(v.fn, dim3(grid_for(n_cw, 1 << 30)), dim3(v.nw * 32), kargs, v.smem,
                              (cudaStream_t)stream));
@@ -1887,9 +1478,11 @@ sg_status sg_backward_device(const double* d_llr, size_t n_cw, const sg_params* 
     a.n_cw = n_cw;
     a.L = p->L;
     a.nph = 3 * p->Imax;
+    order_meta(0xffffffffu, &a.meta);
     a.loss_mode = loss_mode;
     a.thres = p->thres;
     memcpy(a.alpha, p->alpha, sizeof a.alpha);
+    a.k = k_consts;
     void* kargs[] = {(void*)&a};
     SG_CUDA(cudaLaunchKernel((const void*)sg_backward_kernel<8>, dim3(grid_for(n_cw, 1 << 30)), dim3(256), kargs,
                              sizeof(SgBackSmem<8>), (cudaStream_t)stream));
@@ -1936,7 +1529,7 @@ int sg_decoder_variant_count(void) { return SG_NVARIANTS; }
 
 const char* sg_decoder_variant_name(int v)
 {
-    return (v >= 0 && v < SG_NVARIANTS) ? g_variants[v].name : "";
+    return (v >= 0 && v < SG_NVARIANTS) ? k_variants[v].name : "";
 }
 
 sg_status sg_decoder_set_variant(int v)

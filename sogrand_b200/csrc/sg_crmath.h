@@ -50,7 +50,7 @@
 #define SG_CR_EPS_SLOW 0x1p-101
 
 #if defined(__CUDACC__)
-#define SG_NOINL __host__ __device__ __noinline__
+#define SG_NOINL static __host__ __device__ __noinline__
 #else
 #define SG_NOINL static __attribute__((noinline))
 #endif
@@ -169,26 +169,26 @@ SG_HD int sg_cr_round_sub(double yh, double yl, int e, double eps, int force, do
 /* Argument reduction of exp: x = (128 e + j) ln2/128 + r, r = rh + rl to
  * 2^-110 absolute, |r| < 2^-8.5.  kd*C1 and kd*C2 are exact (|kd| < 2^18,
  * 35-bit constants) and x - kd*C1 is exact (Sterbenz). */
-SG_HD void sg_exp_reduce(double x, double* rh, double* rl, int* j, int* e)
+SG_HD void sg_exp_reduce(double x, SgTab tab, double* rh, double* rl, int* j, int* e)
 {
-    const double kd0 = x * SG_EXP_INV_LN2_N + SG_EXP_SHIFT;
+    const double kd0 = x * SGK(EXP_INV_LN2_N) + SG_EXP_SHIFT;
     const int k = (int)(uint32_t)sg_bits(kd0); /* round(x * 128/ln2) */
     const double kd = kd0 - SG_EXP_SHIFT;
-    const double t1 = sg_fma(-kd, SG_CR_EXP_C1, x);
+    const double t1 = sg_fma(-kd, SGK(CR_EXP_C1), x);
     double re;
-    *rh = sg_two_sum(t1, -(kd * SG_CR_EXP_C2), &re);
-    *rl = re - kd * SG_CR_EXP_C3;
+    *rh = sg_two_sum(t1, -(kd * SGK(CR_EXP_C2)), &re);
+    *rl = re - kd * SGK(CR_EXP_C3);
     *j = k & 127;
     *e = k >> 7;
 }
 
 /* exp(x) / 2^e as a double-double to about 2^-104 (e and the reduction as
  * sg_exp_reduce): e^r and 2^(j/128) in double-double arithmetic. */
-SG_HD sg_dd sg_exp_cr_dd(double x, const double* tab, int* e)
+SG_HD sg_dd sg_exp_cr_dd(double x, SgTab tab, int* e)
 {
     double rh, rl;
     int j;
-    sg_exp_reduce(x, &rh, &rl, &j, e);
+    sg_exp_reduce(x, tab, &rh, &rl, &j, e);
     double rle;
     const double r0 = sg_two_sum(rh, rl, &rle);
     const sg_dd r = sg_dd_mk(r0, rle);
@@ -206,13 +206,13 @@ SG_HD sg_dd sg_exp_cr_dd(double x, const double* tab, int* e)
     P = sg_dd_add(sg_dd_mul(P, r), sg_dd_mk(SG_CR_EXP_F2_HI, SG_CR_EXP_F2_LO));
     P = sg_dd_add(sg_dd_mul(P, r), sg_dd_mk(1.0, 0.0));
     P = sg_dd_mul(P, r); /* e^r - 1 */
-    const double H = tab[2 * j];
-    const sg_dd T = sg_dd_mk(H, H * tab[2 * j + 1]); /* 2^(j/128) */
+    const double H = SG_EXP_H(j);
+    const sg_dd T = sg_dd_mk(H, H * SG_EXP_T(j)); /* 2^(j/128) */
     return sg_dd_add(T, sg_dd_mul(T, P));
 }
 
 /* exp slow path: the double-double value, rounded. */
-SG_NOINL double sg_exp_cr_slow(double x, const double* tab)
+SG_NOINL double sg_exp_cr_slow(double x, SgTab tab)
 {
     SG_CR_PROBE(1);
     int e;
@@ -228,20 +228,20 @@ SG_NOINL double sg_exp_cr_slow(double x, const double* tab)
 }
 
 /* Fast path of exp: 2^(j/128) e^r / 2^e = yh + yl to 2^-67 relative. */
-SG_HD double sg_exp_cr_fast(double rh, double rl, int j, const double* tab, double* yl)
+SG_HD double sg_exp_cr_fast(double rh, double rl, int j, SgTab tab, double* yl)
 {
 #if defined(__CUDA_ARCH__)
-    const double2 Ht = reinterpret_cast<const double2*>(tab)[j];
+    const double2 Ht = *reinterpret_cast<const double2*>(&SG_EXP_H(j));
     const double H = Ht.x, t = Ht.y;
 #else
-    const double H = tab[2 * j], t = tab[2 * j + 1];
+    const double H = SG_EXP_H(j), t = SG_EXP_T(j);
 #endif
     /* q = e^r - 1 - r to 2^-69.3 absolute (|r| < 2^-8.5) */
     const double r2 = rh * rh;
-    double p = sg_fma(rh, SG_EXP_C7, SG_EXP_C6);
-    p = sg_fma(rh, p, SG_EXP_C5);
-    p = sg_fma(rh, p, SG_EXP_C4);
-    p = sg_fma(rh, p, SG_EXP_C3);
+    double p = sg_fma(rh, SGK(EXP_C7), SGK(EXP_C6));
+    p = sg_fma(rh, p, SGK(EXP_C5));
+    p = sg_fma(rh, p, SGK(EXP_C4));
+    p = sg_fma(rh, p, SGK(EXP_C3));
     p = sg_fma(rh, p, SG_EXP_C2);
     const double q = sg_fma(r2, p, rh * rl);
     /* 2^(j/128) e^r = H (1 + t)(1 + rh + rl + q)
@@ -256,7 +256,7 @@ SG_HD double sg_exp_cr_fast(double rh, double rl, int j, const double* tab, doub
 
 /* Correctly rounded exp(x).  tab: the SG_EXP_TAB_LEN doubles {H_j, t_j} of
  * sg_math.h. */
-SG_HD double sg_exp_cr(double x, const double* tab)
+SG_HD double sg_exp_cr(double x, SgTab tab)
 {
     if (!(x <= SG_CR_EXP_XMAX)) /* NaN or overflow */
         return x != x ? x : sg_from_bits(0x7ff0000000000000ULL);
@@ -264,7 +264,7 @@ SG_HD double sg_exp_cr(double x, const double* tab)
         return 0.0;
     double rh, rl, yl, y;
     int j, e;
-    sg_exp_reduce(x, &rh, &rl, &j, &e);
+    sg_exp_reduce(x, tab, &rh, &rl, &j, &e);
     const double yh = sg_exp_cr_fast(rh, rl, j, tab, &yl);
     if (e >= -1021) {
         if (sg_cr_round(yh, yl, SG_CR_EPS_EXP, &y))
@@ -278,13 +278,13 @@ SG_HD double sg_exp_cr(double x, const double* tab)
 /* sg_exp_cr for x in [-707.5, 0] (the guess loop's exp(-PM), PM >= 0),
  * where the result is normal: the same operations without the range checks
  * and the subnormal rounding. */
-SG_HD double sg_exp_cr_neg(double x, const double* tab)
+SG_HD double sg_exp_cr_neg(double x, SgTab tab)
 {
     if (x < -707.5)
         return sg_exp_cr(x, tab);
     double rh, rl, yl, y;
     int j, e;
-    sg_exp_reduce(x, &rh, &rl, &j, &e);
+    sg_exp_reduce(x, tab, &rh, &rl, &j, &e);
     const double yh = sg_exp_cr_fast(rh, rl, j, tab, &yl);
     if (sg_cr_round(yh, yl, SG_CR_EPS_EXP, &y))
         return y * sg_pow2i(e);
@@ -294,7 +294,7 @@ SG_HD double sg_exp_cr_neg(double x, const double* tab)
 /* Argument reduction of log: x = 2^e z, z in [0.6875, 1.375) in
  * subinterval j; r = z c_j - 1 = rh + rl exactly, |r| < 2^-7.  x must be
  * positive and finite. */
-SG_HD void sg_log_reduce(double x, const double* tab, double* rh, double* rl, int* e, int* j)
+SG_HD void sg_log_reduce(double x, SgTab tab, double* rh, double* rl, int* e, int* j)
 {
     uint64_t ix = sg_bits(x);
     int escale = 0;
@@ -307,7 +307,7 @@ SG_HD void sg_log_reduce(double x, const double* tab, double* rh, double* rl, in
     *j = (int)((tmpb >> 45) & 127);
     *e = (int)((int64_t)tmpb >> 52) + escale;
     const double zz = sg_from_bits(ix - (tmpb & (0xfffULL << 52)));
-    const double c = tab[3 * *j];
+    const double c = SG_T(3 * *j);
     const double pr = zz * c;
     const double pe = sg_fma(zz, c, -pr);
     const double pm1 = pr - 1.0; /* exact (Sterbenz) */
@@ -317,12 +317,12 @@ SG_HD void sg_log_reduce(double x, const double* tab, double* rh, double* rl, in
 
 /* log(x) as a double-double to about 2^-104 (x positive and finite):
  * log1p(r), e ln2 and -log(c_j) in double-double arithmetic. */
-SG_HD sg_dd sg_log_cr_dd(double x, const double* tab)
+SG_HD sg_dd sg_log_cr_dd(double x, SgTab tab)
 {
     double rh, rl;
     int e, j;
     sg_log_reduce(x, tab, &rh, &rl, &e, &j);
-    const double lch = tab[3 * j + 1], lcl = tab[3 * j + 2];
+    const double lch = SG_T(3 * j + 1), lcl = SG_T(3 * j + 2);
     double rle;
     const double r0 = sg_two_sum(rh, rl, &rle);
     const sg_dd r = sg_dd_mk(r0, rle);
@@ -334,8 +334,8 @@ SG_HD sg_dd sg_log_cr_dd(double x, const double* tab)
     h = sg_fma(r0, h, SG_CR_LOG_G14);
     h = sg_fma(r0, h, SG_CR_LOG_G13);
     h = sg_fma(r0, h, SG_CR_LOG_G12);
-    h = sg_fma(r0, h, SG_CR_LOG_G11);
-    h = sg_fma(r0, h, SG_CR_LOG_G10);
+    h = sg_fma(r0, h, SGK(CR_LOG_G11));
+    h = sg_fma(r0, h, SGK(CR_LOG_G10));
     sg_dd P = sg_dd_mk(h, 0.0);
     P = sg_dd_add(sg_dd_mul(P, r), sg_dd_mk(SG_CR_LOG_G9_HI, SG_CR_LOG_G9_LO));
     P = sg_dd_add(sg_dd_mul(P, r), sg_dd_mk(SG_CR_LOG_G8_HI, SG_CR_LOG_G8_LO));
@@ -348,16 +348,16 @@ SG_HD sg_dd sg_log_cr_dd(double x, const double* tab)
     P = sg_dd_add(sg_dd_mul(P, r), sg_dd_mk(1.0, 0.0));
     P = sg_dd_mul(P, r); /* log1p(r) */
     const double ed = (double)e;
-    const double a = ed * SG_LOG_LN2_HI; /* exact */
-    const double b = ed * SG_LOG_LN2_LO;
-    const double be = sg_fma(ed, SG_LOG_LN2_LO, -b);
+    const double a = ed * SGK(LOG_LN2_HI); /* exact */
+    const double b = ed * SGK(LOG_LN2_LO);
+    const double be = sg_fma(ed, SGK(LOG_LN2_LO), -b);
     sg_dd E = sg_dd_add(sg_dd_mk(a, 0.0), sg_dd_mk(b, be + ed * SG_CR_LOG_LN2_LO2));
     E = sg_dd_add(E, sg_dd_mk(lch, lcl));
     return sg_dd_add(E, P);
 }
 
 /* log slow path: the double-double value, rounded. */
-SG_NOINL double sg_log_cr_slow(double x, const double* tab)
+SG_NOINL double sg_log_cr_slow(double x, SgTab tab)
 {
     SG_CR_PROBE(2);
     const sg_dd R = sg_log_cr_dd(x, tab);
@@ -368,7 +368,7 @@ SG_NOINL double sg_log_cr_slow(double x, const double* tab)
 
 /* Correctly rounded log(x).  tab: the SG_LOG_TAB_LEN doubles
  * {c_j, hi(-log c_j), lo(-log c_j)} of sg_math.h. */
-SG_HD double sg_log_cr(double x, const double* tab)
+SG_HD double sg_log_cr(double x, SgTab tab)
 {
     const uint64_t ix = sg_bits(x);
     if (ix - 0x0010000000000000ULL >= 0x7ff0000000000000ULL - 0x0010000000000000ULL) {
@@ -383,10 +383,10 @@ SG_HD double sg_log_cr(double x, const double* tab)
     double rh, rl;
     int e, j;
     sg_log_reduce(x, tab, &rh, &rl, &e, &j);
-    const double lch = tab[3 * j + 1];
-    const double lcl = tab[3 * j + 2];
+    const double lch = SG_T(3 * j + 1);
+    const double lcl = SG_T(3 * j + 2);
     double y, yl;
-    if (e == 0 && tab[3 * j] == 1.0 && fabs(rh) < 0x1p-30) {
+    if (e == 0 && SG_T(3 * j) == 1.0 && fabs(rh) < 0x1p-30) {
         /* x within 2^-30 of 1: r = x - 1 exactly, and log(x) = r - r^2/2 +
          * t with t = r^3/3 - r^4/4 (next term below 2^-120 relative).  The
          * first two terms are kept exact (h + u + ue) and only t is
@@ -399,7 +399,7 @@ SG_HD double sg_log_cr(double x, const double* tab)
         double he, ue, y1e;
         const double h = sg_two_sum(rh, -0.5 * s, &he);
         const double u = sg_two_sum(he, -0.5 * se, &ue);
-        const double t = (rh * s) * sg_fma(-0.25, rh, SG_CR_LOG_G3);
+        const double t = (rh * s) * sg_fma(-0.25, rh, SGK(CR_LOG_G3));
         const double y1 = sg_two_sum(h, u, &y1e);
         const double w = ue + t;
         /* w: rounding (2^-53), t's own error (< 2^-50 relative) and the
@@ -415,22 +415,22 @@ SG_HD double sg_log_cr(double x, const double* tab)
     const double se = sg_fma(rh, rh, -s);
     double he;
     const double h = sg_two_sum(rh, -0.5 * s, &he);
-    double p = sg_fma(rh, SG_CR_LOG_G11, SG_CR_LOG_G10);
-    p = sg_fma(rh, p, SG_CR_LOG_G9);
+    double p = sg_fma(rh, SGK(CR_LOG_G11), SGK(CR_LOG_G10));
+    p = sg_fma(rh, p, SGK(CR_LOG_G9));
     p = sg_fma(rh, p, SG_CR_LOG_G8);
-    p = sg_fma(rh, p, SG_CR_LOG_G7);
-    p = sg_fma(rh, p, SG_CR_LOG_G6);
-    p = sg_fma(rh, p, SG_CR_LOG_G5);
+    p = sg_fma(rh, p, SGK(CR_LOG_G7));
+    p = sg_fma(rh, p, SGK(CR_LOG_G6));
+    p = sg_fma(rh, p, SGK(CR_LOG_G5));
     p = sg_fma(rh, p, SG_CR_LOG_G4);
-    p = sg_fma(rh, p, SG_CR_LOG_G3);
+    p = sg_fma(rh, p, SGK(CR_LOG_G3));
     const double lo1 = he + (-0.5 * se + (sg_fma(-rl, rh, rl) + (s * rh) * p));
     /* + e ln2 - log(c) */
     const double ed = (double)e;
-    const double a = ed * SG_LOG_LN2_HI; /* exact */
+    const double a = ed * SGK(LOG_LN2_HI); /* exact */
     double t1, t2;
     const double s1 = sg_two_sum(a, lch, &t1);
     const double s2 = sg_two_sum(s1, h, &t2);
-    const double lo = ((t1 + t2) + (lcl + ed * SG_LOG_LN2_LO)) + lo1;
+    const double lo = ((t1 + t2) + (lcl + ed * SGK(LOG_LN2_LO))) + lo1;
     const double yh = sg_fast_two_sum(s2, lo, &yl);
     if (sg_cr_round(yh, yl, SG_CR_EPS_LOG, &y))
         return y;

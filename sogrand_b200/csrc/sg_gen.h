@@ -44,7 +44,7 @@ SG_HD double sg_sym_unit(uint64_t r)
  * rejected with probability 1 - pi/4; after SG_POLAR_TRIES rejections in a
  * row (probability < 1e-42) the sample is 0. */
 #define SG_POLAR_TRIES 64
-SG_HD double sg_normal(uint64_t seed, uint64_t c, uint32_t p, const double* ltab)
+SG_HD double sg_normal(uint64_t seed, uint64_t c, uint32_t p, SgTab ltab)
 {
     uint64_t ctr = c * 4096u + p;
     /* draw until a pair lands inside the unit disc; the transform runs once,
@@ -79,7 +79,7 @@ SG_HD double sg_normal(uint64_t seed, uint64_t c, uint32_t p, const double* ltab
 /* Noise deviation of codeword c when Eb/N0 is drawn uniformly from
  * [lo, hi] dB: sigma = 1/sqrt(10^(EsN0/10)), EsN0 = EbN0 + 10*log10(2R),
  * R = 1/8 (channel_sim.c:34-39), with 10^x = exp(x*ln 10) by sg_exp. */
-SG_HD double sg_sigma_draw(uint64_t seed, uint64_t c, double lo, double hi, const double* etab)
+SG_HD double sg_sigma_draw(uint64_t seed, uint64_t c, double lo, double hi, SgTab etab)
 {
     double u = (double)(sg_rand(seed, 7, c) >> 11) * 0x1p-53;
     double eb = lo + (hi - lo) * u;

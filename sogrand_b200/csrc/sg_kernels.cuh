@@ -1,0 +1,501 @@
+/* sg_kernels.cuh -- the decoder kernels, instantiated by sg_api.cu with the
+ * table-driven exp/log and by sg_cr.cu with the correctly rounded ones.  The
+ * two are separate translation units because the compiler's register
+ * allocation of one set moved with the other's code (the table-driven
+ * decoders by up to 13 %).
+ *
+ *   sg_decode_kernel   the whole iterative decode of a codeword per CTA
+ *                      (SOGRAND_C/cubic_decoder_final.c:119-289): the
+ *                      extrinsic cube stays in shared memory for all
+ *                      iterations, the channel cube too (one bulk
+ *                      asynchronous copy, cp.async.bulk on an mbarrier) or in
+ *                      L2; the warps take the 256 lines of a phase from a
+ *                      shared counter and decode one line each
+ *                      (sg_line.cuh); after every phase one warp runs the
+ *                      early-termination test on the 256 hard-decision words.
+ *   sg_persist_kernel  the batched form (sg_persist.cuh)
+ *   sg_bitso_kernel    SOGRAND_bitSO on independent lines, one warp per line.
+ *
+ * Built with -fmad=false: no floating-point contraction anywhere, as in the
+ * reference's plain gcc build; the exp/log routines use explicit FMAs.
+ */
+#pragma once
+#include <cuda_runtime.h>
+#include <stddef.h>
+
+#include "../../include/sogrand_b200.h"
+#include "sg_code.h"
+#include "sg_enum.h"
+#include "sg_line.cuh"
+#include "sg_line16.cuh"
+#include "sg_math.h"
+
+#define SG_THREADS 256
+#define SG_WARPS (SG_THREADS / 32)
+/* Bounded device-side waits.  The limit of a wait that can give up (the
+ * bulk-copy wait here, the persistent decoder's idle rounds) is a launch
+ * argument, SG_WAIT_LIMIT_DEFAULT unless sg_set_wait_limit() changed it.
+ * After a bulk-copy wait gave up, the copy may still be writing into the
+ * CTA's shared memory: the CTA waits for it again, up to SG_DRAIN_LIMIT
+ * polls, before it releases that memory. */
+#define SG_WAIT_LIMIT_DEFAULT (1ll << 22)
+#define SG_DRAIN_LIMIT (1ll << 26)
+
+static __device__ const double g_etab[SG_EXP_TAB_LEN] = SG_EXP_TAB_INIT;
+static __device__ const double g_ltab[SG_LOG_TAB_LEN] = SG_LOG_TAB_INIT;
+
+/* ------------------------------------------------------------ device -- */
+
+struct SgDecodeArgs {
+    const double* llr;
+    uint8_t* bits;
+    double* lapp;
+    sg_cw_stats* stats;
+    const uint32_t* enum_tabs;
+    unsigned int* err;
+    double* ckpt; /* nullable: [n_cw][3*imax][4096], L_E entering each phase */
+    unsigned long long n_cw;
+    long long wait_limit; /* polls or idle rounds before a bounded wait gives up */
+    int32_t L;
+    int32_t imax;
+    int32_t use_bulk;
+    int32_t pad;
+    double thres;
+    double alpha[SG_MAX_PHASES];
+    SgK k; /* constants of exp and log */
+    sg_order_meta meta;
+};
+
+/* Poll the mbarrier for phase `parity` at most `limit` times; 1 when it
+ * completed. */
+__device__ __forceinline__ uint32_t sg_mbar_wait(uint32_t mbar, uint32_t parity, long long limit)
+{
+    uint32_t ok = 0;
+    for (long long it = 0; it < limit && !ok; it++) {
+        asm volatile(
+            "{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
+            : "=r"(ok)
+            : "r"(mbar), "r"(parity)
+            : "memory");
+    }
+    return ok;
+}
+
+/* Outputs of a codeword that is not decoded: zero bits and statistics with
+ * the given converged code (-1 non-finite input, -2 a wait gave up).
+ * Called by the whole CTA. */
+__device__ __forceinline__ void sg_cw_not_decoded(const SgDecodeArgs& args, unsigned long long cw, int code)
+{
+    if (threadIdx.x < SG_INFO_BYTES)
+        args.bits[cw * SG_INFO_BYTES + threadIdx.x] = 0;
+    if (threadIdx.x == 0 && args.stats) {
+        sg_cw_stats st;
+        st.iterations = 0;
+        st.ng = 0;
+        st.ng_p = 0;
+        st.converged = code;
+        st.phases = 0;
+        args.stats[cw] = st;
+    }
+}
+
+/* Shared memory of a decode CTA.  With LCH_SMEM the channel cube is staged
+ * here by one bulk copy; otherwise each line reads its 16 channel LLRs from
+ * global memory (L2-resident) once per phase. */
+template <int NW, bool LCH_SMEM, int LPW = 1> /* LPW: lines decoded per warp at a time */
+struct SgCwSmem {
+    alignas(16) double lch[LCH_SMEM ? SG_CUBE : 2]; /* bulk-copy destination */
+    double le[SG_CUBE];
+    /* eight copies where the configuration's CTAs per SM still fit */
+    static constexpr bool T8 = NW * LPW >= 16 && !LCH_SMEM;
+    SgEtab<T8> etab;
+    alignas(16) double ltab[SG_LOG_TAB_LEN];
+    SgExpK ek;
+    SgWarpScratch ws[NW * LPW];
+    uint16_t hdw[256];
+    unsigned long long mbar;
+    unsigned long long ng;
+    unsigned int ngmax;
+    int line_next;
+    int conv;
+    int bad;
+};
+
+/* Cube index of bit `i` of line `l` in phase `axis` (lines of the reference's
+ * column phase run along the stride-1 index, rows along stride 16, slices
+ * along stride 256; cubic_decoder_final.c:157-247). */
+__device__ __forceinline__ int sg_pos(int axis, int l, int i)
+{
+    const int a = l >> 4, b = l & 15;
+    if (axis == 0)
+        return a * 256 + b * 16 + i;
+    if (axis == 1)
+        return a * 256 + i * 16 + b;
+    return i * 256 + a * 16 + b;
+}
+
+/* Early termination (cubic_decoder_final.c:317-391) on the 256 line words
+ * of the phase just run: the hard decisions form a product codeword iff
+ * every word is a component codeword and the words satisfy the component
+ * parity equations along both other axes (bitwise).  Warp-wide. */
+__device__ __forceinline__ bool sg_is_codeword(const uint16_t* hdw, int lane)
+{
+    bool bad = false;
+    for (int q = lane; q < 256; q += 32) {
+        const uint32_t x = hdw[q];
+        bad |= ((x >> 8) & 0xffu) != c_ptab[x & 0xffu];
+    }
+    for (int q = lane; q < 128; q += 32) {
+        const int a = q >> 3, j = q & 7;
+        uint32_t acc = 0;
+#pragma unroll
+        for (int b = 0; b < 8; b++)
+            if ((c_prow[b] >> j) & 1u)
+                acc ^= hdw[a * 16 + b];
+        bad |= acc != hdw[a * 16 + 8 + j];
+    }
+    for (int q = lane; q < 128; q += 32) {
+        const int b = q >> 3, j = q & 7;
+        uint32_t acc = 0;
+#pragma unroll
+        for (int a = 0; a < 8; a++)
+            if ((c_prow[a] >> j) & 1u)
+                acc ^= hdw[a * 16 + b];
+        bad |= acc != hdw[(8 + j) * 16 + b];
+    }
+    return !__any_sync(SG_FULL, bad);
+}
+
+__device__ __forceinline__ uint32_t sg_smem_u32(const void* p)
+{
+    return (uint32_t)__cvta_generic_to_shared(p);
+}
+
+extern __shared__ __align__(1024) unsigned char sg_smem_raw[];
+
+template <int NW, bool LCH_SMEM, int MINB, int G, bool CR, int LPW = 1>
+__global__ void __launch_bounds__(NW * 32, MINB) sg_decode_kernel(const __grid_constant__ SgDecodeArgs args)
+{
+    constexpr int NT = NW * 32;
+    SgCwSmem<NW, LCH_SMEM, LPW>& S = *reinterpret_cast<SgCwSmem<NW, LCH_SMEM, LPW>*>(sg_smem_raw);
+    constexpr bool T8 = SgCwSmem<NW, LCH_SMEM, LPW>::T8;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const bool use_bulk = LCH_SMEM && args.use_bulk;
+    sg_etab_fill<CR, T8>(S.etab, g_etab, tid, NT);
+    for (int i = tid; i < SG_LOG_TAB_LEN; i += NT)
+        S.ltab[i] = g_ltab[i];
+    if (tid == 0)
+        S.ek = sg_exp_k();
+    const uint32_t mbar = sg_smem_u32(&S.mbar);
+    if (tid == 0 && use_bulk) {
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(mbar) : "memory");
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    __syncthreads();
+    uint32_t phase_bit = 0;
+    const SgTab etab = sg_etab_of<CR, T8>(S.etab, args.k.v), ltab{S.ltab, args.k.v};
+    SgLineParams lp;
+    lp.L = args.L;
+    lp.meta = &args.meta;
+    lp.ek = &S.ek;
+    lp.thres = args.thres;
+
+    for (unsigned long long cw = blockIdx.x; cw < args.n_cw; cw += gridDim.x) {
+        const double* g = args.llr + cw * SG_CUBE;
+        if (use_bulk) {
+            if (tid == 0) {
+                /* order earlier generic-proxy reads of lch before the async write */
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(mbar),
+                             "r"((uint32_t)(SG_CUBE * 8))
+                             : "memory");
+                asm volatile(
+                    "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                        sg_smem_u32(S.lch)),
+                    "l"(g), "r"((uint32_t)(SG_CUBE * 8)), "r"(mbar)
+                    : "memory");
+            }
+        } else if (LCH_SMEM) {
+            for (int i = tid; i < SG_CUBE; i += NT)
+                S.lch[i] = g[i];
+        }
+        for (int i = tid; i < SG_CUBE; i += NT)
+            S.le[i] = 0.0;
+        if (tid == 0) {
+            S.ng = 0;
+            S.conv = 0;
+            S.bad = 0;
+        }
+        if (use_bulk && tid == 0) {
+            if (!sg_mbar_wait(mbar, phase_bit, args.wait_limit)) {
+                /* gave up: report it, then let the copy land before this
+                 * CTA's shared memory is reused or released */
+                atomicOr(args.err, 1u);
+                if (!sg_mbar_wait(mbar, phase_bit, SG_DRAIN_LIMIT))
+                    atomicOr(args.err, 2u);
+                S.bad = 2;
+            }
+        }
+        phase_bit ^= 1u;
+        __syncthreads();
+        if (S.bad == 2) {
+            /* this codeword and the CTA's later ones are reported as not
+             * decoded (converged = -2) */
+            for (unsigned long long c = cw; c < args.n_cw; c += gridDim.x)
+                sg_cw_not_decoded(args, c, -2);
+            return;
+        }
+        bool nonfinite = false;
+        for (int i = tid; i < SG_CUBE; i += NT)
+            nonfinite |= !isfinite(LCH_SMEM ? S.lch[i] : __ldg(g + i));
+        if (__syncthreads_or(nonfinite)) {
+            sg_cw_not_decoded(args, cw, -1);
+            __syncthreads();
+            continue;
+        }
+
+        int phases = 0;
+        unsigned long long ng_p = 0;
+        int axis_last = 0;
+        bool conv = false;
+        for (int iter = 1; iter <= args.imax && !conv; iter++) {
+            for (int axis = 0; axis < 3 && !conv; axis++) {
+                const double alpha = args.alpha[3 * (iter - 1) + axis];
+                if (tid == 0) {
+                    S.line_next = 0;
+                    S.ngmax = 0;
+                }
+                __syncthreads();
+                if constexpr (LPW == 2) {
+                    /* the warp takes two lines at a time, one per half, and
+                     * decodes them in lockstep (sg_line16.cuh) */
+                    const int hb = lane & 16, sl = lane & 15;
+                    SgWarpScratch* wsl = &S.ws[2 * warp + (hb >> 4)];
+                    for (;;) {
+                        int l = 0;
+                        if (lane == 0)
+                            l = atomicAdd(&S.line_next, 2);
+                        l = __shfl_sync(SG_FULL, l, 0) + (hb >> 4);
+                        if (l >= 256) /* 256 lines: both halves leave together */
+                            break;
+                        const int pos = sg_pos(axis, l, sl);
+                        const double le0 = S.le[pos];
+                        const double v = __dadd_rn(LCH_SMEM ? S.lch[pos] : __ldg(g + pos), __dmul_rn(alpha, le0));
+                        if (args.ckpt)
+                            args.ckpt[(cw * (3ull * args.imax) + 3 * (iter - 1) + axis) * SG_CUBE + pos] = le0;
+                        const SgLineResult r = sg_decode_line16<G, CR>(v, lp, args.enum_tabs, etab, ltab, wsl);
+                        S.le[pos] = r.le;
+                        if (args.lapp)
+                            args.lapp[cw * SG_CUBE + pos] = r.lapp;
+                        if (sl == 0) {
+                            S.hdw[l] = (uint16_t)r.hdword;
+                            atomicAdd(&S.ng, (unsigned long long)r.T);
+                            atomicMax(&S.ngmax, r.T);
+                        }
+                    }
+                } else {
+                    for (;;) {
+                        int l = 0;
+                        if (lane == 0)
+                            l = atomicAdd(&S.line_next, 1);
+                        l = __shfl_sync(SG_FULL, l, 0);
+                        if (l >= 256)
+                            break;
+                        const int pos = sg_pos(axis, l, lane & 15);
+                        double v = 1.0;
+                        if (lane < 16) { /* L_ch + (alpha*L_E) */
+                            v = __dadd_rn(LCH_SMEM ? S.lch[pos] : __ldg(g + pos), __dmul_rn(alpha, S.le[pos]));
+                            if (args.ckpt)
+                                args.ckpt[(cw * (3ull * args.imax) + 3 * (iter - 1) + axis) * SG_CUBE + pos] = S.le[pos];
+                        }
+                        const SgLineResult r =
+                            sg_decode_line<false, CR, T8>(v, lp, args.enum_tabs, etab, ltab, &S.ws[warp]);
+                        if (lane < 16) {
+                            S.le[pos] = r.le;
+                            if (args.lapp)
+                                args.lapp[cw * SG_CUBE + pos] = r.lapp;
+                        }
+                        if (lane == 0) {
+                            S.hdw[l] = (uint16_t)r.hdword;
+                            atomicAdd(&S.ng, (unsigned long long)r.T);
+                            atomicMax(&S.ngmax, r.T);
+                        }
+                    }
+                }
+                __syncthreads();
+                phases++;
+                axis_last = axis;
+                ng_p += S.ngmax;
+                if (warp == 0) {
+                    const bool c = sg_is_codeword(S.hdw, lane);
+                    if (lane == 0)
+                        S.conv = c;
+                }
+                __syncthreads();
+                conv = S.conv != 0;
+            }
+        }
+
+        /* hard_decision (:393-415): info bit b = s*64 + r*8 + c is the sign of
+         * L_APP at cube index s*256 + r*16 + c; packed MSB first (:272-280) */
+        if (tid < SG_INFO_BYTES) {
+            uint32_t byte = 0;
+            for (int q = 0; q < 8; q++) {
+                const int b = tid * 8 + q;
+                const int p = (b >> 6) * 256 + ((b >> 3) & 7) * 16 + (b & 7);
+                int l, bit;
+                if (axis_last == 0) {
+                    l = (p >> 8) * 16 + ((p >> 4) & 15);
+                    bit = p & 15;
+                } else if (axis_last == 1) {
+                    l = (p >> 8) * 16 + (p & 15);
+                    bit = (p >> 4) & 15;
+                } else {
+                    l = ((p >> 4) & 15) * 16 + (p & 15);
+                    bit = p >> 8;
+                }
+                byte = (byte << 1) | ((S.hdw[l] >> bit) & 1u);
+            }
+            args.bits[cw * SG_INFO_BYTES + tid] = (uint8_t)byte;
+        }
+        if (tid == 0 && args.stats) {
+            sg_cw_stats st;
+            st.iterations = 0.5 * phases;
+            st.ng = S.ng;
+            st.ng_p = ng_p;
+            st.converged = conv ? 1 : 0;
+            st.phases = phases;
+            args.stats[cw] = st;
+        }
+        __syncthreads();
+    }
+}
+
+#include "sg_persist.cuh"
+
+struct SgLineSmem {
+    SgEtab<false> etab;
+    alignas(16) double ltab[SG_LOG_TAB_LEN];
+    SgExpK ek;
+    SgWarpScratch ws[SG_WARPS];
+};
+
+template <bool CR>
+__global__ void __launch_bounds__(SG_THREADS) sg_bitso_kernel(const double* __restrict__ llr,
+                                                               unsigned long long n_lines,
+                                                               int32_t L, double thres, double* lapp, double* le,
+                                                               int32_t* nguess, int32_t* ncw,
+                                                               const uint32_t* enum_tabs,
+                                                               const __grid_constant__ SgK k,
+                                                               const __grid_constant__ sg_order_meta meta)
+{
+    __shared__ SgLineSmem S;
+    const SgTab etab = sg_etab_of<CR, false>(S.etab, k.v), ltab{S.ltab, k.v};
+    const SgLineParams lp{L, thres, &meta, &S.ek};
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    sg_etab_fill<CR, false>(S.etab, g_etab, tid, SG_THREADS);
+    for (int i = tid; i < SG_LOG_TAB_LEN; i += SG_THREADS)
+        S.ltab[i] = g_ltab[i];
+    if (tid == 0)
+        S.ek = sg_exp_k();
+    __syncthreads();
+    for (unsigned long long l = (unsigned long long)blockIdx.x * SG_WARPS + warp; l < n_lines;
+         l += (unsigned long long)gridDim.x * SG_WARPS) {
+        const double v = lane < 16 ? llr[l * 16 + lane] : 1.0;
+        if (__any_sync(SG_FULL, !isfinite(v))) { /* not decoded: NaN out, N_guess -1 */
+            if (lane < 16) {
+                lapp[l * 16 + lane] = __longlong_as_double(0x7ff8000000000000ll);
+                le[l * 16 + lane] = __longlong_as_double(0x7ff8000000000000ll);
+            }
+            if (lane == 0) {
+                nguess[l] = -1;
+                if (ncw)
+                    ncw[l] = 0;
+            }
+            continue;
+        }
+        const SgLineResult r = sg_decode_line<false, CR, false>(v, lp, enum_tabs, etab, ltab, &S.ws[warp]);
+        if (lane < 16) {
+            lapp[l * 16 + lane] = r.lapp;
+            le[l * 16 + lane] = r.le;
+        }
+        if (lane == 0) {
+            nguess[l] = (int32_t)r.T;
+            if (ncw)
+                ncw[l] = r.ncw;
+        }
+    }
+}
+
+/* SG_TU_CR: the math of this translation unit's instantiations. */
+#ifndef SG_TU_CR
+#define SG_TU_CR false
+#endif
+
+/* Decoder kernel configurations: warps per codeword CTA, channel cube in
+ * shared memory (bulk copy) or read from global memory, minimum resident
+ * CTAs per SM for the register budget, and lines per warp (1: 32 lanes per
+ * line, sg_line.cuh; 2: 16 lanes per line and G patterns per lane,
+ * sg_line16.cuh).  The "-g2" names of one-line configurations date from a
+ * guess loop with two patterns per lane; they are the same kernels. */
+struct SgVariant {
+    const char* name;
+    int nw;
+    bool lch_smem;
+    size_t smem;
+    const void* fn;
+};
+
+#define SG_VARIANT(NW, L, M, NAME) \
+    { NAME, NW, L, sizeof(SgCwSmem<NW, L>), (const void*)sg_decode_kernel<NW, L, M, 1, SG_TU_CR> }
+#define SG_VARIANT_L2(NW, M, G, NAME) \
+    { NAME, NW, false, sizeof(SgCwSmem<NW, false, 2>), (const void*)sg_decode_kernel<NW, false, M, G, SG_TU_CR, 2> }
+static const SgVariant k_variants[] = {
+    SG_VARIANT(8, false, 3, "w8-gmem"),
+    SG_VARIANT(8, true, 2, "w8-smem"),
+    SG_VARIANT(12, true, 2, "w12-smem"),
+    SG_VARIANT(16, false, 2, "w16-gmem"),
+    SG_VARIANT(16, false, 2, "w16-gmem-g2"),
+    SG_VARIANT(8, false, 3, "w8-gmem-g2"),
+    SG_VARIANT(12, true, 2, "w12-smem-g2"),
+    SG_VARIANT_L2(8, 2, 2, "w8-l2-g2"),
+    SG_VARIANT_L2(8, 2, 4, "w8-l2-g4"),
+    SG_VARIANT_L2(10, 1, 2, "w10-l2-g2"),
+    SG_VARIANT_L2(16, 1, 2, "w16-l2-g2"),
+};
+#define SG_NVARIANTS ((int)(sizeof(k_variants) / sizeof(k_variants[0])))
+
+/* Batched persistent decoder configurations: warps per CTA (one CTA per
+ * SM), codeword slots per CTA. */
+struct SgPVariant {
+    const char* name;
+    int nw;
+    int slots;
+    size_t smem;
+    const void* fn;
+};
+#define SG_PVARIANT(NW, C, NAME) \
+    { NAME, NW, C, sizeof(SgPersistSmem<NW, C>), (const void*)sg_persist_kernel<NW, C, SG_TU_CR> }
+static const SgPVariant k_pvariants[] = {
+    SG_PVARIANT(24, 3, "p24x3"),
+    SG_PVARIANT(28, 3, "p28x3"),
+    SG_PVARIANT(16, 3, "p16x3"),
+    SG_PVARIANT(20, 4, "p20x4"),
+    SG_PVARIANT(32, 3, "p32x3"),
+    SG_PVARIANT(32, 3, "p32x3-g2"),
+    SG_PVARIANT(24, 3, "p24x3-g2"),
+    SG_PVARIANT(28, 3, "p28x3-g2"),
+};
+#define SG_NPVARIANTS ((int)(sizeof(k_pvariants) / sizeof(k_pvariants[0])))
+
+
+/* The code tables, for this translation unit's kernels. */
+static cudaError_t sg_load_code(const sg_code_tables& code)
+{
+    cudaError_t e = cudaMemcpyToSymbol(c_hcol, code.hcol, sizeof code.hcol);
+    if (e == cudaSuccess)
+        e = cudaMemcpyToSymbol(c_prow, code.prow, sizeof code.prow);
+    if (e == cudaSuccess)
+        e = cudaMemcpyToSymbol(c_ptab, code.ptab, sizeof code.ptab);
+    return e;
+}

@@ -17,23 +17,34 @@
  *             synlo/hi  syndrome of each byte of a pattern (ParityCheck,
  *                       :748-755, is linear), the hard decision's own
  *                       syndrome folded into synlo.
- *  guesses  32*G consecutive patterns of the order table per step, G per
+ *  guesses  32 consecutive patterns of the order table per step, one per
  *           lane: PM = A[lo] + increments of the high bits (ascending),
  *           syndrome = synlo[lo] ^ synhi[hi], e = exp(-PM).
  *  P_notGuess  the reference subtracts e of every guess in order (:626,
- *           :672, :712).  Within one binade [2^E, 2^(E+1)) every difference
- *           rounds to the grid u = 2^(E-52), so fl(P - e) = u*round(M - e/u)
- *           with M = P/u an integer: when a step holds no codeword and no
- *           lane's term is large, ties, or leaves the binade, the running
- *           value after the step is M minus the warp's exact integer sum
- *           (two 32-bit warp reductions of the terms' 26-bit halves).
- *           Every other step replays the reference's sequence itself: the
- *           32 terms are staged in shared memory and every lane performs the
- *           32 IEEE subtractions in order.  The result equals the sequential
- *           loop bit for bit.
+ *           :672, :712).  Within one binade every difference rounds to the
+ *           binade's grid, so a step without codeword, exact tie or binade
+ *           crossing moves P's bit pattern by the warp's exact integer sum of
+ *           the rounded terms (SgGrid).  A step with codewords only takes the
+ *           sum up to each of them; any other step replays the reference's
+ *           sequence from shared memory, every lane performing the 32 IEEE
+ *           subtractions in order.  The result equals the sequential loop
+ *           bit for bit.
  *  list     codewords are taken in lane order; getLConf (:767-774) uses the
  *           running P_notGuess at each, so T and the list match exactly.
  *  output   soft output of :536-577 on lanes 0..15.
+ *
+ * What bounds it: issue slots and shared-memory cycles, about evenly (of
+ * 23 steps per line decode at 2 dB, 15 end in the sum, 2 hold codewords, 6
+ * are replayed).  Per line decode at 2 dB, B200 counters: 4 720 warp
+ * instructions and 1 010 shared-memory cycles with the former loop of two
+ * patterns per lane (steps of 64, of which half had to be replayed, term
+ * rounding tested by difference, an exp from one table copy); 3 300 and 780
+ * with this one.  20 000 codewords at 2 dB, batched form: 245.8 -> 202.1 ms;
+ * 8 000, plain form: 101.2 -> 84.0 ms; 2 000 at 1 dB under Tmax 1000: 146.5
+ * -> 97.5 ms; correctly rounded math, 4 000 at 2 dB: 68.3 -> 60.0 ms.
+ * Steps of 64 patterns were slower once the sum was cheap (229 ms): a step
+ * twice as long is summed half as often, and has to be looked at again by
+ * halves.
  * The file is built with -fmad=false: every floating-point operation the
  * reference performs is a separately rounded IEEE operation here.
  */
@@ -51,22 +62,106 @@
  * with which every result equals the reference's under a correctly rounded
  * libm, at about 2x the cost per exp. */
 template <bool CR>
-__device__ __forceinline__ double sg_dec_exp(double x, const double* tab)
+__device__ __forceinline__ double sg_dec_exp(double x, SgTab tab)
 {
     return CR ? sg_exp_cr(x, tab) : sg_exp(x, tab);
 }
 template <bool CR>
-__device__ __forceinline__ double sg_dec_exp_neg(double x, const double* tab)
+__device__ __forceinline__ double sg_dec_exp_neg(double x, SgTab tab)
 {
     return CR ? sg_exp_cr_neg(x, tab) : sg_exp_neg(x, tab);
 }
 template <bool CR>
-__device__ __forceinline__ double sg_dec_log(double x, const double* tab)
+__device__ __forceinline__ double sg_dec_log(double x, SgTab tab)
 {
     return CR ? sg_log_cr(x, tab) : sg_log(x, tab);
 }
 
 #define SG_FULL 0xffffffffu
+
+/* Shared-memory loads at a 32-bit shared address.  Plain C++ accesses add
+ * the kernel's shared base to every index; the guess loop's addresses hold
+ * it already. */
+__device__ __forceinline__ uint32_t sg_saddr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+template <int OFF>
+__device__ __forceinline__ double sg_lds_f64(uint32_t a)
+{
+    double v;
+    asm volatile("ld.shared.f64 %0, [%1 + %2];" : "=d"(v) : "r"(a), "n"(OFF));
+    return v;
+}
+template <int OFF>
+__device__ __forceinline__ uint32_t sg_lds_u8(uint32_t a)
+{
+    uint32_t v;
+    asm volatile("ld.shared.u8 %0, [%1 + %2];" : "=r"(v) : "r"(a), "n"(OFF));
+    return v;
+}
+__device__ __forceinline__ double2 sg_lds_f64x2(uint32_t a)
+{
+    double2 v;
+    asm volatile("ld.shared.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "r"(a));
+    return v;
+}
+
+/* The constants of sg_exp_neg, read from the kernel's shared memory copy
+ * once per line: a value that came from memory stays in its registers
+ * through the guess loop. */
+struct alignas(16) SgExpK {
+    double inv, ln2_hi, ln2_lo, c3, c4, c5, c6, c7;
+};
+__device__ __forceinline__ SgExpK sg_exp_k()
+{
+    return {SG_EXP_INV_LN2_N, SG_EXP_LN2_N_HI, SG_EXP_LN2_N_LO, SG_EXP_C3, SG_EXP_C4, SG_EXP_C5, SG_EXP_C6, SG_EXP_C7};
+}
+
+/* A kernel's exp table in shared memory: T8 -- eight copies, with the
+ * adjusted H_j for the table-driven exp (sg_math.h); otherwise one. */
+template <bool T8>
+struct SgEtab {
+    static constexpr int len = T8 ? 8 * SG_EXP_TAB_LEN : SG_EXP_TAB_LEN;
+    alignas(16) double d[len];
+};
+template <bool CR, bool T8>
+__device__ __forceinline__ void sg_etab_fill(SgEtab<T8>& dst, const double* src, int tid, int nt)
+{
+    for (int i = tid; i < SgEtab<T8>::len; i += nt) {
+        const int j = T8 ? i >> 4 : i >> 1;
+        double v = src[2 * j + (i & 1)];
+        if (T8 && !CR && !(i & 1))
+            v = sg_from_bits(sg_bits(v) - ((uint64_t)j << 45));
+        dst.d[i] = v;
+    }
+}
+template <bool CR, bool T8>
+__device__ __forceinline__ SgTab sg_etab_of(const SgEtab<T8>& tab, const double* k)
+{
+    return {tab.d + (T8 ? 2 * (threadIdx.x & 7) : 0), k, T8 ? 16 : 2, T8 && !CR};
+}
+
+/* exp(x) for x in [-707.5, 0]: sg_exp_neg's operations with the constants
+ * of k and the lane's copy of the table (its shared address). */
+__device__ __forceinline__ double sg_exp_neg_k(double x, uint32_t tab, const SgExpK& k)
+{
+    const double z = __dmul_rn(x, k.inv);
+    double kd = __dadd_rn(z, SG_EXP_SHIFT);
+    const int n = __double2loint(kd);
+    kd = __dsub_rn(kd, SG_EXP_SHIFT);
+    double r = __fma_rn(-kd, k.ln2_hi, x);
+    r = __fma_rn(-kd, k.ln2_lo, r);
+    const double2 Ht = sg_lds_f64x2(tab + (uint32_t)(n & 127) * 128u);
+    const double r2 = __dmul_rn(r, r);
+    double p = __fma_rn(r, k.c7, k.c6);
+    p = __fma_rn(r, p, k.c5);
+    p = __fma_rn(r, p, k.c4);
+    p = __fma_rn(r, p, k.c3);
+    p = __fma_rn(r, p, SG_EXP_C2);
+    p = __dmul_rn(p, r2);
+    const double u = __fma_rn(Ht.y, r, Ht.y);
+    const double tmp = __dadd_rn(r, __dadd_rn(u, p));
+    const double S = __hiloint2double(__double2hiint(Ht.x) + (n << 13), __double2loint(Ht.x));
+    return __fma_rn(S, tmp, S);
+}
 
 template <bool B>
 struct SgBoolTag {
@@ -75,43 +170,49 @@ struct SgBoolTag {
 
 struct SgLineParams {
     int32_t L;
-    uint32_t tmax;     /* Tmax clamped to 2^32-1 (T never exceeds 65536) */
     double thres;
+    const sg_order_meta* meta; /* per IC, Tmax included */
+    const SgExpK* ek;          /* shared memory copy */
 };
 
 /* Per-warp shared scratch of one line decode. */
 #define SG_LIST_MAX 8 /* SG_MAX_L of the C ABI; the entry points reject larger L */
 
-struct alignas(16) SgWarpScratch { /* A is read as double2 */
+/* Every record starts at a multiple of 256 bytes: the guess loop puts an
+ * entry's byte into the low byte of the record's shared address to address
+ * the tables below (A by a scaled index). */
+struct alignas(256) SgWarpScratch {
     double A[256];      /* PM prefix over the low byte of a pattern, entry lo
                            stored at sg_swz(lo) */
-    double dz[16];      /* dz[0] = 0, dz[1 + j] = PM increment of sorted
-                           position 8 + j (j < 8), the rest 0; indexed by the
-                           byte offsets of an order-table entry */
-    double qa[16];      /* values for the tie-exact sort, then the input LLRs */
-    double ex[16];      /* exp(input LLR) of each position, for the soft output */
-    double es[32];      /* general case: exp(-PM) of the 32 patterns of a half */
-    double ps[32];      /* general case: P_notGuess after each of them */
-    int32_t perm[16];   /* sorted rank -> position */
-    int32_t rank[16];   /* position -> sorted rank */
     uint8_t synlo[256]; /* syndrome of the low byte (and of the hard decision),
                            entry lo stored at sg_swz(lo) */
     uint8_t synhi[256]; /* syndrome of the high byte */
+    double dz[9];       /* dz[0] = 0, dz[1 + j] = PM increment of sorted
+                           position 8 + j; indexed by the byte offsets of an
+                           order-table entry */
     /* the list (touched only at codewords and in the soft output, so it
-     * lives here rather than in registers): entry k = exp(-PM) of the k-th
-     * codeword found and its bits (bit i = position i) */
+     * lives here rather than in registers): entry k = exp(-PM) and pattern
+     * (bit r = sorted position r) of the k-th codeword found */
     double lst_e[SG_LIST_MAX];
-    uint32_t lst_cm[SG_LIST_MAX];
+    double ppos;        /* sum of lst_e in order */
+    uint32_t lst_m[SG_LIST_MAX];
     double pnl;         /* pNL of the last getLConf */
     int32_t curl;       /* codewords listed */
     uint32_t hdm;       /* hard decision, bit i = position i */
+    int32_t itab;       /* order table of the line's IC */
+    uint8_t rank[16];   /* position -> sorted rank */
+    uint8_t perm[16];   /* sorted rank -> position */
+    alignas(256) double es[32]; /* replay: exp(-PM) of the 32 patterns of a step */
+    double qa[16];      /* values for the tie-exact sort, then the input LLRs */
+    double ex[16];      /* exp(input LLR) of each position, for the soft output */
 };
-static_assert(offsetof(SgWarpScratch, synlo) % 8 == 0 && offsetof(SgWarpScratch, synhi) % 8 == 0,
-              "syndrome tables are written 8 bytes at a time");
+static_assert(offsetof(SgWarpScratch, synlo) == 2048 && offsetof(SgWarpScratch, synhi) == 2304 &&
+                  offsetof(SgWarpScratch, dz) == 2560 && sizeof(SgWarpScratch) == 3328,
+              "tables addressed by a byte in the record's address");
 
-__constant__ uint8_t c_hcol[16];
-__constant__ uint8_t c_prow[8];
-__constant__ uint8_t c_ptab[256];
+static __constant__ uint8_t c_hcol[16];
+static __constant__ uint8_t c_prow[8];
+static __constant__ uint8_t c_ptab[256];
 
 /* (int32_t) of a double as x86-64 cvttsd2si computes it: NaN and values
  * outside int32 give INT32_MIN (the reference casts round(...) at :621). */
@@ -127,7 +228,7 @@ __device__ __forceinline__ int32_t sg_cvt_i32(double v)
  * processing order of the stack does not change the result.  Run by one
  * lane, only when the line has tied reliabilities (a rank sort orders ties
  * differently). */
-__device__ __noinline__ void sg_quicksort16(double* a, int32_t* perm)
+static __device__ __noinline__ void sg_quicksort16(double* a, uint8_t* perm)
 {
     int32_t st_off[32], st_n[32];
     int sp = 0;
@@ -140,7 +241,7 @@ __device__ __noinline__ void sg_quicksort16(double* a, int32_t* perm)
         if (n < 2)
             continue;
         double* x = a + off;
-        int32_t* pm = perm + off;
+        uint8_t* pm = perm + off;
         double p = x[n / 2];
         int32_t i = 0, j = n - 1;
         while (i <= j) {
@@ -152,7 +253,7 @@ __device__ __noinline__ void sg_quicksort16(double* a, int32_t* perm)
                 double t = x[i];
                 x[i] = x[j];
                 x[j] = t;
-                int32_t tt = pm[i];
+                uint8_t tt = pm[i];
                 pm[i] = pm[j];
                 pm[j] = tt;
                 i++;
@@ -180,84 +281,128 @@ struct SgLineResult {
     int32_t ncw;      /* codewords found (all lanes) */
 };
 
-/* A codeword found at pattern mask `mj` (sorted positions) whose guess left
- * P_notGuess = P and contributed ej = exp(-PM): list insertion and getLConf
- * (:674-686, :767-774).  Returns true when the line decode stops. */
-__device__ __forceinline__ bool sg_list_hit(SgWarpScratch* ws, const SgLineParams& lp, uint32_t mj, double P,
-                                            double ej, int lane)
+/* The codeword of lane j, whose guess left P_notGuess = P: list insertion
+ * and getLConf (:674-686, :767-774), by that lane.  Returns true (all lanes)
+ * when the line decode stops.  The confidence ppos / (ppos + pneg) is
+ * divided out only within a few units of the threshold, where its rounding
+ * could matter; the products decide everywhere else. */
+__device__ __forceinline__ bool sg_list_hit(SgWarpScratch* ws, const SgLineParams& lp, uint32_t ent, double P, double e,
+                                            int j, int lane)
 {
-    /* AddTEP (:761): position i flips when its sorted rank is in the pattern */
-    const int myrank = lane < 16 ? ws->rank[lane] : 0;
-    const uint32_t cm = ws->hdm ^ (__ballot_sync(SG_FULL, lane < 16 && ((mj >> myrank) & 1u)) & 0xffffu);
     const int curl = ws->curl;
-    double ppos = 0.0;
-    for (int i = 0; i < curl; i++)
-        ppos = __dadd_rn(ppos, ws->lst_e[i]);
-    ppos = __dadd_rn(ppos, ej);
-    const double pneg = __dmul_rn(0x1p-8, P); /* 2^-(n-k) * P_notGuess */
+    bool stop = curl + 1 == lp.L;
     __syncwarp();
-    if (lane == 0) {
-        ws->lst_e[curl] = ej;
-        ws->lst_cm[curl] = cm;
+    if (lane == j) {
+        const double pneg = __dmul_rn(0x1p-8, P); /* 2^-(n-k) * P_notGuess */
+        const double ppos = __dadd_rn(ws->ppos, e);
+        ws->lst_e[curl] = e;
+        ws->lst_m[curl] = sg_ent_pattern(ent);
+        ws->ppos = ppos;
         ws->pnl = pneg;
         ws->curl = curl + 1;
+        if (!stop) {
+            const double den = __dadd_rn(ppos, pneg);
+            const double b = __dmul_rn(lp.thres, den), m = __fma_rn(fabs(b), 0x1p-50, 0x1p-900);
+            if (!(den > 1e-40))
+                stop = 1.0 > lp.thres;
+            else if (ppos > __dadd_rn(b, m))
+                stop = true;
+            else if (!(ppos < __dsub_rn(b, m)))
+                stop = __ddiv_rn(ppos, den) > lp.thres;
+        }
     }
     __syncwarp();
-    const double den = __dadd_rn(ppos, pneg);
-    const double conf = (den > 1e-40) ? __ddiv_rn(ppos, den) : 1.0;
-    return conf > lp.thres || curl + 1 == lp.L;
+    return __any_sync(SG_FULL, stop);
 }
 
-/* General case of one 32-pattern half (first pattern index bh, nv valid
- * patterns): the reference's own sequence P -= e (:626, :672, :712), one
- * IEEE subtraction per pattern in order, evaluated redundantly by every lane
- * from the terms staged in shared memory.  Exact whatever the step holds
- * (codewords, binade crossings, ties, large or tiny terms).  Terms of lanes
- * >= nv are finite and subtracted too: nv < 32 only when the line decode
- * ends in this half, after which P is not read.  With codewords in the half
- * P is recorded after every term, then the codewords are listed in order
- * with the P that followed each.  Sets T and done when the decode stops. */
-__device__ __forceinline__ void sg_seq_half(double e, uint32_t ent, uint32_t hits, uint32_t bh, double& P,
-                                            SgWarpScratch* ws, uint32_t& T, bool& done, const SgLineParams& lp,
-                                            int lane)
+/* P_notGuess in the guess loop.  P in [2^E, 2^(E+1)) has the grid
+ * u = 2^(E-52), and its binary64 bit pattern counts units of u: subtracting
+ * k*u subtracts k from the pattern.  Each lane rounds its term to the grid as
+ * P - e does by adding it to 2^E (s1) and to 2^E + u (s2).  The two start
+ * with different parity, so an exact tie (a term whose units end in 1/2,
+ * rounded to even) leaves them something else than one unit apart.
+ * SgGrid: the two addends of P's binade.  A P below 2^-970 or not positive
+ * has no such grid: infinities, whose sums never differ by one unit, send
+ * every step to the replay. */
+struct SgGrid {
+    double b1, b2;
+};
+
+__device__ __forceinline__ SgGrid sg_grid(uint64_t Pb)
+{
+    const int32_t ph = (int32_t)(Pb >> 32);
+    const int32_t hi = ph >= 0x03500000 ? (int32_t)(ph & 0xfff00000) : 0x7ff00000;
+    SgGrid g;
+    g.b1 = __hiloint2double(hi, 0);
+    g.b2 = __hiloint2double(hi, ph >= 0x03500000 ? 1 : 0);
+    return g;
+}
+
+/* The warp's sum of units given as 26-bit halves per lane. */
+__device__ __forceinline__ uint64_t sg_units_sum(uint32_t lo, uint32_t hi)
+{
+    const uint32_t tlo = __reduce_add_sync(SG_FULL, lo);
+    const uint32_t thi = __reduce_add_sync(SG_FULL, hi);
+    return (uint64_t)thi * (1u << 26) + tlo;
+}
+
+/* The reference's own sequence P -= e (:626, :672, :712) over a step's 32
+ * patterns, one IEEE subtraction per pattern in order, evaluated by every
+ * lane from the terms staged in shared memory: exact whatever the step
+ * holds.  With codewords (hits), P at each of them goes to the list.
+ * Returns true when one stops the decode, at pattern T of the line. */
+__device__ __forceinline__ bool sg_replay(double e, uint32_t ent, uint32_t hits, uint32_t base, uint64_t& Pb,
+                                          SgWarpScratch* ws, uint32_t& T, const SgLineParams& lp, int lane)
 {
     ws->es[lane] = e;
     __syncwarp();
-    const double2* e2 = reinterpret_cast<const double2*>(ws->es);
-    double p = P;
+    double p = sg_from_bits(Pb);
     if (!hits) {
+        const double2* e2 = reinterpret_cast<const double2*>(ws->es);
 #pragma unroll
-        for (int k = 0; k < 16; k++) {
-            const double2 v = e2[k];
+        for (int q = 0; q < 16; q++) {
+            const double2 v = e2[q];
             p = __dsub_rn(p, v.x);
             p = __dsub_rn(p, v.y);
         }
-        P = p;
     } else {
-        double2* p2 = reinterpret_cast<double2*>(ws->ps);
-#pragma unroll
-        for (int k = 0; k < 16; k++) {
-            const double2 v = e2[k];
-            const double p0 = __dsub_rn(p, v.x);
-            p = __dsub_rn(p0, v.y);
-            if (lane == 0)
-                p2[k] = make_double2(p0, p);
-        }
-        P = p;
-        __syncwarp();
-        uint32_t hm = hits;
-        while (hm) {
-            const int j = __ffs(hm) - 1;
-            const uint32_t mj = sg_ent_pattern(__shfl_sync(SG_FULL, ent, j));
-            if (sg_list_hit(ws, lp, mj, ws->ps[j], ws->es[j], lane)) {
-                T = bh + (uint32_t)j + 1u;
-                done = true;
-                break;
+        int k = 0;
+        do {
+            const int j = hits ? __ffs(hits) - 1 : 31;
+#pragma unroll 4
+            for (; k <= j; k++)
+                p = __dsub_rn(p, ws->es[k]);
+            if (hits && sg_list_hit(ws, lp, ent, p, e, j, lane)) {
+                T = base + (uint32_t)j + 1u;
+                return true;
             }
-            hm &= hm - 1u;
-        }
+            hits &= hits - 1u;
+        } while (k < 32);
     }
+    Pb = sg_bits(p);
     __syncwarp();
+    return false;
+}
+
+/* A step that holds codewords and neither ties nor crosses: P at each of
+ * them is P less the units up to its lane, and nb after the step.  Returns
+ * as sg_replay. */
+__device__ __forceinline__ bool sg_sum_hits(double e, uint32_t ent, uint32_t hits, uint32_t lo, uint32_t hi, uint32_t base,
+                                            uint64_t& Pb, uint64_t nb, SgWarpScratch* ws, uint32_t& T,
+                                            const SgLineParams& lp, int lane)
+{
+    do {
+        const int j = __ffs(hits) - 1;
+        const bool in = lane <= j;
+        const uint64_t pj = Pb - sg_units_sum(in ? lo : 0u, in ? hi : 0u);
+        if (sg_list_hit(ws, lp, ent, sg_from_bits(pj), e, j, lane)) {
+            T = base + (uint32_t)j + 1u;
+            return true;
+        }
+        hits &= hits - 1u;
+    } while (hits);
+    Pb = nb;
+    return false;
 }
 
 /* Extra results of a line decode run for the adjoint (ADJ = true): the
@@ -277,12 +422,13 @@ struct SgAdjOut {
 /* Decode one line.  llr: this lane's input LLR (lanes 0..15; others
  * ignored).  enum_tabs: SG_ENUM_NTAB tables of SG_ENUM_LEN entries.
  * etab/ltab: shared-memory copies of the exp/log tables. */
-template <int G, bool ADJ = false, bool CR = false>
+template <bool ADJ = false, bool CR = false, bool T8 = true>
 __device__ __forceinline__ SgLineResult sg_decode_line(double llr, const SgLineParams& lp,
                                                         const uint32_t* __restrict__ enum_tabs,
-                                                        const double* etab, const double* ltab,
-                                                        SgWarpScratch* ws, SgAdjOut* adj = nullptr)
+                                                        SgTab etab, SgTab ltab, SgWarpScratch* ws,
+                                                        SgAdjOut* adj = nullptr)
 {
+    const uint32_t ra = sg_saddr(ws); /* low byte zero */
     const int lane = threadIdx.x & 31;
     const bool act = lane < 16;
     if (!act)
@@ -341,11 +487,11 @@ __device__ __forceinline__ SgLineResult sg_decode_line(double llr, const SgLineP
     /* ties (and NaN, which no comparison orders) take the exact quicksort */
     if (!__any_sync(SG_FULL, act && (eq > 0 || a != a))) {
         if (act)
-            ws->perm[lt] = lane;
+            ws->perm[lt] = (uint8_t)lane;
     } else {
         if (act) {
             ws->qa[lane] = a;
-            ws->perm[lane] = lane;
+            ws->perm[lane] = (uint8_t)lane;
         }
         __syncwarp();
         if (lane == 0)
@@ -366,7 +512,7 @@ __device__ __forceinline__ SgLineResult sg_decode_line(double llr, const SgLineP
     __syncwarp();
     const int src = act ? ws->perm[lane] : 0;
     if (act)
-        ws->rank[src] = lane;
+        ws->rank[src] = (uint8_t)lane;
     const double as = __shfl_sync(SG_FULL, a, src);
 
     /* IC (:619-622): beta = (|L|_(7) - |L|_(0)) / 7, IC = max(round(.), 0) */
@@ -444,178 +590,146 @@ __device__ __forceinline__ SgLineResult sg_decode_line(double llr, const SgLineP
             reinterpret_cast<uint2*>(ws->synlo)[lane ^ (g >> 3)] = (g & 4u) ? make_uint2(w1, w0) : make_uint2(w0, w1);
         }
         reinterpret_cast<uint2*>(ws->synhi)[lane] = make_uint2(hi0, hi0 ^ hh[2] * 0x01010101u);
-        if (lane < 16)
-            ws->dz[lane] = (lane >= 1 && lane <= 8) ? ws->es[lane + 7] : 0.0;
+        if (lane < 9)
+            ws->dz[lane] = lane ? ws->es[lane + 7] : 0.0;
     }
+    /* largest path metric of the line: exp(-PM) needs no range check below it */
+    double pmax = dl;
+    for (int off = 8; off > 0; off >>= 1)
+        pmax = __dadd_rn(pmax, __shfl_xor_sync(SG_FULL, pmax, off));
+    const bool wide = !(__shfl_sync(SG_FULL, pmax, 0) + pmhd < 700.0);
     /* the sort is done with qa: it keeps the input LLRs for the soft output */
     if (act)
         ws->qa[lane] = llr;
     if (lane == 0) {
         ws->curl = 0;
         ws->pnl = 0.0;
+        ws->ppos = 0.0;
         ws->hdm = hdm;
+        ws->itab = itab;
     }
     __syncwarp();
 
-    /* Guess loop (:624-744) */
-    const uint32_t* tab = enum_tabs + (size_t)itab * SG_ENUM_LEN;
-    const bool has_tmax = lp.tmax < SG_ENUM_LEN;
-    double P = 1.0; /* P_notGuess */
-
+    /* Guess loop (:624-744), 32 patterns a step.  From pattern `special` on
+     * a step may hold patterns with three or more high positions, end at the
+     * Tmax cut, or (special = 0) hold terms below the normal range. */
+    uint32_t idx = (uint32_t)itab * SG_ENUM_LEN + (uint32_t)lane; /* low 16 bits: the pattern, low 5: the lane */
+    const uint32_t special =
+        (uint32_t)itab * SG_ENUM_LEN + (wide ? 0u : min(lp.meta->h3[itab], lp.meta->lim[itab]) & ~31u);
+    const uint32_t ea = sg_saddr(etab.t);
+    uint64_t Pb = 0x3ff0000000000000ull; /* P_notGuess, as its bit pattern */
+    SgGrid g = sg_grid(Pb);
     uint32_t T = 0;
-    bool done = false;
     double adj_tot = 0.0, adj_r[ADJ ? 16 : 1];
 #pragma unroll
     for (int r = 0; r < (ADJ ? 16 : 1); r++)
         adj_r[r] = 0.0;
-    /* The loop is instantiated twice.  Without a Tmax cut (TM false) every
-     * step holds 32 * G valid patterns: SG_ENUM_LEN is a multiple of 32 * G,
-     * so a step either lies inside the order table or starts at its end,
-     * where the line decode ends with T = SG_ENUM_LEN. */
-    auto guess_loop = [&](auto tm_tag) {
-    constexpr bool TM = decltype(tm_tag)::value;
-    static_assert(SG_ENUM_LEN % (32u * G) == 0, "steps tile the order table");
-    for (uint32_t base = 0; !done; base += 32u * G) {
-        if (!TM && base >= SG_ENUM_LEN) {
-            T = SG_ENUM_LEN;
-            break;
-        }
-        /* G patterns per lane: lane j of half h tests pattern base + 32h + j */
-        uint32_t ent[G];
-        double e[G];
-        uint32_t hits[G];
-        int nv[G];
-        int nvt = 0; /* valid patterns of the step, in order */
+    auto adj_add = [&](double e, uint32_t ent) { /* a guess that entered P_notGuess */
+        adj_tot += e;
+        const uint32_t m = sg_ent_pattern(ent);
 #pragma unroll
-        for (int h = 0; h < G; h++) {
-            const uint32_t bh = base + 32u * h;
-            const uint32_t t = bh + lane;
-            if (TM) {
-                ent[h] = __ldg(tab + (t < SG_ENUM_LEN ? t : SG_ENUM_LEN - 1u));
-                nv[h] = bh >= SG_ENUM_LEN ? 0 : (bh + 32u <= SG_ENUM_LEN ? 32 : (int)(SG_ENUM_LEN - bh));
-            } else {
-                ent[h] = __ldg(tab + t);
-                nv[h] = 32;
-            }
-        }
-        if (TM) {
-            /* T < Tmax is checked before each new logistic weight (:652); a cut
-             * in one half ends the step there */
-            bool cut_seen = false;
-#pragma unroll
-            for (int h = 0; h < G; h++) {
-                const uint32_t t = base + 32u * h + lane;
-                const uint32_t cut =
-                    __ballot_sync(SG_FULL, lane < nv[h] && (ent[h] & SG_ENUM_GS) && t > 0 && t >= lp.tmax);
-                if (cut_seen)
-                    nv[h] = 0;
-                else if (cut) {
-                    nv[h] = __ffs(cut) - 1;
-                    cut_seen = true;
-                }
-            }
-        }
-#pragma unroll
-        for (int h = 0; h < G; h++) {
-            const uint32_t lo = ent[h] & 0xffu; /* already the storage index sg_swz(low byte) */
-            const uint32_t hi = (ent[h] >> 8) & 0xffu;
-            double pm = ws->A[lo];
-            const uint32_t syn = (uint32_t)ws->synlo[lo] ^ (uint32_t)ws->synhi[hi];
-            /* high positions in ascending order: the first two from the
-             * entry's offsets (offset 0 reads dz[0] = 0, and pm + 0 = pm
-             * since pm >= +0), any further ones in a loop few steps enter */
-            const char* dzb = reinterpret_cast<const char*>(ws->dz);
-            pm = __dadd_rn(pm, *reinterpret_cast<const double*>(dzb + ((ent[h] >> 17) & 0x7fu)));
-            pm = __dadd_rn(pm, *reinterpret_cast<const double*>(dzb + ((ent[h] >> 24) & 0x7fu)));
-            if (__any_sync(SG_FULL, (ent[h] & SG_ENUM_HI3) != 0u)) {
-                uint32_t rest = hi & (hi - 1u);
-                rest &= rest - 1u;
-                while (rest) {
-                    pm = __dadd_rn(pm, ws->dz[__ffs(rest)]);
-                    rest &= rest - 1u;
-                }
-            }
-            e[h] = sg_dec_exp_neg<CR>(-pm, etab);
-            hits[h] = __ballot_sync(SG_FULL, syn == 0u) & (nv[h] >= 32 ? SG_FULL : ((1u << nv[h]) - 1u));
-            nvt += nv[h];
-        }
-
-        /* common case: no codeword, no large term, no tie and no binade
-         * crossing in the step -- P_notGuess moves by the exact integer sum */
-        bool any_hit = false, stepped = false;
-#pragma unroll
-        for (int h = 0; h < G; h++)
-            any_hit |= hits[h] != 0u;
-        if (!any_hit && P >= 0x1p-970) {
-            const int E = (int)((sg_bits(P) >> 52) & 0x7ffu) - 1023;
-            const double iu = sg_from_bits((uint64_t)(52 - E + 1023) << 52);
-            /* d = round(q) < 2^52 is the mantissa of q + 2^52; its two 26-bit
-             * halves are summed over the warp in 32-bit integers (at most
-             * 32 * G terms below 2^26 each) */
-            static_assert(G <= 2, "32-bit sums of 26-bit halves hold 64 terms");
-            uint32_t slo = 0u, shi = 0u;
-            bool bad = false;
-#pragma unroll
-            for (int h = 0; h < G; h++) {
-                const double q = lane < nv[h] ? __dmul_rn(e[h], iu) : 0.0;
-                const double t = __dadd_rn(q, 0x1p52);
-                const double d = __dsub_rn(t, 0x1p52);
-                bad |= !(q < 0x1p52) || fabs(__dsub_rn(q, d)) == 0.5;
-                const uint64_t tb = sg_bits(t);
-                slo += (uint32_t)tb & 0x3ffffffu;
-                shi += (uint32_t)(tb >> 26) & 0x3ffffffu;
-            }
-            if (!__any_sync(SG_FULL, bad)) {
-                const uint32_t tlo = __reduce_add_sync(SG_FULL, slo);
-                const uint32_t thi = __reduce_add_sync(SG_FULL, shi);
-                /* exact below 2^53; a larger (rounded) total fails the test below */
-                const double tot = __dadd_rn(__dmul_rn(__uint2double_rn(thi), 0x1p26), __uint2double_rn(tlo));
-                const double M0 = __dmul_rn(P, iu);
-                if (tot <= __dsub_rn(M0, 0x1p52 + 1.0)) {
-                    P = __dmul_rn(__dsub_rn(M0, tot), sg_from_bits((uint64_t)(E - 52 + 1023) << 52));
-                    T = base + (uint32_t)nvt;
-                    if (nvt < 32 * G)
-                        done = true;
-                    stepped = true;
-                }
-            }
-        }
-
-        /* general case, one half after the other */
-        if (!stepped) {
-#pragma unroll
-            for (int h = 0; h < G; h++) {
-                if (done)
-                    break;
-                sg_seq_half(e[h], ent[h], hits[h], base + 32u * h, P, ws, T, done, lp, lane);
-                if (!done && nv[h] < 32) {
-                    T = base + 32u * h + (uint32_t)nv[h];
-                    done = true;
-                }
-            }
-            if (!done)
-                T = base + 32u * G;
-        }
-        if (ADJ) {
-            /* the guesses of this step that entered P_notGuess: [base, T) */
-#pragma unroll
-            for (int h = 0; h < G; h++) {
-                if (base + 32u * h + (uint32_t)lane < T) {
-                    adj_tot += e[h];
-                    const uint32_t m = sg_ent_pattern(ent[h]);
-#pragma unroll
-                    for (int r = 0; r < (ADJ ? 16 : 1); r++)
-                        if ((m >> r) & 1u)
-                            adj_r[r] += e[h];
-                }
-            }
-        }
-    }
+        for (int r = 0; r < (ADJ ? 16 : 1); r++)
+            if ((m >> r) & 1u)
+                adj_r[r] += e;
     };
-    if (has_tmax)
-        guess_loop(SgBoolTag<true>());
-    else
-        guess_loop(SgBoolTag<false>());
+    /* path metric (up to two high positions) and syndrome of an entry: the
+     * high positions in ascending order, from the entry's offsets (offset 0
+     * reads dz[0] = 0, and pm + 0 = pm since pm >= +0) */
+    auto metric = [&](uint32_t ent) {
+        double pm = sg_lds_f64<offsetof(SgWarpScratch, A)>(ra + (ent & 0xffu) * 8u);
+        pm = __dadd_rn(pm, sg_lds_f64<offsetof(SgWarpScratch, dz)>(__byte_perm(ent, ra, 0x7652)));
+        return __dadd_rn(pm, sg_lds_f64<offsetof(SgWarpScratch, dz)>(__byte_perm(ent, ra, 0x7653)));
+    };
+    auto is_codeword = [&](uint32_t ent) {
+        return sg_lds_u8<offsetof(SgWarpScratch, synlo)>(__byte_perm(ent, ra, 0x7650)) ==
+               sg_lds_u8<offsetof(SgWarpScratch, synhi)>(__byte_perm(ent, ra, 0x7651));
+    };
+    /* Units of a lane's term on the grid, as 26-bit halves; true when it
+     * ties or leaves the binade. */
+    auto term_units = [&](double e, uint32_t& lo, uint32_t& hi) {
+        const double s1 = __dadd_rn(g.b1, e), s2 = __dadd_rn(g.b2, e);
+        const uint32_t l1 = (uint32_t)__double2loint(s1);
+        const uint32_t dh = (uint32_t)(__double2hiint(s1) - __double2hiint(g.b1));
+        lo = l1 & 0x3ffffffu;
+        hi = __funnelshift_r(l1, dh, 26);
+        return (uint32_t)__double2loint(s2) - l1 != 1u || dh >= 0x100000u;
+    };
+    for (;;) {
+        uint32_t ent, lo, hi;
+        double e;
+        uint64_t tot;
+        bool out = false, hit, tie;
+        const SgExpK ek = *lp.ek;
+        /* P is moved by the step's units.  2^26 in place of the upper half of
+         * a lane that cannot be summed, or that holds a codeword, makes them
+         * 2^52 or more, which leaves the binade. */
+#pragma unroll 1
+        while (idx < special) {
+            ent = __ldg(enum_tabs + idx);
+            const double pm = metric(ent);
+            hit = is_codeword(ent);
+            e = CR || !T8 ? sg_dec_exp_neg<CR>(-pm, etab) : sg_exp_neg_k(-pm, ea, ek);
+            tie = term_units(e, lo, hi);
+            tot = sg_units_sum(lo, (tie || hit) ? 0x4000000u : hi);
+            Pb -= tot;
+            if ((int32_t)(Pb >> 32) <= __double2hiint(g.b1)) {
+                out = true;
+                break;
+            }
+            if (ADJ)
+                adj_add(e, ent);
+            idx += 32u;
+        }
+        if (!out) {
+            const uint32_t end = (uint32_t)ws->itab * SG_ENUM_LEN + lp.meta->lim[ws->itab];
+            if (idx - (uint32_t)lane >= end) {
+                T = lp.meta->lim[ws->itab];
+                break;
+            }
+            ent = __ldg(enum_tabs + idx);
+            double pm = metric(ent);
+            uint32_t rest = (ent >> 8) & 0xffu;
+            rest &= rest - 1u;
+            rest &= rest - 1u;
+            while (rest) {
+                pm = __dadd_rn(pm, ws->dz[__ffs(rest)]);
+                rest &= rest - 1u;
+            }
+            hit = idx < end && is_codeword(ent);
+            e = idx < end ? sg_dec_exp<CR>(-pm, etab) : 0.0;
+            tie = term_units(e, lo, hi);
+            tot = sg_units_sum(lo, (tie || hit) ? 0x4000000u : hi);
+            Pb -= tot;
+            if ((int32_t)(Pb >> 32) > __double2hiint(g.b1)) {
+                if (ADJ)
+                    adj_add(e, ent);
+                idx += 32u;
+                continue;
+            }
+        }
+        Pb += tot;
+        const uint32_t hits = __ballot_sync(SG_FULL, hit);
+        const uint32_t base = (idx - (uint32_t)lane) & (SG_ENUM_LEN - 1u);
+        bool done;
+        uint64_t nb = 0;
+        /* a step without codewords failed the sum because it ties or crosses */
+        bool exact = hits != 0u && !__any_sync(SG_FULL, tie);
+        if (exact) {
+            nb = Pb - sg_units_sum(lo, hi);
+            exact = (int32_t)(nb >> 32) > __double2hiint(g.b1);
+        }
+        if (exact) {
+            done = sg_sum_hits(e, ent, hits, lo, hi, base, Pb, nb, ws, T, lp, lane);
+        } else {
+            done = sg_replay(e, ent, hits, base, Pb, ws, T, lp, lane);
+            g = sg_grid(Pb);
+        }
+        if (ADJ && (!done || (idx & (SG_ENUM_LEN - 1u)) < T))
+            adj_add(e, ent);
+        if (done)
+            break;
+        idx += 32u;
+    }
     if (ADJ) {
         /* sums over the warp; lane r keeps sorted position r */
         for (int off = 16; off > 0; off >>= 1)
@@ -634,7 +748,14 @@ __device__ __forceinline__ SgLineResult sg_decode_line(double llr, const SgLineP
         const int curl = ws->curl;
         adj->pnl = ws->pnl;
         adj->my_e = lane < curl ? ws->lst_e[lane] : 0.0;
-        adj->my_cm = lane < curl ? ws->lst_cm[lane] : 0u;
+        /* codeword bits of the list entries (AddTEP, :761): position i flips
+         * when its sorted rank is in the pattern */
+        adj->my_cm = 0u;
+        for (int k = 0; k < curl; k++) {
+            const uint32_t cm = hdm ^ (__ballot_sync(SG_FULL, act && ((ws->lst_m[k] >> ws->rank[lane & 15]) & 1u)) & 0xffffu);
+            if (lane == k)
+                adj->my_cm = cm;
+        }
         adj->hdm = hdm;
         adj->curl = curl;
         adj->myrank = act ? ws->rank[lane] : 0;
@@ -655,6 +776,7 @@ __device__ __forceinline__ SgLineResult sg_decode_line(double llr, const SgLineP
         /* every lane works on position lane & 15; lanes 0..15 then take
          * log(p0), lanes 16..31 log(p1) */
         const int pos = lane & 15;
+        const uint32_t rk = ws->rank[pos], hb = ws->hdm >> pos;
         const double pnlc = fmax(ws->pnl, 1e-40);
         double pp1 = __ddiv_rn(1.0, __dadd_rn(1.0, ws->ex[pos]));
         double pp0 = __dsub_rn(1.0, pp1);
@@ -662,7 +784,8 @@ __device__ __forceinline__ SgLineResult sg_decode_line(double llr, const SgLineP
         pp0 = fmin(fmax(pp0, 1e-40), 1.0);
         double p1 = 0.0, p0 = 0.0;
         for (int j = 0; j < curl; j++) {
-            const double c = (double)((ws->lst_cm[j] >> pos) & 1u);
+            /* AddTEP (:761): position i flips when its sorted rank is in the pattern */
+            const double c = (double)(((ws->lst_m[j] >> rk) ^ hb) & 1u);
             const double pj = ws->lst_e[j];
             p1 = __dadd_rn(p1, __dmul_rn(c, pj));
             p0 = __dadd_rn(p0, __dmul_rn(__dsub_rn(1.0, c), pj));

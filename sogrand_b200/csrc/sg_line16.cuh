@@ -45,10 +45,8 @@ __device__ __forceinline__ uint32_t sg_pxor_u32(uint32_t v)
  * the same order; only a half with `act` set changes its list.  Returns
  * true when that half's line decode stops. */
 __device__ __forceinline__ bool sg_list_hit16(SgWarpScratch* ws, const SgLineParams& lp, uint32_t mj, double P,
-                                              double ej, int sl, int hb, bool act)
+                                              double ej, int sl, bool act)
 {
-    const int myrank = ws->rank[sl];
-    const uint32_t cm = ws->hdm ^ sg_pballot(hb, (mj >> myrank) & 1u);
     const int curl = ws->curl;
     double ppos = 0.0;
     for (int i = 0; i < curl; i++)
@@ -58,7 +56,7 @@ __device__ __forceinline__ bool sg_list_hit16(SgWarpScratch* ws, const SgLinePar
     __syncwarp();
     if (act && sl == 0) {
         ws->lst_e[curl] = ej;
-        ws->lst_cm[curl] = cm;
+        ws->lst_m[curl] = mj;
         ws->pnl = pneg;
         ws->curl = curl + 1;
     }
@@ -75,12 +73,13 @@ __device__ __forceinline__ bool sg_list_hit16(SgWarpScratch* ws, const SgLinePar
  * whole warp (sg_seq_half for two 16-lane lines). */
 __device__ __forceinline__ void sg_seq_sub16(double e, uint32_t ent, uint32_t hits, uint32_t bh, double& P,
                                              SgWarpScratch* ws, uint32_t& T, bool& done, bool run,
-                                             const SgLineParams& lp, int sl, int hb)
+                                             const SgLineParams& lp, int sl)
 {
     ws->es[sl] = e;
     __syncwarp();
     const double2* e2 = reinterpret_cast<const double2*>(ws->es);
-    double2* p2 = reinterpret_cast<double2*>(ws->ps);
+    double* ps = ws->es + 16; /* a sub-step has 16 terms; P after each of them follows */
+    double2* p2 = reinterpret_cast<double2*>(ps);
     const bool rec = __any_sync(SG_FULL, run && hits != 0u);
     double p = P;
     if (!rec) {
@@ -108,7 +107,7 @@ __device__ __forceinline__ void sg_seq_sub16(double e, uint32_t ent, uint32_t hi
         const bool act = hm != 0u;
         const int j = act ? __ffs(hm) - 1 : 0;
         const uint32_t mj = sg_ent_pattern(__shfl_sync(SG_FULL, ent, j, 16));
-        const bool stop = sg_list_hit16(ws, lp, mj, ws->ps[j], ws->es[j], sl, hb, act);
+        const bool stop = sg_list_hit16(ws, lp, mj, ps[j], ws->es[j], sl, act);
         if (act && stop) {
             T = bh + (uint32_t)j + 1u;
             done = true;
@@ -128,7 +127,7 @@ __device__ __forceinline__ void sg_seq_sub16(double e, uint32_t ent, uint32_t hi
 template <int G, bool CR>
 __device__ __forceinline__ SgLineResult sg_decode_line16(double llr, const SgLineParams& lp,
                                                           const uint32_t* __restrict__ enum_tabs,
-                                                          const double* etab, const double* ltab,
+                                                          SgTab etab, SgTab ltab,
                                                           SgWarpScratch* ws)
 {
     const int lane = threadIdx.x & 31;
@@ -174,10 +173,10 @@ __device__ __forceinline__ SgLineResult sg_decode_line16(double llr, const SgLin
     /* ties (and NaN, which no comparison orders) take the exact quicksort */
     const bool qsort = sg_pballot(hb, eq > 0 || a != a) != 0u;
     if (!qsort) {
-        ws->perm[lt] = sl;
+        ws->perm[lt] = (uint8_t)sl;
     } else {
         ws->qa[sl] = a;
-        ws->perm[sl] = sl;
+        ws->perm[sl] = (uint8_t)sl;
     }
     __syncwarp();
     if (qsort && sl == 0)
@@ -194,7 +193,7 @@ __device__ __forceinline__ SgLineResult sg_decode_line16(double llr, const SgLin
     }
     __syncwarp();
     const int src = ws->perm[sl]; /* this lane now also speaks for sorted rank sl */
-    ws->rank[src] = sl;
+    ws->rank[src] = (uint8_t)sl;
     const double as = __shfl_sync(SG_FULL, a, src, 16);
 
     /* IC (:619-622) */
@@ -269,7 +268,8 @@ __device__ __forceinline__ SgLineResult sg_decode_line16(double llr, const SgLin
             ws->synlo[sg_swz(byte)] = (uint8_t)(bl ^ gl);
             ws->synhi[byte] = (uint8_t)(bhi ^ gh);
         }
-        ws->dz[sl] = (sl >= 1 && sl <= 8) ? ws->es[sl + 7] : 0.0;
+        if (sl < 9)
+            ws->dz[sl] = sl ? ws->es[sl + 7] : 0.0;
     }
     /* the input LLRs for the soft output */
     ws->qa[sl] = llr;
@@ -283,7 +283,8 @@ __device__ __forceinline__ SgLineResult sg_decode_line16(double llr, const SgLin
     /* Guess loop (:624-744), 16 * G patterns of each line per step, while
      * either line is undecided */
     const uint32_t* tab = enum_tabs + (size_t)itab * SG_ENUM_LEN;
-    const bool has_tmax = lp.tmax < SG_ENUM_LEN;
+    const uint32_t lim = lp.meta->lim[itab]; /* the Tmax cut */
+    const bool has_tmax = lim < SG_ENUM_LEN;
     double P = 1.0; /* P_notGuess */
     uint32_t T = 0;
     bool done = false;
@@ -318,17 +319,11 @@ __device__ __forceinline__ SgLineResult sg_decode_line16(double llr, const SgLin
         }
         if (TM) {
             /* T < Tmax is checked before each new logistic weight (:652) */
-            bool cut_seen = false;
 #pragma unroll
             for (int h = 0; h < G; h++) {
-                const uint32_t t = base + 16u * h + (uint32_t)sl;
-                const uint32_t cut = sg_pballot(hb, sl < nv[h] && (ent[h] & SG_ENUM_GS) && t > 0 && t >= lp.tmax);
-                if (cut_seen)
-                    nv[h] = 0;
-                else if (cut) {
-                    nv[h] = __ffs(cut) - 1;
-                    cut_seen = true;
-                }
+                const uint32_t bh = base + 16u * h;
+                const int left = bh < lim ? (int)(lim - bh) : 0;
+                nv[h] = nv[h] < left ? nv[h] : left;
             }
         }
 #pragma unroll
@@ -338,11 +333,11 @@ __device__ __forceinline__ SgLineResult sg_decode_line16(double llr, const SgLin
             double pm = ws->A[lo];
             const uint32_t syn = (uint32_t)ws->synlo[lo] ^ (uint32_t)ws->synhi[hi];
             const char* dzb = reinterpret_cast<const char*>(ws->dz);
-            pm = __dadd_rn(pm, *reinterpret_cast<const double*>(dzb + ((ent[h] >> 17) & 0x7fu)));
-            pm = __dadd_rn(pm, *reinterpret_cast<const double*>(dzb + ((ent[h] >> 24) & 0x7fu)));
-            if (__any_sync(SG_FULL, (ent[h] & SG_ENUM_HI3) != 0u)) {
-                uint32_t rest = hi & (hi - 1u);
-                rest &= rest - 1u;
+            pm = __dadd_rn(pm, *reinterpret_cast<const double*>(dzb + ((ent[h] >> 16) & 0xffu)));
+            pm = __dadd_rn(pm, *reinterpret_cast<const double*>(dzb + (ent[h] >> 24)));
+            uint32_t rest = hi & (hi - 1u);
+            rest &= rest - 1u;
+            if (__any_sync(SG_FULL, rest != 0u)) {
                 while (rest) {
                     pm = __dadd_rn(pm, ws->dz[__ffs(rest)]);
                     rest &= rest - 1u;
@@ -398,7 +393,7 @@ __device__ __forceinline__ SgLineResult sg_decode_line16(double llr, const SgLin
             bool run = need;
 #pragma unroll
             for (int h = 0; h < G; h++) {
-                sg_seq_sub16(e[h], ent[h], hits[h], base + 16u * h, P, ws, T, done, run, lp, sl, hb);
+                sg_seq_sub16(e[h], ent[h], hits[h], base + 16u * h, P, ws, T, done, run, lp, sl);
                 if (run && !done && nv[h] < 16) {
                     T = base + 16u * h + (uint32_t)nv[h];
                     done = true;
@@ -423,6 +418,7 @@ __device__ __forceinline__ SgLineResult sg_decode_line16(double llr, const SgLin
     const double x = ws->qa[sl];
     double lapp = x, le = 0.0;
     if (curl != 0) {
+        const uint32_t rk = ws->rank[sl], hbit = ws->hdm >> sl;
         const double pnlc = fmax(ws->pnl, 1e-40);
         double pp1 = __ddiv_rn(1.0, __dadd_rn(1.0, ws->ex[sl]));
         double pp0 = __dsub_rn(1.0, pp1);
@@ -430,7 +426,8 @@ __device__ __forceinline__ SgLineResult sg_decode_line16(double llr, const SgLin
         pp0 = fmin(fmax(pp0, 1e-40), 1.0);
         double p1 = 0.0, p0 = 0.0;
         for (int j = 0; j < curl; j++) {
-            const double c = (double)((ws->lst_cm[j] >> sl) & 1u);
+            /* AddTEP (:761): position i flips when its sorted rank is in the pattern */
+            const double c = (double)(((ws->lst_m[j] >> rk) ^ hbit) & 1u);
             const double pj = ws->lst_e[j];
             p1 = __dadd_rn(p1, __dmul_rn(c, pj));
             p0 = __dadd_rn(p0, __dmul_rn(__dsub_rn(1.0, c), pj));

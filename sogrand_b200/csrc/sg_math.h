@@ -43,6 +43,57 @@
 #define SG_EXP_TAB_LEN 256 /* 128 x {H_j, t_j} */
 #define SG_LOG_TAB_LEN 384 /* 128 x {c_j, hi, lo} */
 
+/* The functions below take their table as an SgTab.
+ *
+ * The decoders hold the exp table in eight copies, entry j of copy c at
+ * 16-byte slot 8 j + c, lane l reading copy l mod 8: the 16-byte loads of
+ * eight lanes then fall into eight different bank groups whatever their
+ * entries (4.0 shared-memory cycles per warp load; 9.0 from a single copy).
+ * Their H_j have j * 2^45 taken off the bit pattern, so that adding k * 2^45,
+ * k = 128 e + j, gives 2^e H_j in one step.
+ *
+ * On the device an SgTab also points to the constants of the correctly
+ * rounded routines, which the kernels receive as launch arguments: a
+ * binary64 literal whose low word is not zero costs two moves wherever no
+ * register pair can hold it, an argument one load.  SGK(name) is the constant
+ * SG_name, SG_T(i) entry i of the table. */
+#define SG_CONSTANTS(X)                                                                                          \
+    X(EXP_INV_LN2_N) X(EXP_C3) X(EXP_C4) X(EXP_C5) X(EXP_C6) X(EXP_C7) X(LOG_LN2_HI) X(LOG_LN2_LO)                \
+    X(CR_EXP_C1) X(CR_EXP_C2) X(CR_EXP_C3) X(CR_LOG_G3) X(CR_LOG_G5) X(CR_LOG_G6) X(CR_LOG_G7) X(CR_LOG_G9)       \
+    X(CR_LOG_G10) X(CR_LOG_G11)
+#if defined(__CUDACC__)
+#define SG_K_INDEX(n) SG_K_##n,
+#define SG_K_VALUE(n) SG_##n,
+enum { SG_CONSTANTS(SG_K_INDEX) SG_K_COUNT };
+struct SgK {
+    double v[SG_K_COUNT];
+};
+#define SG_K_INIT {{SG_CONSTANTS(SG_K_VALUE)}}
+struct SgTab {
+    const double* t;
+    const double* k;
+    int st = 2;       /* exp table: distance of its entries, in doubles */
+    bool adj = false; /* exp table: H_j with j taken off its bit pattern (sg_exp_scale) */
+};
+#define SG_T(i) tab.t[i]
+#if defined(SG_K_ARGS)
+#define SGK(n) tab.k[SG_K_##n]
+#else
+#define SGK(n) SG_##n
+#endif
+#define SG_ST tab.st
+#define SG_ADJ tab.adj
+#else
+typedef const double* SgTab;
+#define SG_T(i) tab[i]
+#define SGK(n) tab.k[SG_K_##n]
+#define SG_ST 2
+#define SG_ADJ 0
+#endif
+/* Entry j of the exp table: {H_j, t_j}. */
+#define SG_EXP_H(j) SG_T(SG_ST * (j))
+#define SG_EXP_T(j) SG_T(SG_ST * (j) + 1)
+
 SG_HD uint64_t sg_bits(double x)
 {
 #if defined(__CUDA_ARCH__)
@@ -80,9 +131,16 @@ SG_HD double sg_pow2i(int e)
     return sg_from_bits((uint64_t)(int64_t)(e + 1023) << 52);
 }
 
+/* 2^(e + de) H_j for k = 128 e + j. */
+SG_HD double sg_exp_scale(double H, int k, int de, int adj)
+{
+    const int64_t add = adj ? (int64_t)((uint64_t)(int64_t)k << 45) : (int64_t)((uint64_t)(int64_t)(k >> 7) << 52);
+    return sg_from_bits(sg_bits(H) + (uint64_t)add + ((uint64_t)(int64_t)de << 52));
+}
+
 /* exp(x), round-to-nearest result within ~0.505 ulp.
  * tab: SG_EXP_TAB_LEN doubles, {H_j, t_j} interleaved. */
-SG_HD double sg_exp(double x, const double* tab)
+SG_HD double sg_exp(double x, SgTab tab)
 {
     if (!(x <= 709.782712893384)) /* NaN or overflow */
         return x != x ? x : sg_from_bits(0x7ff0000000000000ULL);
@@ -96,8 +154,8 @@ SG_HD double sg_exp(double x, const double* tab)
     r = sg_fma(-kd, SG_EXP_LN2_N_LO, r);
     int j = k & 127;
     int e = k >> 7; /* floor(k / 128) */
-    double H = tab[2 * j];
-    double t = tab[2 * j + 1];
+    double H = SG_EXP_H(j);
+    double t = SG_EXP_T(j);
     double r2 = r * r;
     double p = sg_fma(r, SG_EXP_C7, SG_EXP_C6);
     p = sg_fma(r, p, SG_EXP_C5);
@@ -108,13 +166,12 @@ SG_HD double sg_exp(double x, const double* tab)
     double u = sg_fma(t, r, t);   /* t * (1 + r) */
     double tmp = r + (u + p);     /* (1 + t) e^r - 1 */
     if (e >= -1021 && e <= 1022) {
-        double S = sg_from_bits(sg_bits(H) + ((uint64_t)(int64_t)e << 52));
+        double S = sg_exp_scale(H, k, 0, SG_ADJ);
         return sg_fma(S, tmp, S);
     }
     /* Near overflow or underflow: scale in two exact steps.  A subnormal
      * result is rounded twice. */
-    int e1 = e > 0 ? e - 64 : e + 64;
-    double S = sg_from_bits(sg_bits(H) + ((uint64_t)(int64_t)e1 << 52));
+    double S = sg_exp_scale(H, k, e > 0 ? -64 : 64, SG_ADJ);
     double y = sg_fma(S, tmp, S);
     return e > 0 ? y * 0x1p64 : y * 0x1p-64;
 }
@@ -122,7 +179,7 @@ SG_HD double sg_exp(double x, const double* tab)
 /* exp(x) for x <= 0, bit-identical to sg_exp: the same operations without
  * the range checks that cannot fire for arguments above -707.5 (the guess
  * loop's exp(-PM), PM >= 0). */
-SG_HD double sg_exp_neg(double x, const double* tab)
+SG_HD double sg_exp_neg(double x, SgTab tab)
 {
     if (x < -707.5)
         return sg_exp(x, tab);
@@ -133,12 +190,11 @@ SG_HD double sg_exp_neg(double x, const double* tab)
     double r = sg_fma(-kd, SG_EXP_LN2_N_HI, x);
     r = sg_fma(-kd, SG_EXP_LN2_N_LO, r);
     int j = k & 127;
-    int e = k >> 7;
 #if defined(__CUDA_ARCH__)
-    const double2 Ht = reinterpret_cast<const double2*>(tab)[j];
+    const double2 Ht = *reinterpret_cast<const double2*>(&SG_EXP_H(j));
     const double H = Ht.x, t = Ht.y;
 #else
-    const double H = tab[2 * j], t = tab[2 * j + 1];
+    const double H = SG_EXP_H(j), t = SG_EXP_T(j);
 #endif
     double r2 = r * r;
     double p = sg_fma(r, SG_EXP_C7, SG_EXP_C6);
@@ -149,7 +205,7 @@ SG_HD double sg_exp_neg(double x, const double* tab)
     p = p * r2;
     double u = sg_fma(t, r, t);
     double tmp = r + (u + p);
-    double S = sg_from_bits(sg_bits(H) + ((uint64_t)(int64_t)e << 52));
+    double S = sg_exp_scale(H, k, 0, SG_ADJ);
     return sg_fma(S, tmp, S);
 }
 
@@ -164,7 +220,7 @@ SG_HD double sg_two_sum(double a, double b, double* err)
 
 /* log(x), round-to-nearest result within ~0.502 ulp.
  * tab: SG_LOG_TAB_LEN doubles, {c_j, hi(-log c_j), lo(-log c_j)}. */
-SG_HD double sg_log(double x, const double* tab)
+SG_HD double sg_log(double x, SgTab tab)
 {
     uint64_t ix = sg_bits(x);
     int escale = 0;
@@ -184,9 +240,9 @@ SG_HD double sg_log(double x, const double* tab)
     int j = (int)((tmpb >> 45) & 127);
     int e = (int)((int64_t)tmpb >> 52) + escale;
     double zz = sg_from_bits(ix - (tmpb & (0xfffULL << 52)));
-    double c = tab[3 * j];
-    double lch = tab[3 * j + 1];
-    double lcl = tab[3 * j + 2];
+    double c = SG_T(3 * j);
+    double lch = SG_T(3 * j + 1);
+    double lcl = SG_T(3 * j + 2);
     /* r_hi + r_lo = z*c - 1 exactly */
     double pr = zz * c;
     double pe = sg_fma(zz, c, -pr);

@@ -36,8 +36,9 @@ struct SgSlot {
 template <int NW, int C>
 struct SgPersistSmem {
     SgSlot slot[C];
-    alignas(16) double etab[SG_EXP_TAB_LEN]; /* read as double2 by the exp routines */
+    SgEtab<true> etab;
     alignas(16) double ltab[SG_LOG_TAB_LEN];
+    SgExpK ek;
     SgWarpScratch ws[NW];
 };
 
@@ -139,17 +140,18 @@ __device__ __forceinline__ void sg_slot_admit(SgSlot& sl, const SgDecodeArgs& ar
     }
 }
 
-template <int NW, int C, int G, bool CR>
+template <int NW, int C, bool CR>
 __global__ void __launch_bounds__(NW * 32, 1) sg_persist_kernel(const __grid_constant__ SgDecodeArgs args,
                                                                 SgQueue* q)
 {
     constexpr int NT = NW * 32;
     SgPersistSmem<NW, C>& S = *reinterpret_cast<SgPersistSmem<NW, C>*>(sg_smem_raw);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    for (int i = tid; i < SG_EXP_TAB_LEN; i += NT)
-        S.etab[i] = g_etab[i];
+    sg_etab_fill<CR, true>(S.etab, g_etab, tid, NT);
     for (int i = tid; i < SG_LOG_TAB_LEN; i += NT)
         S.ltab[i] = g_ltab[i];
+    if (tid == 0)
+        S.ek = sg_exp_k();
     if (tid < C) {
         S.slot[tid].cw = -1;
         S.slot[tid].next = 256;
@@ -159,9 +161,11 @@ __global__ void __launch_bounds__(NW * 32, 1) sg_persist_kernel(const __grid_con
         sg_slot_admit(S.slot[warp], args, q, lane);
     __syncthreads();
 
+    const SgTab etab = sg_etab_of<CR, true>(S.etab, args.k.v), ltab{S.ltab, args.k.v};
     SgLineParams lp;
     lp.L = args.L;
-    lp.tmax = args.tmax;
+    lp.meta = &args.meta;
+    lp.ek = &S.ek;
     lp.thres = args.thres;
     const int nphase = 3 * args.imax;
     int idle = 0;
@@ -206,7 +210,7 @@ __global__ void __launch_bounds__(NW * 32, 1) sg_persist_kernel(const __grid_con
         double v = 1.0;
         if (lane < 16) /* L_ch + (alpha*L_E) */
             v = __dadd_rn(__ldg(g + pos), __dmul_rn(alpha, sl.le[pos]));
-        const SgLineResult r = sg_decode_line<G, false, CR>(v, lp, args.enum_tabs, S.etab, S.ltab, &S.ws[warp]);
+        const SgLineResult r = sg_decode_line<false, CR>(v, lp, args.enum_tabs, etab, ltab, &S.ws[warp]);
         if (lane < 16) {
             sl.le[pos] = r.le;
             if (args.lapp)
