@@ -90,13 +90,21 @@ __device__ __forceinline__ void sg_slot_retire(const SgSlot& sl, const SgDecodeA
 /* Take the next codeword of the batch into slot `sl` (warp-wide), or mark
  * the slot empty when the batch is exhausted.  Codewords with non-finite
  * LLRs are reported (converged = -1) and skipped. */
-__device__ __forceinline__ void sg_slot_admit(SgSlot& sl, const SgDecodeArgs& args, SgQueue* q, int lane)
+__device__ __forceinline__ void sg_slot_admit(SgSlot& sl, const SgDecodeArgs& args, SgQueue* q, int lane,
+                                              unsigned long long first, unsigned long long queued)
 {
-    for (;;) {
-        unsigned long long idx = 0;
-        if (lane == 0)
-            idx = atomicAdd(&q->head, 1ull);
-        idx = __shfl_sync(SG_FULL, idx, 0);
+    /* `first`: the codeword to take, or ~0 for the queue's next.  The queue
+     * hands out codewords from `queued` on: the first of each slot is fixed,
+     * slot s of CTA b taking s * CTAs + b, so that a batch smaller than the
+     * slots spreads over the SMs (the queue let the first CTAs fill all their
+     * slots: 7 codewords at 2 dB took 4.38 ms on 3 SMs, 2.0 ms on 7). */
+    for (;; first = ~0ull) {
+        unsigned long long idx = first;
+        if (first == ~0ull) {
+            if (lane == 0)
+                idx = queued + atomicAdd(&q->head, 1ull);
+            idx = __shfl_sync(SG_FULL, idx, 0);
+        }
         if (idx >= args.n_cw) {
             if (lane == 0)
                 *(volatile int*)&sl.cw = -1;
@@ -157,8 +165,9 @@ __global__ void __launch_bounds__(NW * 32, 1) sg_persist_kernel(const __grid_con
         S.slot[tid].next = 256;
     }
     __syncthreads();
+    const unsigned long long queued = (unsigned long long)C * gridDim.x;
     if (warp < C)
-        sg_slot_admit(S.slot[warp], args, q, lane);
+        sg_slot_admit(S.slot[warp], args, q, lane, (unsigned long long)warp * gridDim.x + blockIdx.x, queued);
     __syncthreads();
 
     const SgTab etab = sg_etab_of<CR, true>(S.etab, args.k.v), ltab{S.ltab, args.k.v};
@@ -185,17 +194,33 @@ __global__ void __launch_bounds__(NW * 32, 1) sg_persist_kernel(const __grid_con
             }
         }
         if (s < 0) {
-            bool live = false;
-            for (int c = 0; c < C; c++)
-                live |= sg_ld_volatile(&S.slot[c].cw) >= 0;
-            if (!live)
-                break;
-            if (++idle > args.wait_limit) {
-                if (lane == 0)
-                    atomicOr(&q->err, 2u);
-                break;
+            /* Nothing to take: sleep until a slot opens a phase or all are
+             * empty.  The idle warps share the issue slots with those that
+             * still work (at a batch's end one warp may hold the last line of
+             * the last codeword), so a look costs few instructions and comes
+             * once a microsecond. */
+            bool open = false, live = true;
+            for (; !open; idle++) {
+                live = false;
+#pragma unroll
+                for (int c = 0; c < C; c++) {
+                    live |= sg_ld_volatile(&S.slot[c].cw) >= 0;
+                    open |= sg_ld_volatile(&S.slot[c].next) < 256;
+                }
+                live |= open; /* a slot opens after its codeword is set */
+                if (open || !live)
+                    break;
+                if (idle >= args.wait_limit) {
+                    if (lane == 0)
+                        atomicOr(&q->err, 2u);
+                    live = false;
+                    break;
+                }
+                __nanosleep(1000);
             }
-            __nanosleep(256);
+            __syncwarp();
+            if (!__any_sync(SG_FULL, live))
+                break;
             continue;
         }
         idle = 0;
@@ -242,7 +267,7 @@ __global__ void __launch_bounds__(NW * 32, 1) sg_persist_kernel(const __grid_con
         if (conv || phases == nphase) {
             sg_slot_retire(sl, args, cw, phases, conv, lane);
             __syncwarp();
-            sg_slot_admit(sl, args, q, lane);
+            sg_slot_admit(sl, args, q, lane, ~0ull, queued);
         } else {
             if (lane == 0) {
                 sl.ngmax = 0;
