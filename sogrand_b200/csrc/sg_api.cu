@@ -305,13 +305,6 @@ sg_status cuda_fail(cudaError_t e, const char* what)
             return cuda_fail(e_, #call);      \
     } while (0)
 
-struct DevCtx {
-    bool ready = false;
-    uint32_t* enum_tabs = nullptr;
-    unsigned int* err = nullptr;
-    double* err_sink = nullptr; /* never-read output of the ceiling kernel */
-    int sms = 0;
-};
 
 std::mutex g_mu;
 std::atomic<long long> g_wait_limit{SG_WAIT_LIMIT_DEFAULT};
@@ -320,11 +313,10 @@ std::atomic<int> g_math_mode{0}; /* 0: table-driven exp/log, 1: correctly rounde
  * measures them).  B200, 12 000 codewords at 2 dB, table math: p32x3 122.0
  * ms, p28x3 124.2, p24x3 127.1; w16-gmem 124.8, w8-gmem 139.1, w12-smem
  * 140.7, w8-smem 169.1. */
-int g_pvariant_by_mode[2] = {5, 4};
-int g_variant_by_mode[2] = {4, 3};
+int g_pvariant_by_mode[2] = {SG_PVARIANT_AUTO, SG_PVARIANT_AUTO};
+int g_variant_by_mode[2] = {SG_VARIANT_AUTO, SG_VARIANT_AUTO};
 #define g_pvariant (g_pvariant_by_mode[g_math_mode.load()])
 #define g_variant (g_variant_by_mode[g_math_mode.load()])
-DevCtx g_ctx[64];
 std::vector<uint32_t> g_enum_host;
 sg_code_tables g_code;
 bool g_host_ready = false;
@@ -338,6 +330,8 @@ const SgTab k_etab_tab{k_etab_host, k_consts.v}, k_ltab_tab{k_ltab_host, k_const
 const void* decode_fn(int v, bool cr) { return cr ? sg_cr_decode_fn(v) : k_variants[v].fn; }
 const void* persist_fn(int v, bool cr) { return cr ? sg_cr_persist_fn(v) : k_pvariants[v].fn; }
 
+const void* cluster_fn(int v, bool cr) { return cr ? sg_cr_cluster_fn(v) : k_cvariants[v].fn; }
+
 sg_status host_init_locked()
 {
     if (g_host_ready)
@@ -349,6 +343,95 @@ sg_status host_init_locked()
             return fail(SG_ERR_ARG, "error-pattern order table incomplete");
     g_host_ready = true;
     return SG_OK;
+}
+
+/* What the choice of a cluster configuration needs to know of a device. */
+struct ClusterInfo {
+    int sms = 0;
+    int fit[SG_NCVARIANTS] = {}; /* clusters that run at the same time */
+};
+
+struct DevCtx {
+    bool ready = false;
+    uint32_t* enum_tabs = nullptr;
+    unsigned int* err = nullptr;
+    double* err_sink = nullptr; /* never-read output of the ceiling kernel */
+    int sms = 0;
+    ClusterInfo clusters;
+};
+DevCtx g_ctx[64];
+
+cudaLaunchConfig_t cluster_config(int v, unsigned long long clusters, cudaStream_t st, cudaLaunchAttribute* at)
+{
+    const SgCVariant& c = k_cvariants[v];
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(clusters * c.cs));
+    cfg.blockDim = dim3(c.nw * 32);
+    cfg.dynamicSmemBytes = c.smem;
+    cfg.stream = st;
+    at->id = cudaLaunchAttributeClusterDimension;
+    at->val.clusterDim.x = c.cs;
+    at->val.clusterDim.y = at->val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cfg;
+}
+
+cudaError_t cluster_setup(int dev, ClusterInfo* info)
+{
+    cudaError_t e = cudaDeviceGetAttribute(&info->sms, cudaDevAttrMultiProcessorCount, dev);
+    for (int v = 0; v < SG_NCVARIANTS && e == cudaSuccess; v++) {
+        for (bool cr : {false, true}) {
+            if (e == cudaSuccess)
+                e = cudaFuncSetAttribute(cluster_fn(v, cr), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)k_cvariants[v].smem);
+            if (e == cudaSuccess && k_cvariants[v].cs > 8)
+                e = cudaFuncSetAttribute(cluster_fn(v, cr), cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+        }
+        if (e == cudaSuccess) {
+            cudaLaunchAttribute at;
+            const cudaLaunchConfig_t cfg = cluster_config(v, 1, nullptr, &at);
+            e = cudaOccupancyMaxActiveClusters(&info->fit[v], cluster_fn(v, false), &cfg);
+        }
+    }
+    return e;
+}
+
+/* The cluster configuration for a batch of n codewords, -1 when it is large
+ * enough for one CTA per codeword: the most CTAs per codeword with which all
+ * clusters run at the same time; with two, also up to 7/4 codewords per SM.
+ * B200, one call at 2 dB: n = 1 plain 2.29 ms, 16 CTAs 0.43, 8 CTAs 0.52;
+ * n = 9: 8 CTAs 0.58, 16 (the ninth cluster waits) 0.66; n = 18: 4 CTAs 1.02,
+ * 8 1.18; n = 33: 4 CTAs 1.02, 2 1.57; n = 37 (one too many): 4 CTAs 1.66, 2
+ * 1.74; n = 100: 2 CTAs 2.00, plain 3.81; n = 220: 3.92, 4.46; n = 296: 4.35,
+ * 4.63 but 4.51 in the batched form; n = 600: 8.7, 8.5. */
+int cluster_for(unsigned long long n, const ClusterInfo& info)
+{
+    for (int v = 0; v < SG_NCVARIANTS; v++)
+        if (n <= (unsigned long long)info.fit[v])
+            return v;
+    return info.fit[SG_NCVARIANTS - 1] > 0 && 4 * n <= 7ull * info.sms ? SG_NCVARIANTS - 1 : -1;
+}
+
+cudaError_t launch_cluster(const SgDecodeArgs& a, int v, int mode, cudaStream_t st)
+{
+    void* kargs[] = {(void*)&a};
+    cudaLaunchAttribute at;
+    const cudaLaunchConfig_t cfg = cluster_config(v, a.n_cw, st, &at);
+    return cudaLaunchKernelExC(&cfg, cluster_fn(v, mode == 1), kargs);
+}
+
+/* Launch of the plain form. */
+cudaError_t launch_decode(const SgDecodeArgs& a, const ClusterInfo& info, int mode, cudaStream_t st)
+{
+    const int vi = g_variant_by_mode[mode];
+    const int cv = vi == SG_VARIANT_AUTO ? cluster_for(a.n_cw, info) : -1;
+    if (cv >= 0)
+        return launch_cluster(a, cv, mode, st);
+    const SgVariant& v = k_variants[vi];
+    void* kargs[] = {(void*)&a};
+    return cudaLaunchKernel(decode_fn(vi, mode == 1), dim3((unsigned)std::min<unsigned long long>(a.n_cw, 1 << 30)),
+                            dim3(v.nw * 32), kargs, v.smem, st);
 }
 
 sg_status get_ctx(DevCtx** out)
@@ -383,6 +466,7 @@ sg_status get_ctx(DevCtx** out)
             SG_CUDA(cudaFuncSetAttribute(persist_fn(v, true), cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)k_pvariants[v].smem));
         }
+        SG_CUDA(cluster_setup(dev, &c.clusters));
         SG_CUDA(cudaFuncSetAttribute(sg_backward_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)sizeof(SgBackSmem<8>)));
         SG_CUDA(cudaDeviceGetAttribute(&c.sms, cudaDevAttrMultiProcessorCount, dev));
@@ -508,12 +592,7 @@ sg_status sg_decode_device(const double* d_llr, size_t n_cw, const sg_params* p,
     a.thres = p->thres;
     memcpy(a.alpha, p->alpha, sizeof a.alpha);
     a.k = k_consts;
-    const int mode = g_math_mode.load(), vi = g_variant_by_mode[mode];
-    const SgVariant& v = k_variants[vi];
-    const int grid = grid_for(n_cw, 1 << 30);
-    void* kargs[] = {(void*)&a};
-    SG_CUDA(cudaLaunchKernel(decode_fn(vi, mode == 1), dim3(grid), dim3(v.nw * 32), kargs, v.smem,
-                             (cudaStream_t)stream));
+    SG_CUDA(launch_decode(a, c->clusters, g_math_mode.load(), (cudaStream_t)stream));
     return SG_OK;
 }
 
@@ -784,6 +863,7 @@ struct NoAllocCtx {
     bool ready = false;
     unsigned char* scratch = nullptr; /* device address of g_noalloc_scratch */
     uint32_t* enum_tabs = nullptr;    /* device address of g_noalloc_enum */
+    ClusterInfo clusters;
 };
 NoAllocCtx g_noalloc[64];
 
@@ -811,6 +891,7 @@ sg_status noalloc_setup(NoAllocCtx** out)
             SG_CUDA(cudaFuncSetAttribute(decode_fn(v, true), cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)k_variants[v].smem));
         }
+        SG_CUDA(cluster_setup(dev, &c.clusters));
         /* the completion flags of the build borrow the scratch array */
         unsigned int* ok = reinterpret_cast<unsigned int*>(c.scratch);
         SG_CUDA(cudaMemset(ok, 0, SG_ENUM_NTAB * sizeof(unsigned int)));
@@ -878,11 +959,7 @@ sg_status sg_decode_summary_device_noalloc(const double* d_llr, size_t n_cw, con
     a.thres = p->thres;
     memcpy(a.alpha, p->alpha, sizeof a.alpha);
     a.k = k_consts;
-    const int mode = g_math_mode.load(), vi = g_variant_by_mode[mode];
-    const SgVariant& v = k_variants[vi];
-    void* kargs[] = {(void*)&a};
-    SG_CUDA(cudaLaunchKernel(decode_fn(vi, mode == 1), dim3(grid_for(n_cw, 1 << 30)), dim3(v.nw * 32), kargs, v.smem,
-                             st));
+    SG_CUDA(launch_decode(a, c->clusters, g_math_mode.load(), st));
     sg_summary_kernel<<<grid_for((n_cw + 255) / 256, 148 * 8), 256, 0, st>>>(stats, bits, d_ref_info, n_cw, err,
                                                                               d_summary);
     SG_CUDA(cudaGetLastError());
@@ -939,6 +1016,14 @@ sg_status batch_enqueue(sg_batch b, const double* d_llr, size_t n_cw, const sg_p
     memcpy(a.alpha, p->alpha, sizeof a.alpha);
     a.k = k_consts;
     const int mode = g_math_mode.load(), vi = g_pvariant_by_mode[mode];
+    /* a small batch goes to clusters; under a lowered wait limit it keeps the
+     * kernel whose waits that limit bounds (clusters only meet at hardware
+     * barriers) */
+    const int cv = vi == SG_PVARIANT_AUTO && a.wait_limit == SG_WAIT_LIMIT_DEFAULT ? cluster_for(n_cw, c->clusters) : -1;
+    if (cv >= 0) {
+        SG_CUDA(launch_cluster(a, cv, mode, st));
+        return SG_OK;
+    }
     const SgPVariant& v = k_pvariants[vi];
     SgQueue* q = b->q;
     void* kargs[] = {(void*)&a, (void*)&q};
@@ -1440,10 +1525,7 @@ sg_status sg_forward_device(const double* d_llr, size_t n_cw, const sg_params* p
     a.thres = p->thres;
     memcpy(a.alpha, p->alpha, sizeof a.alpha);
     a.k = k_consts;
-    const SgVariant& v = k_variants[g_variant];
-    void* kargs[] = {(void*)&a};
-    SG_CUDA(cudaLaunchKernel(v.fn, dim3(grid_for(n_cw, 1 << 30)), dim3(v.nw * 32), kargs, v.smem,
-                             (cudaStream_t)stream));
+    SG_CUDA(launch_decode(a, c->clusters, 0, (cudaStream_t)stream));
     return SG_OK;
 }
 

@@ -372,6 +372,7 @@ __global__ void __launch_bounds__(NW * 32, MINB) sg_decode_kernel(const __grid_c
 }
 
 #include "sg_persist.cuh"
+#include "sg_cluster.cuh"
 
 struct SgLineSmem {
     SgEtab<false> etab;
@@ -437,7 +438,9 @@ __global__ void __launch_bounds__(SG_THREADS) sg_bitso_kernel(const double* __re
  * CTAs per SM for the register budget, and lines per warp (1: 32 lanes per
  * line, sg_line.cuh; 2: 16 lanes per line and G patterns per lane,
  * sg_line16.cuh).  The "-g2" names of one-line configurations date from a
- * guess loop with two patterns per lane; they are the same kernels. */
+ * guess loop with two patterns per lane; they are the same kernels, and
+ * w16-gmem-g2 and p32x3-g2, the defaults, hand small batches to the cluster
+ * configurations below. */
 struct SgVariant {
     const char* name;
     int nw;
@@ -465,6 +468,8 @@ static const SgVariant k_variants[] = {
 };
 #define SG_NVARIANTS ((int)(sizeof(k_variants) / sizeof(k_variants[0])))
 
+#define SG_VARIANT_AUTO 4 /* w16-gmem-g2 */
+
 /* Batched persistent decoder configurations: warps per CTA (one CTA per
  * SM), codeword slots per CTA. */
 struct SgPVariant {
@@ -487,7 +492,19 @@ static const SgPVariant k_pvariants[] = {
     SG_PVARIANT(28, 3, "p28x3-g2"),
 };
 #define SG_NPVARIANTS ((int)(sizeof(k_pvariants) / sizeof(k_pvariants[0])))
+#define SG_PVARIANT_AUTO 5 /* p32x3-g2 */
 
+/* Cluster configurations (sg_cluster.cuh): warps per CTA and CTAs per
+ * codeword, the latter descending. */
+struct SgCVariant {
+    int nw;
+    int cs;
+    size_t smem;
+    const void* fn;
+};
+#define SG_CVARIANT(NW, CS) {NW, CS, sizeof(SgClusterSmem<NW>), (const void*)sg_cluster_kernel<NW, CS, SG_TU_CR>}
+static const SgCVariant k_cvariants[] = {SG_CVARIANT(16, 16), SG_CVARIANT(32, 8), SG_CVARIANT(32, 4), SG_CVARIANT(32, 2)};
+#define SG_NCVARIANTS ((int)(sizeof(k_cvariants) / sizeof(k_cvariants[0])))
 
 /* The code tables, for this translation unit's kernels. */
 static cudaError_t sg_load_code(const sg_code_tables& code)
