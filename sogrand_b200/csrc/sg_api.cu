@@ -214,7 +214,8 @@ static_assert(sg_tables_aligned<SgPersistSmem<24, 3>>() && sg_tables_aligned<SgP
                   sg_tables_aligned<SgCwSmem<8, false>>() && sg_tables_aligned<SgCwSmem<8, true>>() &&
                   sg_tables_aligned<SgCwSmem<12, true>>() && sg_tables_aligned<SgCwSmem<16, false>>() &&
                   sg_tables_aligned<SgCwSmem<8, false, 2>>() && sg_tables_aligned<SgCwSmem<10, false, 2>>() &&
-                  sg_tables_aligned<SgCwSmem<16, false, 2>>() && sg_tables_aligned<SgLineSmem>(),
+                  sg_tables_aligned<SgCwSmem<16, false, 2>>() && sg_tables_aligned<SgLineSmem<4, false>>() &&
+                  sg_tables_aligned<SgLineSmem<16, true>>(),
               "shared table alignment");
 template <class T>
 constexpr bool sg_bulk_aligned()
@@ -330,6 +331,7 @@ const SgTab k_etab_tab{k_etab_host, k_consts.v}, k_ltab_tab{k_ltab_host, k_const
 const void* decode_fn(int v, bool cr) { return cr ? sg_cr_decode_fn(v) : k_variants[v].fn; }
 const void* persist_fn(int v, bool cr) { return cr ? sg_cr_persist_fn(v) : k_pvariants[v].fn; }
 
+const void* bitso_fn(int v, bool cr) { return cr ? sg_cr_bitso_fn(v) : k_bvariants[v].fn; }
 const void* cluster_fn(int v, bool cr) { return cr ? sg_cr_cluster_fn(v) : k_cvariants[v].fn; }
 
 sg_status host_init_locked()
@@ -467,6 +469,10 @@ sg_status get_ctx(DevCtx** out)
                                          (int)k_pvariants[v].smem));
         }
         SG_CUDA(cluster_setup(dev, &c.clusters));
+        for (int v = 0; v < 2; v++)
+            for (bool cr : {false, true})
+                SG_CUDA(cudaFuncSetAttribute(bitso_fn(v, cr), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             (int)k_bvariants[v].smem));
         SG_CUDA(cudaFuncSetAttribute(sg_backward_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)sizeof(SgBackSmem<8>)));
         SG_CUDA(cudaDeviceGetAttribute(&c.sms, cudaDevAttrMultiProcessorCount, dev));
@@ -611,13 +617,17 @@ sg_status sg_bitso_device(const double* d_llr, size_t n_lines, int32_t L, uint64
         return s;
     sg_order_meta meta;
     order_meta(tmax_eff(Tmax), &meta);
-    const unsigned long long blocks = (n_lines + SG_WARPS - 1) / SG_WARPS;
+    /* few lines: one per warp, spread over the SMs; more than the warps two
+     * CTAs of 16 keep resident: those, each with an equal share */
+    const unsigned long long full = 2ull * c->sms;
+    const int bv = n_lines > 16 * full ? 1 : 0;
+    const SgBVariant& v = k_bvariants[bv];
+    unsigned long long n = n_lines, per = bv ? (n + full - 1) / full : (n < full ? 1 : v.nw);
     const uint32_t* tabs = c->enum_tabs;
     SgK k = k_consts;
-    unsigned long long n = n_lines;
-    void* kargs[] = {&d_llr, &n, &L, &thres, &d_lapp, &d_le, &d_nguess, &d_ncw, &tabs, &k, &meta};
-    SG_CUDA(cudaLaunchKernel(g_math_mode.load() ? sg_cr_bitso_fn() : (const void*)sg_bitso_kernel<false>,
-                             dim3(grid_for(blocks, 148 * 64)), dim3(SG_THREADS), kargs, 0, (cudaStream_t)stream));
+    void* kargs[] = {&d_llr, &n, &per, &L, &thres, &d_lapp, &d_le, &d_nguess, &d_ncw, &tabs, &k, &meta};
+    SG_CUDA(cudaLaunchKernel(bitso_fn(bv, g_math_mode.load() == 1), dim3((unsigned)((n + per - 1) / per)),
+                             dim3(v.nw * 32), kargs, v.smem, (cudaStream_t)stream));
     return SG_OK;
 }
 

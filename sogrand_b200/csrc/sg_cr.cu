@@ -8,5 +8,5 @@
 const void* sg_cr_decode_fn(int v) { return k_variants[v].fn; }
 const void* sg_cr_persist_fn(int v) { return k_pvariants[v].fn; }
 const void* sg_cr_cluster_fn(int v) { return k_cvariants[v].fn; }
-const void* sg_cr_bitso_fn() { return (const void*)sg_bitso_kernel<true>; }
+const void* sg_cr_bitso_fn(int v) { return k_bvariants[v].fn; }
 cudaError_t sg_cr_load_code(const sg_code_tables& code) { return sg_load_code(code); }

@@ -31,7 +31,6 @@
 #include "sg_math.h"
 
 #define SG_THREADS 256
-#define SG_WARPS (SG_THREADS / 32)
 /* Bounded device-side waits.  The limit of a wait that can give up (the
  * bulk-copy wait here, the persistent decoder's idle rounds) is a launch
  * argument, SG_WAIT_LIMIT_DEFAULT unless sg_set_wait_limit() changed it.
@@ -374,34 +373,45 @@ __global__ void __launch_bounds__(NW * 32, MINB) sg_decode_kernel(const __grid_c
 #include "sg_persist.cuh"
 #include "sg_cluster.cuh"
 
+template <int NW, bool T8>
 struct SgLineSmem {
-    SgEtab<false> etab;
+    SgEtab<T8> etab;
     alignas(16) double ltab[SG_LOG_TAB_LEN];
     SgExpK ek;
-    SgWarpScratch ws[SG_WARPS];
+    int next; /* of the CTA's lines, the next to hand out */
+    SgWarpScratch ws[NW];
 };
 
-template <bool CR>
-__global__ void __launch_bounds__(SG_THREADS) sg_bitso_kernel(const double* __restrict__ llr,
-                                                               unsigned long long n_lines,
-                                                               int32_t L, double thres, double* lapp, double* le,
-                                                               int32_t* nguess, int32_t* ncw,
-                                                               const uint32_t* enum_tabs,
-                                                               const __grid_constant__ SgK k,
-                                                               const __grid_constant__ sg_order_meta meta)
+/* SOGRAND_bitSO on independent lines, one per warp.  CTA b takes the lines
+ * [b * per, (b + 1) * per), its warps from a shared counter: the searches'
+ * lengths differ by an order of magnitude, and fixed shares would leave warps
+ * idle. */
+template <int NW, bool T8, bool CR>
+__global__ void __launch_bounds__(NW * 32, NW == 16 ? 2 : 1)
+    sg_bitso_kernel(const double* __restrict__ llr, unsigned long long n_lines, unsigned long long per, int32_t L,
+                    double thres, double* lapp, double* le, int32_t* nguess, int32_t* ncw, const uint32_t* enum_tabs,
+                    const __grid_constant__ SgK k, const __grid_constant__ sg_order_meta meta)
 {
-    __shared__ SgLineSmem S;
-    const SgTab etab = sg_etab_of<CR, false>(S.etab, k.v), ltab{S.ltab, k.v};
+    SgLineSmem<NW, T8>& S = *reinterpret_cast<SgLineSmem<NW, T8>*>(sg_smem_raw);
+    const SgTab etab = sg_etab_of<CR, T8>(S.etab, k.v), ltab{S.ltab, k.v};
     const SgLineParams lp{L, thres, &meta, &S.ek};
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    sg_etab_fill<CR, false>(S.etab, g_etab, tid, SG_THREADS);
-    for (int i = tid; i < SG_LOG_TAB_LEN; i += SG_THREADS)
+    sg_etab_fill<CR, T8>(S.etab, g_etab, tid, NW * 32);
+    for (int i = tid; i < SG_LOG_TAB_LEN; i += NW * 32)
         S.ltab[i] = g_ltab[i];
-    if (tid == 0)
+    if (tid == 0) {
         S.ek = sg_exp_k();
+        S.next = 0;
+    }
     __syncthreads();
-    for (unsigned long long l = (unsigned long long)blockIdx.x * SG_WARPS + warp; l < n_lines;
-         l += (unsigned long long)gridDim.x * SG_WARPS) {
+    const unsigned long long l0 = blockIdx.x * per, l1 = l0 + per < n_lines ? l0 + per : n_lines;
+    for (;;) {
+        int q = 0;
+        if (lane == 0)
+            q = atomicAdd(&S.next, 1);
+        const unsigned long long l = l0 + (unsigned)__shfl_sync(SG_FULL, q, 0);
+        if (l >= l1)
+            break;
         const double v = lane < 16 ? llr[l * 16 + lane] : 1.0;
         if (__any_sync(SG_FULL, !isfinite(v))) { /* not decoded: NaN out, N_guess -1 */
             if (lane < 16) {
@@ -415,7 +425,7 @@ __global__ void __launch_bounds__(SG_THREADS) sg_bitso_kernel(const double* __re
             }
             continue;
         }
-        const SgLineResult r = sg_decode_line<false, CR, false>(v, lp, enum_tabs, etab, ltab, &S.ws[warp]);
+        const SgLineResult r = sg_decode_line<false, CR, T8>(v, lp, enum_tabs, etab, ltab, &S.ws[warp]);
         if (lane < 16) {
             lapp[l * 16 + lane] = r.lapp;
             le[l * 16 + lane] = r.le;
@@ -505,6 +515,15 @@ struct SgCVariant {
 #define SG_CVARIANT(NW, CS) {NW, CS, sizeof(SgClusterSmem<NW>), (const void*)sg_cluster_kernel<NW, CS, SG_TU_CR>}
 static const SgCVariant k_cvariants[] = {SG_CVARIANT(16, 16), SG_CVARIANT(32, 8), SG_CVARIANT(32, 4), SG_CVARIANT(32, 2)};
 #define SG_NCVARIANTS ((int)(sizeof(k_cvariants) / sizeof(k_cvariants[0])))
+
+/* Line kernels: few lines (one per warp), and many (a full SM per two CTAs). */
+struct SgBVariant {
+    int nw;
+    size_t smem;
+    const void* fn;
+};
+#define SG_BVARIANT(NW, T8) {NW, sizeof(SgLineSmem<NW, T8>), (const void*)sg_bitso_kernel<NW, T8, SG_TU_CR>}
+static const SgBVariant k_bvariants[] = {SG_BVARIANT(4, false), SG_BVARIANT(16, true)};
 
 /* The code tables, for this translation unit's kernels. */
 static cudaError_t sg_load_code(const sg_code_tables& code)
