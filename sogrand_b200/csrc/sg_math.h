@@ -86,7 +86,7 @@ struct SgTab {
 #else
 typedef const double* SgTab;
 #define SG_T(i) tab[i]
-#define SGK(n) tab.k[SG_K_##n]
+#define SGK(n) SG_##n
 #define SG_ST 2
 #define SG_ADJ 0
 #endif
