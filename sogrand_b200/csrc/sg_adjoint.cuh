@@ -169,8 +169,8 @@ __global__ void __launch_bounds__(NW * 32, 3) sg_backward_kernel(const __grid_co
                 if (l >= 256)
                     break;
                 const int pos = sg_pos(axis, l, lane & 15);
-                const double lep = lane < 16 ? ck[pos] : 0.0;
-                const double x = lane < 16 ? __dadd_rn(g[pos], __dmul_rn(alpha, lep)) : 1.0;
+                const double lep = ck[pos];
+                const double x = __dadd_rn(g[pos], __dmul_rn(alpha, lep));
                 SgAdjOut a;
                 const SgLineResult r = sg_decode_line<true, false, false>(x, lp, args.enum_tabs, etab, ltab, &S.ws[warp], &a);
                 const double gE = lane < 16 ? S.gle[pos] : 0.0;

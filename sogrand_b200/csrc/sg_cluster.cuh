@@ -102,13 +102,11 @@ __global__ void __launch_bounds__(NW * 32, 1) sg_cluster_kernel(const __grid_con
             if (q >= LPC)
                 break;
             const int l = rank * LPC + q, pos = sg_pos(axis, l, lane & 15);
-            double v = 1.0;
-            if (lane < 16) { /* L_ch + (alpha*L_E) */
-                const double le0 = S.le[pos];
-                v = __dadd_rn(__ldg(g + pos), __dmul_rn(alpha, le0));
-                if (args.ckpt)
-                    args.ckpt[(cw * (unsigned long long)nphase + phase) * SG_CUBE + pos] = le0;
-            }
+            /* L_ch + (alpha*L_E), lanes p and p + 16 alike */
+            const double le0 = S.le[pos];
+            const double v = __dadd_rn(__ldg(g + pos), __dmul_rn(alpha, le0));
+            if (args.ckpt && lane < 16)
+                args.ckpt[(cw * (unsigned long long)nphase + phase) * SG_CUBE + pos] = le0;
             const SgLineResult r = sg_decode_line<false, CR, true>(v, lp, args.enum_tabs, etab, ltab, &S.ws[warp]);
             if (lane < 16) {
                 const uint32_t a = sg_mapa(le_a + 8u * (uint32_t)pos, sg_line_of(axis_next, pos) / LPC);

@@ -301,12 +301,11 @@ __global__ void __launch_bounds__(NW * 32, MINB) sg_decode_kernel(const __grid_c
                         if (l >= 256)
                             break;
                         const int pos = sg_pos(axis, l, lane & 15);
-                        double v = 1.0;
-                        if (lane < 16) { /* L_ch + (alpha*L_E) */
-                            v = __dadd_rn(LCH_SMEM ? S.lch[pos] : __ldg(g + pos), __dmul_rn(alpha, S.le[pos]));
-                            if (args.ckpt)
-                                args.ckpt[(cw * (3ull * args.imax) + 3 * (iter - 1) + axis) * SG_CUBE + pos] = S.le[pos];
-                        }
+                        /* L_ch + (alpha*L_E), lanes p and p + 16 alike */
+                        const double le0 = S.le[pos];
+                        const double v = __dadd_rn(LCH_SMEM ? S.lch[pos] : __ldg(g + pos), __dmul_rn(alpha, le0));
+                        if (args.ckpt && lane < 16)
+                            args.ckpt[(cw * (3ull * args.imax) + 3 * (iter - 1) + axis) * SG_CUBE + pos] = le0;
                         const SgLineResult r =
                             sg_decode_line<false, CR, T8>(v, lp, args.enum_tabs, etab, ltab, &S.ws[warp]);
                         if (lane < 16) {
@@ -412,7 +411,7 @@ __global__ void __launch_bounds__(NW * 32, NW == 16 ? 2 : 1)
         const unsigned long long l = l0 + (unsigned)__shfl_sync(SG_FULL, q, 0);
         if (l >= l1)
             break;
-        const double v = lane < 16 ? llr[l * 16 + lane] : 1.0;
+        const double v = llr[l * 16 + (lane & 15)];
         if (__any_sync(SG_FULL, !isfinite(v))) { /* not decoded: NaN out, N_guess -1 */
             if (lane < 16) {
                 lapp[l * 16 + lane] = __longlong_as_double(0x7ff8000000000000ll);

@@ -77,6 +77,13 @@ __device__ __forceinline__ double sg_dec_log(double x, SgTab tab)
     return CR ? sg_log_cr(x, tab) : sg_log(x, tab);
 }
 
+/* log of a positive normal argument */
+template <bool CR>
+__device__ __forceinline__ double sg_dec_log_pos(double x, SgTab tab)
+{
+    return CR ? sg_log_cr(x, tab) : sg_log_core(sg_bits(x), 0, tab);
+}
+
 #define SG_FULL 0xffffffffu
 
 /* Shared-memory loads at a 32-bit shared address.  Plain C++ accesses add
@@ -201,9 +208,10 @@ struct alignas(256) SgWarpScratch {
     uint32_t hdm;       /* hard decision, bit i = position i */
     int32_t itab;       /* order table of the line's IC */
     uint8_t rank[16];   /* position -> sorted rank */
-    uint8_t perm[16];   /* sorted rank -> position */
+    uint8_t perm[16];   /* sorted rank -> position (tied magnitudes only) */
+    alignas(16) uint8_t hcol[16]; /* syndrome columns of sorted positions r and r + 8 at bytes 2r, 2r + 1 */
     alignas(256) double es[32]; /* replay: exp(-PM) of the 32 patterns of a step */
-    double qa[16];      /* values for the tie-exact sort, then the input LLRs */
+    double qa[16];      /* sorted magnitudes, then the input LLRs */
     double ex[16];      /* exp(input LLR) of each position, for the soft output */
 };
 static_assert(offsetof(SgWarpScratch, synlo) == 2048 && offsetof(SgWarpScratch, synhi) == 2304 &&
@@ -419,8 +427,7 @@ struct SgAdjOut {
     int32_t myrank; /* lane i < 16: sorted rank of position i */
 };
 
-/* Decode one line.  llr: this lane's input LLR (lanes 0..15; others
- * ignored).  enum_tabs: SG_ENUM_NTAB tables of SG_ENUM_LEN entries.
+/* Decode one line.  llr: the input LLR of position lane & 15 (all lanes).  enum_tabs: SG_ENUM_NTAB tables of SG_ENUM_LEN entries.
  * etab/ltab: shared-memory copies of the exp/log tables. */
 template <bool ADJ = false, bool CR = false, bool T8 = true>
 __device__ __forceinline__ SgLineResult sg_decode_line(double llr, const SgLineParams& lp,
@@ -431,77 +438,75 @@ __device__ __forceinline__ SgLineResult sg_decode_line(double llr, const SgLineP
     const uint32_t ra = sg_saddr(ws); /* low byte zero */
     const int lane = threadIdx.x & 31;
     const bool act = lane < 16;
-    if (!act)
-        llr = 1.0;
     const double a = fabs(llr);
     /* HardDec (:758): 1 unless llr > 0 */
-    const uint32_t hdm = __ballot_sync(SG_FULL, act && !(llr > 0.0)) & 0xffffu;
-    /* JacLog(-|L_i|) for getPM_HD (:617, :764) */
-    /* lanes 0..15: JacLog(-|L_i|); lanes 16..31: JacLog(+|L_(lane-16)|), used
-     * for the sorted PM increments below */
-    const double a_all = __shfl_sync(SG_FULL, a, lane & 15);
-    const double xj = act ? -a_all : a_all;
-    const double ex = sg_dec_exp<CR>(xj, etab);
-    /* JacLog(xj) = xj if xj > 50, 0 if xj < -50, else log(1 + e^xj) (:762),
-     * with its exp kept */
-    const double jl = xj > 50 ? xj : (xj < -50 ? 0.0 : sg_dec_log<CR>(1.0 + ex, ltab));
-    const double jn = act ? jl : 0.0;
-    {
-        /* the soft output's exp(LLR) of position p is this exp of lane p + 16
-         * when the LLR is positive, of lane p otherwise (a NaN LLR is its own
-         * exp) */
-        const double lp_ = __shfl_sync(SG_FULL, llr, lane & 15);
-        if (act ? !(lp_ > 0.0) : (lp_ > 0.0))
-            ws->ex[lane & 15] = lp_ == lp_ ? ex : lp_;
-    }
+    const uint32_t hdm = __ballot_sync(SG_FULL, !(llr > 0.0)) & 0xffffu;
+    /* JacLog(xj) = xj if xj > 50, 0 if xj < -50, else log(1 + e^xj) (:762):
+     * lanes 0..15 take -|L| (getPM_HD, :617, :764), lanes 16..31 +|L| (the PM
+     * increments) */
+    const double xj = act ? -a : a;
+    double ex = CR ? sg_exp_cr(xj, etab) : sg_exp_mid(xj, etab);
+    if (!CR && !(a < 700.0))
+        ex = sg_exp(xj, etab);
+    const double jl = xj > 50 ? xj : (xj < -50 ? 0.0 : sg_dec_log_pos<CR>(1.0 + ex, ltab));
+    /* the soft output's exp(LLR) is this exp of lane p + 16 when the LLR is
+     * positive, of lane p otherwise (a NaN LLR is its own exp) */
+    if (act ? !(llr > 0.0) : (llr > 0.0))
+        ws->ex[lane & 15] = llr == llr ? ex : llr;
+    const double dl = __dsub_rn(__shfl_down_sync(SG_FULL, jl, 16), jl); /* lanes 0..15: PM increment (getPM, :765) */
 
     /* QuickSort of |L| ascending (:618): rank of each position.  Lane p and
-     * lane p + 16 count for position p the smaller (and equal) magnitudes
-     * among positions 0..7 and 8..15 respectively, then add.  The
-     * magnitudes are non-negative, so their high 32 bits order them unless
-     * two are equal there; only then are the full values compared. */
-    int lt = 0, eq = 0;
+     * lane p + 16 count the smaller magnitudes among positions 0..7 and
+     * 8..15, then add.  The magnitudes are non-negative, so their high 32
+     * bits order them unless two are equal there, which leaves a rank
+     * unoccupied; only then are the full values compared. */
+    int lt = 0;
     {
-        const int p = lane & 15, j0 = lane & 16 ? 8 : 0;
-        const uint32_t ah = (uint32_t)(sg_bits(a) >> 32), mine = (uint32_t)(sg_bits(a_all) >> 32);
+        const int j0 = lane & 16 ? 8 : 0;
+        const uint32_t ah = (uint32_t)(sg_bits(a) >> 32);
 #pragma unroll
-        for (int k = 0; k < 8; k++) {
-            const uint32_t hj = __shfl_sync(SG_FULL, ah, j0 + k);
-            lt += (hj < mine);
-            eq += (hj == mine);
-        }
-        eq += __shfl_xor_sync(SG_FULL, eq, 16) - 1; /* less the position itself */
-        if (__any_sync(SG_FULL, act && eq > 0)) {
-            lt = 0;
-            eq = 0;
-#pragma unroll
-            for (int k = 0; k < 8; k++) {
-                const double aj = __shfl_sync(SG_FULL, a, j0 + k);
-                lt += (aj < a_all);
-                eq += (aj == a_all) && (j0 + k != p);
-            }
-            eq += __shfl_xor_sync(SG_FULL, eq, 16);
-        }
+        for (int k = 0; k < 8; k++)
+            lt += __shfl_sync(SG_FULL, ah, j0 + k) < ah;
         lt += __shfl_xor_sync(SG_FULL, lt, 16);
-    }
-    /* ties (and NaN, which no comparison orders) take the exact quicksort */
-    if (!__any_sync(SG_FULL, act && (eq > 0 || a != a))) {
-        if (act)
-            ws->perm[lt] = (uint8_t)lane;
-    } else {
-        if (act) {
-            ws->qa[lane] = a;
-            ws->perm[lane] = (uint8_t)lane;
+        bool sorted = __reduce_or_sync(SG_FULL, a == a ? 1u << lt : 0u) == 0xffffu && __all_sync(SG_FULL, a == a);
+        if (!sorted) {
+            lt = 0;
+#pragma unroll 1
+            for (int k = 0; k < 8; k++)
+                lt += __shfl_sync(SG_FULL, a, j0 + k) < a;
+            lt += __shfl_xor_sync(SG_FULL, lt, 16);
+            sorted = __reduce_or_sync(SG_FULL, 1u << lt) == 0xffffu && __all_sync(SG_FULL, a == a);
         }
-        __syncwarp();
-        if (lane == 0)
-            sg_quicksort16(ws->qa, ws->perm);
+        /* ties (and NaN, which no comparison orders) take the exact quicksort */
+        if (sorted) {
+            if (act) {
+                ws->rank[lane] = (uint8_t)lt;
+                ws->qa[lt] = a;
+            }
+        } else {
+            if (act) {
+                ws->qa[lane] = a;
+                ws->perm[lane] = (uint8_t)lane;
+            }
+            __syncwarp();
+            if (lane == 0)
+                sg_quicksort16(ws->qa, ws->perm);
+            __syncwarp();
+            if (act)
+                ws->rank[ws->perm[lane]] = (uint8_t)lane;
+            __syncwarp();
+            lt = ws->rank[lane & 15];
+        }
     }
-    /* getPM_HD: the JacLog terms summed in position order; A[0..15] is free
-     * until the tables below are built */
-    if (act)
-        ws->A[lane] = jn;
+    /* by position: the JacLog terms (A[0..15] is free until the tables below
+     * are built); by sorted rank: increments and syndrome columns */
+    if (act) {
+        ws->A[lane] = jl;
+        ws->es[lt] = dl;
+        ws->hcol[2 * (lt & 7) + (lt >> 3)] = c_hcol[lane];
+    }
     __syncwarp();
+    /* getPM_HD: summed in position order */
     double pmhd = 0.0;
 #pragma unroll
     for (int i = 0; i < 8; i++) {
@@ -509,58 +514,55 @@ __device__ __forceinline__ SgLineResult sg_decode_line(double llr, const SgLineP
         pmhd = __dadd_rn(pmhd, v.x);
         pmhd = __dadd_rn(pmhd, v.y);
     }
-    __syncwarp();
-    const int src = act ? ws->perm[lane] : 0;
-    if (act)
-        ws->rank[src] = (uint8_t)lane;
-    const double as = __shfl_sync(SG_FULL, a, src);
 
-    /* IC (:619-622): beta = (|L|_(7) - |L|_(0)) / 7, IC = max(round(.), 0) */
-    const double a0 = __shfl_sync(SG_FULL, as, 0);
-    const double a7 = __shfl_sync(SG_FULL, as, 7);
-    const double beta = __ddiv_rn(__dsub_rn(a7, a0), 7.0);
-    int32_t ic = sg_cvt_i32(round(__dsub_rn(__ddiv_rn(a0, beta), 1.0)));
-    if (ic < 0)
-        ic = 0;
-    const int itab = ic < SG_ENUM_IC_CANON ? ic : SG_ENUM_IC_CANON;
-
-    /* PM increment of each sorted position (getPM, :765) and its syndrome */
-    const double jn_src = __shfl_sync(SG_FULL, jn, src);
-    const double jp_src = __shfl_sync(SG_FULL, jl, 16 + src); /* JacLog(|L|) of the same position */
-    const double dl = act ? __dsub_rn(jp_src, jn_src) : 0.0;
-    const uint32_t hs = act ? c_hcol[src] : 0u;
-    /* syndrome of the hard decision */
-    const uint32_t s0 = __reduce_xor_sync(SG_FULL, (act && ((hdm >> lane) & 1u)) ? (uint32_t)c_hcol[lane] : 0u);
+    /* IC (:619-622): beta = (|L|_(7) - |L|_(0)) / 7, IC = max(round(.), 0) of
+     * |L|_(0) / beta - 1.  Only the integer matters, and in single precision
+     * the quotient below 64 is good to 1e-4: the divisions are done only near
+     * a half, or outside single precision's range. */
+    int itab;
+    {
+        const double a0 = ws->qa[0], d70 = __dsub_rn(ws->qa[7], a0);
+        const float df = (float)d70, t = __fdividef(7.0f * (float)a0, df) - 1.0f, k = rintf(t);
+        if (df > 1e-30f && df < 1e30f && t < 64.0f && fabsf(t - k) < 0.499f) {
+            itab = max((int)k, 0);
+        } else {
+            const double beta = __ddiv_rn(d70, 7.0);
+            itab = max(sg_cvt_i32(round(__dsub_rn(__ddiv_rn(a0, beta), 1.0))), 0);
+        }
+        itab = min(itab, SG_ENUM_IC_CANON);
+    }
+    /* exp(-PM) needs no range check when no path metric of the line passes
+     * 700: JacLog(-|L|) and increment of a position add up to |L| + log 2 */
+    bool wide = false;
+    if (!(ws->qa[15] < 42.0)) {
+        double pmax = act ? dl : 0.0;
+        for (int off = 16; off > 0; off >>= 1)
+            pmax = __dadd_rn(pmax, __shfl_xor_sync(SG_FULL, pmax, off));
+        wide = !(pmax + pmhd < 700.0);
+    }
 
     /* per-line tables; lane j fills A entries j + 32*i, i = 0..7, and
      * syndrome entries 8*j + k, k = 0..7 */
     {
-        /* the increments by sorted rank, through es (free until the guess
-         * loop) */
-        if (act)
-            ws->es[lane] = dl;
-        __syncwarp();
         double d[8];
-        uint32_t hl[8], hh[8];
 #pragma unroll
         for (int b = 0; b < 8; b += 2) {
             const double2 v = reinterpret_cast<const double2*>(ws->es)[b / 2];
             d[b] = v.x;
             d[b + 1] = v.y;
         }
-#pragma unroll
-        for (int b = 0; b < 8; b++) {
-            hl[b] = __shfl_sync(SG_FULL, hs, b);
-            hh[b] = __shfl_sync(SG_FULL, hs, 8 + b);
-        }
+        const uint4 h = *reinterpret_cast<const uint4*>(ws->hcol); /* columns of bits b of the low and high byte: 16-bit b */
+        __syncwarp(); /* A, qa read before they are overwritten */
         double v0 = pmhd;
-        uint32_t sl = s0, sh = 0;
+        /* low byte: the hard decision's own syndrome, H = [P^T | I]; both:
+         * columns of the lane's bits */
+        uint32_t s = c_ptab[hdm & 0xffu] ^ (hdm >> 8);
+        const uint32_t h5[5] = {h.y >> 16, h.z, h.z >> 16, h.w, h.w >> 16};
 #pragma unroll
         for (int b = 0; b < 5; b++)
             if ((lane >> b) & 1) {
                 v0 = __dadd_rn(v0, d[b]);
-                sl ^= hl[3 + b];
-                sh ^= hh[3 + b];
+                s ^= h5[b];
             }
         const double v1 = __dadd_rn(v0, d[5]);
         const double v2 = __dadd_rn(v0, d[6]);
@@ -574,31 +576,27 @@ __device__ __forceinline__ SgLineResult sg_decode_line(double llr, const SgLineP
         ws->A[sg_swz(lane + 160)] = __dadd_rn(v1, d[7]);
         ws->A[sg_swz(lane + 192)] = __dadd_rn(v2, d[7]);
         ws->A[sg_swz(lane + 224)] = __dadd_rn(v3, d[7]);
-        /* byte k of the 8 entries 8*lane + k: the lane's syndrome (positions
-         * 3..7) XOR those of positions 0..2 selected by k, built in place
-         * in two 32-bit words (every value is below 256) */
-        const uint32_t lo0 = sl * 0x01010101u ^ hl[0] * 0x01000100u ^ hl[1] * 0x01010000u;
-        const uint32_t hi0 = sh * 0x01010101u ^ hh[0] * 0x01000100u ^ hh[1] * 0x01010000u;
+        /* byte k of the 8 entries 8*lane + k: the lane's syndrome (bits 3..7)
+         * XOR those of bits 0..2 selected by k, built in place in two 32-bit
+         * words by byte permutes */
+        const uint32_t lo0 = __byte_perm(s, 0u, 0x0000) ^ __byte_perm(h.x, 0u, 0x0404) ^ __byte_perm(h.x, 0u, 0x2244);
+        const uint32_t hi0 = __byte_perm(s, 0u, 0x1111) ^ __byte_perm(h.x, 0u, 0x1414) ^ __byte_perm(h.x, 0u, 0x3344);
         {
             /* stored at sg_swz(8*lane + k) = 8*lane' + (k ^ c): group lane' =
              * lane ^ (g >> 3), bytes permuted by c = g & 7, g the XOR value
              * of the group's bits 5..7 */
             const uint32_t g = (0x14AFEB50u >> (4 * (lane >> 2))) & 15u;
-            const uint32_t lo1 = lo0 ^ hl[2] * 0x01010101u;
+            const uint32_t lo1 = lo0 ^ __byte_perm(h.y, 0u, 0x0000);
             const uint32_t sel = 0x3210u ^ ((g & 3u) * 0x1111u);
             const uint32_t w0 = __byte_perm(lo0, 0u, sel), w1 = __byte_perm(lo1, 0u, sel);
             reinterpret_cast<uint2*>(ws->synlo)[lane ^ (g >> 3)] = (g & 4u) ? make_uint2(w1, w0) : make_uint2(w0, w1);
         }
-        reinterpret_cast<uint2*>(ws->synhi)[lane] = make_uint2(hi0, hi0 ^ hh[2] * 0x01010101u);
+        reinterpret_cast<uint2*>(ws->synhi)[lane] = make_uint2(hi0, hi0 ^ __byte_perm(h.y, 0u, 0x1111));
         if (lane < 9)
             ws->dz[lane] = lane ? ws->es[lane + 7] : 0.0;
     }
-    /* largest path metric of the line: exp(-PM) needs no range check below it */
-    double pmax = dl;
-    for (int off = 8; off > 0; off >>= 1)
-        pmax = __dadd_rn(pmax, __shfl_xor_sync(SG_FULL, pmax, off));
-    const bool wide = !(__shfl_sync(SG_FULL, pmax, 0) + pmhd < 700.0);
-    /* the sort is done with qa: it keeps the input LLRs for the soft output */
+    /* the sorted magnitudes are done with: qa keeps the input LLRs for the soft
+     * output */
     if (act)
         ws->qa[lane] = llr;
     if (lane == 0) {
@@ -778,22 +776,25 @@ __device__ __forceinline__ SgLineResult sg_decode_line(double llr, const SgLineP
         const int pos = lane & 15;
         const uint32_t rk = ws->rank[pos], hb = ws->hdm >> pos;
         const double pnlc = fmax(ws->pnl, 1e-40);
-        double pp1 = __ddiv_rn(1.0, __dadd_rn(1.0, ws->ex[pos]));
-        double pp0 = __dsub_rn(1.0, pp1);
-        pp1 = fmin(fmax(pp1, 1e-40), 1.0);
-        pp0 = fmin(fmax(pp0, 1e-40), 1.0);
+        /* 1/(1 + e^L) and its complement are at most 1, so only the lower
+         * clamps of :541-:548 can act */
+        const double q1 = __drcp_rn(__dadd_rn(1.0, ws->ex[pos]));
+        const double pp0 = fmax(__dsub_rn(1.0, q1), 1e-40), pp1 = fmax(q1, 1e-40);
         double p1 = 0.0, p0 = 0.0;
         for (int j = 0; j < curl; j++) {
-            /* AddTEP (:761): position i flips when its sorted rank is in the pattern */
-            const double c = (double)(((ws->lst_m[j] >> rk) ^ hb) & 1u);
+            /* AddTEP (:761): position i flips when its sorted rank is in the
+             * pattern.  The reference adds c * p_j and (1 - c) * p_j; the
+             * zero one changes nothing. */
             const double pj = ws->lst_e[j];
-            p1 = __dadd_rn(p1, __dmul_rn(c, pj));
-            p0 = __dadd_rn(p0, __dmul_rn(__dsub_rn(1.0, c), pj));
+            if (((ws->lst_m[j] >> rk) ^ hb) & 1u)
+                p1 = __dadd_rn(p1, pj);
+            else
+                p0 = __dadd_rn(p0, pj);
         }
         p0 = __dadd_rn(p0, __dmul_rn(pnlc, pp0));
         p1 = __dadd_rn(p1, __dmul_rn(pnlc, pp1));
-        const double lg = sg_dec_log<CR>(fmax(act ? p0 : p1, 1e-40), ltab);
-        lapp = __dsub_rn(lg, __shfl_sync(SG_FULL, lg, (lane & 15) + 16));
+        const double lg = sg_dec_log_pos<CR>(fmax(act ? p0 : p1, 1e-40), ltab);
+        lapp = __dsub_rn(lg, __shfl_down_sync(SG_FULL, lg, 16));
         le = __dsub_rn(lapp, x);
     }
     res.lapp = lapp;

@@ -176,13 +176,10 @@ SG_HD double sg_exp(double x, SgTab tab)
     return e > 0 ? y * 0x1p64 : y * 0x1p-64;
 }
 
-/* exp(x) for x <= 0, bit-identical to sg_exp: the same operations without
- * the range checks that cannot fire for arguments above -707.5 (the guess
- * loop's exp(-PM), PM >= 0). */
-SG_HD double sg_exp_neg(double x, SgTab tab)
+/* exp(x) for |x| <= 707.5, bit-identical to sg_exp: the same operations
+ * without its range checks. */
+SG_HD double sg_exp_mid(double x, SgTab tab)
 {
-    if (x < -707.5)
-        return sg_exp(x, tab);
     double z = x * SG_EXP_INV_LN2_N;
     double kd = z + SG_EXP_SHIFT;
     int k = (int)(uint32_t)sg_bits(kd);
@@ -209,6 +206,9 @@ SG_HD double sg_exp_neg(double x, SgTab tab)
     return sg_fma(S, tmp, S);
 }
 
+/* exp(x) for x <= 0 (the guess loop's exp(-PM), PM >= 0). */
+SG_HD double sg_exp_neg(double x, SgTab tab) { return x < -707.5 ? sg_exp(x, tab) : sg_exp_mid(x, tab); }
+
 /* TwoSum: s + err == a + b exactly. */
 SG_HD double sg_two_sum(double a, double b, double* err)
 {
@@ -220,6 +220,7 @@ SG_HD double sg_two_sum(double a, double b, double* err)
 
 /* log(x), round-to-nearest result within ~0.502 ulp.
  * tab: SG_LOG_TAB_LEN doubles, {c_j, hi(-log c_j), lo(-log c_j)}. */
+SG_HD double sg_log_core(uint64_t ix, int escale, SgTab tab);
 SG_HD double sg_log(double x, SgTab tab)
 {
     uint64_t ix = sg_bits(x);
@@ -236,6 +237,13 @@ SG_HD double sg_log(double x, SgTab tab)
         ix = sg_bits(x);
         escale = -52;
     }
+    return sg_log_core(ix, escale, tab);
+}
+
+/* log of the positive normal number with bit pattern ix, plus escale ln 2
+ * (escale 0: sg_log of it, without the checks for other arguments). */
+SG_HD double sg_log_core(uint64_t ix, int escale, SgTab tab)
+{
     uint64_t tmpb = ix - SG_LOG_OFF;
     int j = (int)((tmpb >> 45) & 127);
     int e = (int)((int64_t)tmpb >> 52) + escale;

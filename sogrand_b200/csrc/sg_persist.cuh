@@ -232,9 +232,8 @@ __global__ void __launch_bounds__(NW * 32, 1) sg_persist_kernel(const __grid_con
         const double alpha = args.alpha[phase];
         const double* g = args.llr + (size_t)cw * SG_CUBE;
         const int pos = sg_pos(axis, l, lane & 15);
-        double v = 1.0;
-        if (lane < 16) /* L_ch + (alpha*L_E) */
-            v = __dadd_rn(__ldg(g + pos), __dmul_rn(alpha, sl.le[pos]));
+        /* L_ch + (alpha*L_E), lanes p and p + 16 alike */
+        const double v = __dadd_rn(__ldg(g + pos), __dmul_rn(alpha, sl.le[pos]));
         const SgLineResult r = sg_decode_line<false, CR>(v, lp, args.enum_tabs, etab, ltab, &S.ws[warp]);
         if (lane < 16) {
             sl.le[pos] = r.le;
