@@ -114,7 +114,6 @@ struct SgBackSmem {
     double gle[SG_CUBE]; /* d loss / d L_E of the phase being processed */
     SgEtab<false> etab;
     alignas(16) double ltab[SG_LOG_TAB_LEN];
-    SgExpK ek;
     SgWarpScratch ws[NW];
     double ga;   /* d loss / d alpha of the phase */
     double lsum; /* loss of the codeword */
@@ -133,9 +132,6 @@ __global__ void __launch_bounds__(NW * 32, 3) sg_backward_kernel(const __grid_co
     SgLineParams lp;
     lp.L = args.L;
     lp.meta = &args.meta;
-    lp.ek = &S.ek;
-    if (tid == 0)
-        S.ek = sg_exp_k();
     lp.thres = args.thres;
     const SgTab etab = sg_etab_of<false, false>(S.etab, args.k.v), ltab{S.ltab, args.k.v};
     __syncthreads();

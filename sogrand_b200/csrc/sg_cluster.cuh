@@ -24,7 +24,6 @@ struct SgClusterSmem {
     double le[SG_CUBE];
     SgEtab<true> etab;
     alignas(16) double ltab[SG_LOG_TAB_LEN];
-    SgExpK ek;
     SgWarpScratch ws[NW];
     uint16_t hdw[2][256];
     unsigned long long ng;   /* rank 0: guesses of the codeword */
@@ -70,7 +69,6 @@ __global__ void __launch_bounds__(NW * 32, 1) sg_cluster_kernel(const __grid_con
     for (int i = tid; i < SG_CUBE; i += NT)
         nonfinite |= !isfinite(__ldg(g + i));
     if (tid == 0) {
-        S.ek = sg_exp_k();
         S.ng = 0;
         S.ngmax[0] = S.ngmax[1] = 0;
         S.line_next[0] = S.line_next[1] = 0;
@@ -82,7 +80,7 @@ __global__ void __launch_bounds__(NW * 32, 1) sg_cluster_kernel(const __grid_con
         return;
     }
     const SgTab etab = sg_etab_of<CR, true>(S.etab, args.k.v), ltab{S.ltab, args.k.v};
-    const SgLineParams lp{args.L, args.thres, &args.meta, &S.ek};
+    const SgLineParams lp{args.L, args.thres, &args.meta};
     const uint32_t le_a = sg_saddr(S.le);
     const uint32_t ng_a = sg_mapa(sg_saddr(&S.ng), 0), ngmax_a = sg_mapa(sg_saddr(S.ngmax), 0);
     const uint32_t hdw_a = sg_mapa(sg_saddr(S.hdw), lane % CS);

@@ -109,7 +109,6 @@ struct SgCwSmem {
     static constexpr bool T8 = NW * LPW >= 16 && !LCH_SMEM;
     SgEtab<T8> etab;
     alignas(16) double ltab[SG_LOG_TAB_LEN];
-    SgExpK ek;
     SgWarpScratch ws[NW * LPW];
     uint16_t hdw[256];
     unsigned long long mbar;
@@ -183,8 +182,6 @@ __global__ void __launch_bounds__(NW * 32, MINB) sg_decode_kernel(const __grid_c
     sg_etab_fill<CR, T8>(S.etab, g_etab, tid, NT);
     for (int i = tid; i < SG_LOG_TAB_LEN; i += NT)
         S.ltab[i] = g_ltab[i];
-    if (tid == 0)
-        S.ek = sg_exp_k();
     const uint32_t mbar = sg_smem_u32(&S.mbar);
     if (tid == 0 && use_bulk) {
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(mbar) : "memory");
@@ -196,7 +193,6 @@ __global__ void __launch_bounds__(NW * 32, MINB) sg_decode_kernel(const __grid_c
     SgLineParams lp;
     lp.L = args.L;
     lp.meta = &args.meta;
-    lp.ek = &S.ek;
     lp.thres = args.thres;
 
     for (unsigned long long cw = blockIdx.x; cw < args.n_cw; cw += gridDim.x) {
@@ -376,7 +372,6 @@ template <int NW, bool T8>
 struct SgLineSmem {
     SgEtab<T8> etab;
     alignas(16) double ltab[SG_LOG_TAB_LEN];
-    SgExpK ek;
     int next; /* of the CTA's lines, the next to hand out */
     SgWarpScratch ws[NW];
 };
@@ -393,13 +388,12 @@ __global__ void __launch_bounds__(NW * 32, NW == 16 ? 2 : 1)
 {
     SgLineSmem<NW, T8>& S = *reinterpret_cast<SgLineSmem<NW, T8>*>(sg_smem_raw);
     const SgTab etab = sg_etab_of<CR, T8>(S.etab, k.v), ltab{S.ltab, k.v};
-    const SgLineParams lp{L, thres, &meta, &S.ek};
+    const SgLineParams lp{L, thres, &meta};
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     sg_etab_fill<CR, T8>(S.etab, g_etab, tid, NW * 32);
     for (int i = tid; i < SG_LOG_TAB_LEN; i += NW * 32)
         S.ltab[i] = g_ltab[i];
     if (tid == 0) {
-        S.ek = sg_exp_k();
         S.next = 0;
     }
     __syncthreads();

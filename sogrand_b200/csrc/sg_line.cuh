@@ -111,15 +111,22 @@ __device__ __forceinline__ double2 sg_lds_f64x2(uint32_t a)
     return v;
 }
 
-/* The constants of sg_exp_neg, read from the kernel's shared memory copy
- * once per line: a value that came from memory stays in its registers
- * through the guess loop. */
-struct alignas(16) SgExpK {
+/* The constants of sg_exp_neg, in constant memory. */
+struct SgExpK {
     double inv, ln2_hi, ln2_lo, c3, c4, c5, c6, c7;
 };
+__constant__ __align__(16) SgExpK sg_exp_consts = {SG_EXP_INV_LN2_N, SG_EXP_LN2_N_HI, SG_EXP_LN2_N_LO, SG_EXP_C3,
+                                     SG_EXP_C4,        SG_EXP_C5,       SG_EXP_C6,       SG_EXP_C7};
+/* Volatile loads: literals, or plain loads, the compiler would put together
+ * again in every step of the guess loop. */
 __device__ __forceinline__ SgExpK sg_exp_k()
 {
-    return {SG_EXP_INV_LN2_N, SG_EXP_LN2_N_HI, SG_EXP_LN2_N_LO, SG_EXP_C3, SG_EXP_C4, SG_EXP_C5, SG_EXP_C6, SG_EXP_C7};
+    SgExpK k;
+    asm volatile("ld.const.v2.f64 {%0, %1}, [sg_exp_consts];" : "=d"(k.inv), "=d"(k.ln2_hi));
+    asm volatile("ld.const.v2.f64 {%0, %1}, [sg_exp_consts + 16];" : "=d"(k.ln2_lo), "=d"(k.c3));
+    asm volatile("ld.const.v2.f64 {%0, %1}, [sg_exp_consts + 32];" : "=d"(k.c4), "=d"(k.c5));
+    asm volatile("ld.const.v2.f64 {%0, %1}, [sg_exp_consts + 48];" : "=d"(k.c6), "=d"(k.c7));
+    return k;
 }
 
 /* A kernel's exp table in shared memory: T8 -- eight copies, with the
@@ -179,7 +186,6 @@ struct SgLineParams {
     int32_t L;
     double thres;
     const sg_order_meta* meta; /* per IC, Tmax included */
-    const SgExpK* ek;          /* shared memory copy */
 };
 
 /* Per-warp shared scratch of one line decode. */
@@ -657,7 +663,7 @@ __device__ __forceinline__ SgLineResult sg_decode_line(double llr, const SgLineP
         double e;
         uint64_t tot;
         bool out = false, hit, tie;
-        const SgExpK ek = *lp.ek;
+        const SgExpK ek = sg_exp_k();
         /* P is moved by the step's units.  2^26 in place of the upper half of
          * a lane that cannot be summed, or that holds a codeword, makes them
          * 2^52 or more, which leaves the binade. */

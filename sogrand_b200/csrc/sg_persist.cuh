@@ -38,7 +38,6 @@ struct SgPersistSmem {
     SgSlot slot[C];
     SgEtab<true> etab;
     alignas(16) double ltab[SG_LOG_TAB_LEN];
-    SgExpK ek;
     SgWarpScratch ws[NW];
 };
 
@@ -158,8 +157,6 @@ __global__ void __launch_bounds__(NW * 32, 1) sg_persist_kernel(const __grid_con
     sg_etab_fill<CR, true>(S.etab, g_etab, tid, NT);
     for (int i = tid; i < SG_LOG_TAB_LEN; i += NT)
         S.ltab[i] = g_ltab[i];
-    if (tid == 0)
-        S.ek = sg_exp_k();
     if (tid < C) {
         S.slot[tid].cw = -1;
         S.slot[tid].next = 256;
@@ -174,7 +171,6 @@ __global__ void __launch_bounds__(NW * 32, 1) sg_persist_kernel(const __grid_con
     SgLineParams lp;
     lp.L = args.L;
     lp.meta = &args.meta;
-    lp.ek = &S.ek;
     lp.thres = args.thres;
     const int nphase = 3 * args.imax;
     int idle = 0;
