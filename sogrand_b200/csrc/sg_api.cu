@@ -31,110 +31,137 @@
 #include "sg_kernels.cuh"
 #include "sg_adjoint.cuh"
 
-__global__ void __launch_bounds__(SG_THREADS) sg_gen_kernel(uint64_t seed, uint64_t cw0,
-                                                             unsigned long long n_cw, double sigma,
-                                                             double lo, double hi, uint8_t* info,
-                                                             double* llr, const __grid_constant__ SgK k)
+struct SgGenSmem {
+    alignas(16) double etab[SG_EXP_TAB_LEN];
+    alignas(16) double ltab[SG_LOG_TAB_LEN];
+    alignas(16) ulonglong2 key[SG_POLAR_TRIES]; /* of the two noise streams of each attempt */
+    double u[SG_CUBE];                          /* accepted pairs: u, and u^2 + v^2 */
+    double ss[SG_CUBE];
+    uint16_t W[256];
+    uint8_t ib[SG_INFO_BYTES];
+    uint8_t prow[8];
+    uint8_t ptab[256];
+};
+
+/* a / b correctly rounded, y = 1 / b correctly rounded, for quotients and
+ * remainders in the normal range: two corrections of a * y by the exact
+ * remainder (P. Markstein, "Computation of elementary functions on the IBM RISC
+ * System/6000 processor", IBM J. Res. Dev. 34(1), 1990). */
+__device__ __forceinline__ double sg_div_by(double a, double b, double y)
 {
-    __shared__ alignas(16) double etab_s[SG_EXP_TAB_LEN];
-    __shared__ alignas(16) double ltab_s[SG_LOG_TAB_LEN];
-    const SgTab etab{etab_s, k.v}, ltab{ltab_s, k.v};
-    __shared__ uint16_t W[256];
-    __shared__ alignas(16) double stage[SG_CUBE]; /* the codeword's LLRs, stored coalesced */
-    __shared__ uint8_t ib[SG_INFO_BYTES];
-    __shared__ uint8_t prow[8];
-    __shared__ uint8_t ptab[256];
+    double q = __dmul_rn(a, y);
+    q = __fma_rn(__fma_rn(-q, b, a), y, q);
+    return __fma_rn(__fma_rn(-q, b, a), y, q);
+}
+
+/* sg_sym_unit from bits 11..63: 1 + (bits 11..62) 2^-52, less 1 or 2 by bit
+ * 63; exact. */
+__device__ __forceinline__ double sg_sym_unit_bits(uint64_t r)
+{
+    const uint32_t hi = (uint32_t)(r >> 32);
+    const double d = __hiloint2double((int)(0x3ff00000u | ((hi >> 11) & 0xfffffu)), (int)__funnelshift_r((uint32_t)r, hi, 11));
+    return __dsub_rn(d, (int32_t)hi < 0 ? 1.0 : 2.0);
+}
+
+/* Seeded codewords and their channel LLRs.  Two passes over a thread's 16
+ * positions p = tid + 256 q: the polar attempts, as one stream (a lane moves
+ * to its next position when a pair is accepted, so a warp does not wait,
+ * position by position, for its unluckiest lane), then log, square root and
+ * divisions of the accepted pairs with every lane busy.  Each position keeps
+ * its first accepted attempt (after SG_POLAR_TRIES rejections, 0), as
+ * sg_normal does.  Bound by issue slots: one attempt is two 64-bit hashes;
+ * keyed per attempt once per CTA, not per sample, and with unit and quotient
+ * from bits and remainders, 20 000 codewords take 0.88 ms (1.37 ms with one
+ * pass, four hashes per attempt and three library divisions per sample). */
+__global__ void __launch_bounds__(SG_THREADS, 3) sg_gen_kernel(uint64_t seed, uint64_t cw0, unsigned long long n_cw,
+                                                               double sigma, double lo, double hi, uint8_t* info,
+                                                               double* llr, const __grid_constant__ SgK k)
+{
+    SgGenSmem& S = *reinterpret_cast<SgGenSmem*>(sg_smem_raw);
+    const SgTab etab{S.etab, k.v}, ltab{S.ltab, k.v};
     const int tid = threadIdx.x;
     for (int i = tid; i < SG_EXP_TAB_LEN; i += SG_THREADS)
-        etab_s[i] = g_etab[i];
+        S.etab[i] = g_etab[i];
     for (int i = tid; i < SG_LOG_TAB_LEN; i += SG_THREADS)
-        ltab_s[i] = g_ltab[i];
+        S.ltab[i] = g_ltab[i];
+    if (tid < SG_POLAR_TRIES)
+        S.key[tid] = make_ulonglong2(sg_rand_key(seed, 1 + 2 * tid), sg_rand_key(seed, 2 + 2 * tid));
     if (tid < 8)
-        prow[tid] = c_prow[tid];
-    ptab[tid] = c_ptab[tid];
+        S.prow[tid] = c_prow[tid];
+    S.ptab[tid] = c_ptab[tid];
     __syncthreads();
     for (unsigned long long c = blockIdx.x; c < n_cw; c += gridDim.x) {
         const uint64_t gc = cw0 + c;
         if (tid < 8) {
             const uint64_t r = sg_rand(seed, 0, gc * 8 + tid);
             for (int q = 0; q < 8; q++)
-                ib[tid * 8 + q] = (uint8_t)(r >> (8 * q));
+                S.ib[tid * 8 + q] = (uint8_t)(r >> (8 * q));
         }
         __syncthreads();
         /* sg_encode_words, each of its four stages spread over the block:
          * info words, parity columns of the first 8 slices, parity rows,
          * parity slices (the same words, every one written once) */
         if (tid < 64)
-            W[(tid >> 3) * 16 + (tid & 7)] = (uint16_t)sg_brev8(ib[tid]);
+            S.W[(tid >> 3) * 16 + (tid & 7)] = (uint16_t)sg_brev8(S.ib[tid]);
         __syncthreads();
         if (tid < 64) {
             const int l = tid >> 3, jj = tid & 7;
             uint16_t acc = 0;
             for (int j = 0; j < 8; j++)
-                if ((prow[j] >> jj) & 1)
-                    acc ^= W[l * 16 + j];
-            W[l * 16 + 8 + jj] = acc;
+                if ((S.prow[j] >> jj) & 1)
+                    acc ^= S.W[l * 16 + j];
+            S.W[l * 16 + 8 + jj] = acc;
         }
         __syncthreads();
         if (tid < 128) {
-            const uint16_t x = W[tid];
-            W[tid] = (uint16_t)((x & 0xff) | (ptab[x & 0xff] << 8));
+            const uint16_t x = S.W[tid];
+            S.W[tid] = (uint16_t)((x & 0xff) | (S.ptab[x & 0xff] << 8));
         }
         __syncthreads();
         if (tid < 128) {
             const int jj = tid >> 4, j = tid & 15;
             uint16_t acc = 0;
             for (int l = 0; l < 8; l++)
-                if ((prow[l] >> jj) & 1)
-                    acc ^= W[l * 16 + j];
-            W[(8 + jj) * 16 + j] = acc;
+                if ((S.prow[l] >> jj) & 1)
+                    acc ^= S.W[l * 16 + j];
+            S.W[(8 + jj) * 16 + j] = acc;
         }
         if (info && tid < SG_INFO_BYTES)
-            info[c * SG_INFO_BYTES + tid] = ib[tid];
+            info[c * SG_INFO_BYTES + tid] = S.ib[tid];
         __syncthreads();
         const double s = sigma > 0.0 ? sigma : sg_sigma_draw(seed, gc, lo, hi, etab);
-        /* sg_normal for this thread's 16 positions p = tid + 256k, taken as
-         * one stream of polar attempts: every pass makes one attempt for every
-         * lane and a lane moves to its next position when its pair is
-         * accepted, so a warp no longer waits, position by position, for its
-         * unluckiest lane.  Each position keeps its first accepted attempt
-         * (after SG_POLAR_TRIES rejections, 0), as sg_normal does; the LLRs
-         * are staged in shared memory and stored coalesced. */
-        int q = 0;
-        uint64_t att = 0;
-        while (q < SG_CUBE / SG_THREADS) {
-            const uint32_t p = (uint32_t)(tid + SG_THREADS * q);
-            const uint64_t ctr = gc * 4096u + p;
-            const double u = sg_sym_unit(sg_rand(seed, 1 + 2 * att, ctr));
-            const double v = sg_sym_unit(sg_rand(seed, 2 + 2 * att, ctr));
-            const double uu = u * u;
-            const double vv = v * v;
-            const double ss = uu + vv;
+        uint64_t base = sg_rand_ctr(gc * 4096u + tid);
+        for (int p = tid, att = 0; p < SG_CUBE;) {
+            const ulonglong2 key = S.key[att];
+            const double u = sg_sym_unit_bits(sg_mix64(key.x ^ base));
+            const double v = sg_sym_unit_bits(sg_mix64(key.y ^ base));
+            const double ss = __dadd_rn(__dmul_rn(u, u), __dmul_rn(v, v));
             const bool ok = ss > 0.0 && ss < 1.0;
             if (ok || att + 1 == SG_POLAR_TRIES) {
-                double z = 0.0;
-                if (ok) {
-                    const double l = sg_log(ss, ltab);
-                    const double m = -2.0 * l;
-                    const double ms = m / ss;
-                    z = u * __dsqrt_rn(ms);
-                }
-                const int bit = (W[p >> 4] >> (p & 15)) & 1;
-                stage[p] = sg_llr_of(bit, s, z);
-                q++;
+                S.u[p] = u;
+                S.ss[p] = ok ? ss : 2.0;
+                p += SG_THREADS;
+                base += (uint64_t)SG_THREADS * SG_RAND_CTR_MUL;
                 att = 0;
             } else {
                 att++;
             }
         }
-        __syncthreads();
+        const double var = __dmul_rn(s, s), rvar = __drcp_rn(var);
+        const bool mid = var > 0x1p-400 && var < 0x1p400; /* noise and quotient stay normal */
         double* out = llr + c * SG_CUBE;
-        if (((uintptr_t)llr & 15u) == 0) {
-            for (int q = tid; q < SG_CUBE / 2; q += SG_THREADS)
-                reinterpret_cast<double2*>(out)[q] = reinterpret_cast<const double2*>(stage)[q];
-        } else {
-            for (int q = tid; q < SG_CUBE; q += SG_THREADS)
-                out[q] = stage[q];
+#pragma unroll 2
+        for (int q = 0; q < SG_CUBE / SG_THREADS; q++) {
+            const int p = tid + SG_THREADS * q;
+            const double ss = S.ss[p];
+            double z = 0.0;
+            if (ss < 1.0) {
+                const double m = __dmul_rn(-2.0, sg_log_core(sg_bits(ss), 0, ltab));
+                z = __dmul_rn(S.u[p], __dsqrt_rn(sg_div_by(m, ss, __drcp_rn(ss))));
+            }
+            /* sg_llr_of */
+            const double y2 = __dmul_rn(2.0, __dadd_rn((S.W[p >> 4] >> (p & 15)) & 1 ? -1.0 : 1.0, __dmul_rn(s, z)));
+            out[p] = mid ? sg_div_by(y2, var, rvar) : __ddiv_rn(y2, var);
         }
         __syncthreads();
     }
@@ -473,6 +500,7 @@ sg_status get_ctx(DevCtx** out)
             for (bool cr : {false, true})
                 SG_CUDA(cudaFuncSetAttribute(bitso_fn(v, cr), cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              (int)k_bvariants[v].smem));
+        SG_CUDA(cudaFuncSetAttribute(sg_gen_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SgGenSmem)));
         SG_CUDA(cudaFuncSetAttribute(sg_backward_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)sizeof(SgBackSmem<8>)));
         SG_CUDA(cudaDeviceGetAttribute(&c.sms, cudaDevAttrMultiProcessorCount, dev));
@@ -849,7 +877,7 @@ sg_status sg_gen_llr_device(uint64_t seed, uint64_t cw0, size_t n_cw, double sig
     sg_status s = get_ctx(&c);
     if (s != SG_OK)
         return s;
-    sg_gen_kernel<<<grid_for(n_cw, 148 * 16), SG_THREADS, 0, (cudaStream_t)stream>>>(
+    sg_gen_kernel<<<grid_for(n_cw, 148 * 16), SG_THREADS, sizeof(SgGenSmem), (cudaStream_t)stream>>>(
         seed, cw0, n_cw, sigma, ebn0_lo_db, ebn0_hi_db, d_info, d_llr, k_consts);
     SG_CUDA(cudaGetLastError());
     return SG_OK;

@@ -28,10 +28,17 @@ SG_HD uint64_t sg_mix64(uint64_t z)
     return z;
 }
 
+/* the stream's key and the counter's word of sg_rand */
+#define SG_RAND_CTR_MUL 0xd1b54a32d192ed03ULL
+SG_HD uint64_t sg_rand_key(uint64_t seed, uint64_t stream)
+{
+    return sg_mix64(seed + 0x9e3779b97f4a7c15ULL * (stream + 1));
+}
+SG_HD uint64_t sg_rand_ctr(uint64_t ctr) { return ctr * SG_RAND_CTR_MUL + 0x8cb92ba72f3d8dd7ULL; }
+
 SG_HD uint64_t sg_rand(uint64_t seed, uint64_t stream, uint64_t ctr)
 {
-    uint64_t k = sg_mix64(seed + 0x9e3779b97f4a7c15ULL * (stream + 1));
-    return sg_mix64(k ^ (ctr * 0xd1b54a32d192ed03ULL + 0x8cb92ba72f3d8dd7ULL));
+    return sg_mix64(sg_rand_key(seed, stream) ^ sg_rand_ctr(ctr));
 }
 
 /* uniform in [-1, 1) with 2^-52 spacing */
