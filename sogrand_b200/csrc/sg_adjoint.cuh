@@ -120,8 +120,11 @@ struct SgBackSmem {
     int line_next;
 };
 
-template <int NW>
-__global__ void __launch_bounds__(NW * 32, 3) sg_backward_kernel(const __grid_constant__ SgBackwardArgs args)
+/* MINB CTAs of NW warps per SM: 24 warps either way, the most with 80
+ * registers.  The sums over the counted guesses take 34 of them; at 64
+ * (32 warps) they spill. */
+template <int NW, int MINB>
+__global__ void __launch_bounds__(NW * 32, MINB) sg_backward_kernel(const __grid_constant__ SgBackwardArgs args)
 {
     constexpr int NT = NW * 32;
     SgBackSmem<NW>& S = *reinterpret_cast<SgBackSmem<NW>*>(sg_smem_raw);
