@@ -105,7 +105,7 @@ __global__ void __launch_bounds__(NW * 32, 1) sg_cluster_kernel(const __grid_con
             const double v = __dadd_rn(__ldg(g + pos), __dmul_rn(alpha, le0));
             if (args.ckpt && lane < 16)
                 args.ckpt[(cw * (unsigned long long)nphase + phase) * SG_CUBE + pos] = le0;
-            const SgLineResult r = sg_decode_line<false, CR, true>(v, lp, args.enum_tabs, etab, ltab, &S.ws[warp]);
+            const SgLineResult r = sg_decode_line<false, CR, true, NW <= 16 ? 2 : 1>(v, lp, args.enum_tabs, etab, ltab, &S.ws[warp]);
             if (lane < 16) {
                 const uint32_t a = sg_mapa(le_a + 8u * (uint32_t)pos, sg_line_of(axis_next, pos) / LPC);
                 asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(a), "d"(r.le) : "memory");

@@ -418,7 +418,7 @@ __global__ void __launch_bounds__(NW * 32, NW == 16 ? 2 : 1)
             }
             continue;
         }
-        const SgLineResult r = sg_decode_line<false, CR, T8>(v, lp, enum_tabs, etab, ltab, &S.ws[warp]);
+        const SgLineResult r = sg_decode_line<false, CR, T8, NW <= 4 ? 2 : 1>(v, lp, enum_tabs, etab, ltab, &S.ws[warp]);
         if (lane < 16) {
             lapp[l * 16 + lane] = r.lapp;
             le[l * 16 + lane] = r.le;
