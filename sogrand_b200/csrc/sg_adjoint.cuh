@@ -27,67 +27,56 @@
  */
 #pragma once
 
-/* sum over lanes 0..15 (lanes 16..31 contribute 0), result in all lanes */
-__device__ __forceinline__ double sg_sum16(double v, int lane)
+/* sum over positions, lanes p and p + 16 holding position p's term alike */
+__device__ __forceinline__ double sg_sum16(double v)
 {
-    v = lane < 16 ? v : 0.0;
-    for (int off = 16; off > 0; off >>= 1)
+    for (int off = 8; off > 0; off >>= 1)
         v += __shfl_xor_sync(SG_FULL, v, off);
     return v;
 }
 
-/* Gradient with respect to the line input x (lanes 0..15) of g . L_APP,
- * g the upstream gradient of L_APP (lanes 0..15). */
-__device__ __forceinline__ double sg_line_vjp(double x, double g, const SgAdjOut& a, SgTab etab, int lane)
+/* Gradient with respect to the line input x of g . L_APP, g the upstream
+ * gradient of L_APP; lanes p and p + 16 hold position p alike.  The soft
+ * output's exp, reciprocal and sums come from the decode. */
+__device__ __forceinline__ double sg_line_vjp(double x, double g, const SgAdjOut& a, int lane)
 {
-    const bool act = lane < 16;
     if (a.curl == 0)
-        return act ? g : 0.0; /* L_APP = x */
+        return g; /* L_APP = x */
+    const bool low = lane < 16;
+    const int pos = lane & 15;
     const double eps = 1e-40;
     const bool pnl_live = a.pnl > eps;
     const double p_nl = fmax(a.pnl, eps);
-    const double ex = sg_exp(act ? x : 0.0, etab);
-    const double pp1r = 1.0 / (1.0 + ex);
-    const double pp0r = 1.0 - pp1r;
-    const double pp1 = fmin(fmax(pp1r, eps), 1.0);
-    const double pp0 = fmin(fmax(pp0r, eps), 1.0);
-    double p0 = 0.0, p1 = 0.0;
-    for (int j = 0; j < a.curl; j++) {
-        const double pj = __shfl_sync(SG_FULL, a.my_e, j);
-        const uint32_t cj = (__shfl_sync(SG_FULL, a.my_cm, j) >> (lane & 15)) & 1u;
-        if (cj)
-            p1 += pj;
-        else
-            p0 += pj;
-    }
-    p0 += p_nl * pp0;
-    p1 += p_nl * pp1;
-    const double a0 = (act && p0 > eps) ? g / p0 : 0.0;
-    const double a1 = (act && p1 > eps) ? -g / p1 : 0.0;
+    const double pp1r = a.q1, pp0r = 1.0 - pp1r;
+    const double pp1 = fmax(pp1r, eps), pp0 = fmax(pp0r, eps); /* at most 1 */
+    /* g / p0 on the low lanes, -g / p1 on the high ones */
+    const double pm = low ? a.p0 : a.p1;
+    const double mine = pm > eps ? (low ? g : -g) / pm : 0.0, other = __shfl_xor_sync(SG_FULL, mine, 16);
+    const double a0 = low ? mine : other, a1 = low ? other : mine;
     const double dsig = pp0r * pp1r; /* d pp0/dx = -d pp1/dx */
     double gx = 0.0;
     if (pp0r > eps)
         gx += a0 * p_nl * dsig;
     if (pp1r > eps)
         gx -= a1 * p_nl * dsig;
-    const double ax = fabs(x);
     const double sgn = x > 0.0 ? 1.0 : (x < 0.0 ? -1.0 : 0.0);
-    const double sm = ax <= 50.0 ? 1.0 / (1.0 + sg_exp(ax, etab)) : 0.0; /* sigma(-|x|) */
+    /* sigma(-|x|): 1/(1 + e^x) for x > 0, e^x/(1 + e^x) otherwise */
+    const double sm = fabs(x) <= 50.0 ? (x > 0.0 ? pp1r : a.ex * pp1r) : 0.0;
     for (int j = 0; j < a.curl; j++) {
         const double pj = __shfl_sync(SG_FULL, a.my_e, j);
         const uint32_t cm = __shfl_sync(SG_FULL, a.my_cm, j);
-        const uint32_t cj = (cm >> (lane & 15)) & 1u;
-        const double gpj = sg_sum16(cj ? a1 : a0, lane);
+        const uint32_t cj = (cm >> pos) & 1u;
+        const double gpj = sg_sum16(cj ? a1 : a0);
         const double gpm = -pj * gpj;
-        const double inS = (((cm ^ a.hdm) >> (lane & 15)) & 1u) ? 1.0 : 0.0;
+        const double inS = (((cm ^ a.hdm) >> pos) & 1u) ? 1.0 : 0.0;
         gx += gpm * sgn * (inS - sm);
     }
     if (pnl_live) {
-        const double gpnl = sg_sum16(a0 * pp0 + a1 * pp1, lane);
-        const double ei = __shfl_sync(SG_FULL, a.esort, a.myrank & 15);
+        const double gpnl = sg_sum16(a0 * pp0 + a1 * pp1);
+        const double ei = __shfl_sync(SG_FULL, a.esort, a.myrank);
         gx += gpnl * 0x1p-8 * sgn * (ei - sm * a.etot);
     }
-    return act ? gx : 0.0;
+    return gx;
 }
 
 struct SgBackwardArgs {
@@ -161,6 +150,8 @@ __global__ void __launch_bounds__(NW * 32, MINB) sg_backward_kernel(const __grid
                 S.ga = 0.0;
             }
             __syncthreads();
+            const bool scored = p == P - 1 || args.loss_mode == 1;
+            double ga = 0.0, ls = 0.0; /* the lane's shares of the phase's sums */
             for (;;) {
                 int l = 0;
                 if (lane == 0)
@@ -172,29 +163,32 @@ __global__ void __launch_bounds__(NW * 32, MINB) sg_backward_kernel(const __grid
                 const double lep = ck[pos];
                 const double x = __dadd_rn(g[pos], __dmul_rn(alpha, lep));
                 SgAdjOut a;
+                a.want_app = scored;
                 const SgLineResult r = sg_decode_line<true, false, true>(x, lp, args.enum_tabs, etab, ltab, &S.ws[warp], &a);
-                const double gE = lane < 16 ? S.gle[pos] : 0.0;
-                double gL = 0.0, lossv = 0.0;
-                const bool scored = p == P - 1 || args.loss_mode == 1;
-                if (scored && lane < 16) {
+                const double gE = S.gle[pos];
+                double gL = 0.0;
+                if (scored) {
+                    const double lapp = __shfl_sync(SG_FULL, r.lapp, lane & 15);
                     const double s = args.code_bits[cw * SG_CUBE + pos] ? 1.0 : -1.0;
-                    const double z = s * r.lapp;
-                    lossv = z > 0.0 ? z + log1p(exp(-z)) : log1p(exp(z)); /* softplus */
-                    gL = s / (1.0 + exp(-z));                              /* s * sigmoid(z) */
+                    const double z = s * lapp, t = exp(-fabs(z));
+                    ls += (z > 0.0 ? z : 0.0) + log1p(t);            /* softplus */
+                    gL = s * (z > 0.0 ? 1.0 : t) / (1.0 + t);         /* s * sigmoid(z) */
                 }
-                const double gx = sg_line_vjp(x, gL + gE, a, etab, lane) - gE;
+                const double gx = sg_line_vjp(x, gL + gE, a, lane) - gE;
+                __syncwarp(); /* gle read by both halves */
                 if (lane < 16) {
                     S.gle[pos] = alpha * gx;
-                    if (args.grad_llr)
-                        args.grad_llr[cw * SG_CUBE + pos] += gx;
+                    if (args.grad_llr) /* one addition per phase: no result to wait for */
+                        atomicAdd(&args.grad_llr[cw * SG_CUBE + pos], gx);
                 }
-                const double ga = sg_sum16(gx * lep, lane);
-                const double ls = sg_sum16(lossv, lane);
-                if (lane == 0) {
-                    atomicAdd(&S.ga, ga);
-                    if (scored)
-                        atomicAdd(&S.lsum, ls);
-                }
+                ga += gx * lep;
+            }
+            ga = sg_sum16(ga);
+            ls = sg_sum16(ls);
+            if (lane == 0) {
+                atomicAdd(&S.ga, ga);
+                if (scored)
+                    atomicAdd(&S.lsum, ls);
             }
             __syncthreads();
             if (tid == 0)

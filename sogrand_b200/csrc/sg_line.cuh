@@ -424,13 +424,16 @@ __device__ __forceinline__ bool sg_sum_hits(double e, uint32_t ent, uint32_t hit
  * Valid for decodes that stop at a list insertion (Tmax >= 65536). */
 struct SgAdjOut {
     double etot;    /* uniform: sum of exp(-PM) over the counted guesses */
-    double esort;   /* lane r < 16: the same sum over guesses whose pattern holds sorted position r */
+    double esort;   /* lanes r and r + 16: the same sum over guesses whose pattern holds sorted position r */
     double pnl;     /* uniform: pNL of the last list insertion (before the 1e-40 clamp) */
     double my_e;    /* lane k < curl: exp(-PM) of list entry k */
     uint32_t my_cm; /* lane k < curl: bits of list entry k */
     uint32_t hdm;   /* hard decision, bit i = position i */
     int32_t curl;
-    int32_t myrank; /* lane i < 16: sorted rank of position i */
+    int32_t myrank; /* lanes i and i + 16: sorted rank of position i */
+    /* lanes i and i + 16, when curl > 0: e^{x_i}, 1/(1 + e^{x_i}), p0_i and p1_i of the soft output */
+    double ex, q1, p0, p1;
+    bool want_app; /* in: L_APP is needed (otherwise left out) */
 };
 
 /* Decode one line.  llr: the input LLR of position lane & 15 (all lanes).  enum_tabs: SG_ENUM_NTAB tables of SG_ENUM_LEN entries.
@@ -786,18 +789,21 @@ __device__ __forceinline__ SgLineResult sg_decode_line(double llr, const SgLineP
         idx += 32u;
     }
     if (ADJ) {
-        /* sums over the warp; lane r keeps sorted position r */
+        /* sums over the warp: halving exchanges, after which lanes r and
+         * r + 16 hold those of sorted position r (15 exchanges and one more
+         * instead of 16 full reductions) */
         for (int off = 16; off > 0; off >>= 1)
             adj_tot += __shfl_xor_sync(SG_FULL, adj_tot, off);
-        double mine_r = 0.0;
 #pragma unroll
-        for (int r = 0; r < (ADJ ? 16 : 1); r++) {
-            double v = adj_r[r];
-            for (int off = 16; off > 0; off >>= 1)
-                v += __shfl_xor_sync(SG_FULL, v, off);
-            if (lane == r)
-                mine_r = v;
+        for (int h = ADJ ? 8 : 0; h > 0; h >>= 1) {
+            const bool up = (lane & h) != 0;
+#pragma unroll
+            for (int r = 0; r < h; r++) {
+                const double give = up ? adj_r[r] : adj_r[r + h], keep = up ? adj_r[r + h] : adj_r[r];
+                adj_r[r] = keep + __shfl_xor_sync(SG_FULL, give, h);
+            }
         }
+        const double mine_r = adj_r[0] + __shfl_xor_sync(SG_FULL, adj_r[0], 16);
         adj->etot = adj_tot;
         adj->esort = mine_r;
         const int curl = ws->curl;
@@ -813,7 +819,7 @@ __device__ __forceinline__ SgLineResult sg_decode_line(double llr, const SgLineP
         }
         adj->hdm = hdm;
         adj->curl = curl;
-        adj->myrank = act ? ws->rank[lane] : 0;
+        adj->myrank = ws->rank[lane & 15];
     }
 
     /* Soft output (:536-577) */
@@ -823,11 +829,8 @@ __device__ __forceinline__ SgLineResult sg_decode_line(double llr, const SgLineP
     res.ncw = curl;
     /* the input LLR of position lane & 15, kept in qa during the loop */
     const double x = ws->qa[lane & 15];
-    double lapp, le;
-    if (curl == 0) {
-        lapp = x;
-        le = 0.0;
-    } else {
+    double lapp = x, le = 0.0;
+    if (curl != 0) {
         /* every lane works on position lane & 15; lanes 0..15 then take
          * log(p0), lanes 16..31 log(p1) */
         const int pos = lane & 15;
@@ -850,9 +853,17 @@ __device__ __forceinline__ SgLineResult sg_decode_line(double llr, const SgLineP
         }
         p0 = __dadd_rn(p0, __dmul_rn(pnlc, pp0));
         p1 = __dadd_rn(p1, __dmul_rn(pnlc, pp1));
-        const double lg = sg_dec_log_pos<CR>(fmax(act ? p0 : p1, 1e-40), ltab);
-        lapp = __dsub_rn(lg, __shfl_down_sync(SG_FULL, lg, 16));
-        le = __dsub_rn(lapp, x);
+        if (ADJ) {
+            adj->ex = ws->ex[pos];
+            adj->q1 = q1;
+            adj->p0 = p0;
+            adj->p1 = p1;
+        }
+        if (!ADJ || adj->want_app) {
+            const double lg = sg_dec_log_pos<CR>(fmax(act ? p0 : p1, 1e-40), ltab);
+            lapp = __dsub_rn(lg, __shfl_down_sync(SG_FULL, lg, 16));
+            le = __dsub_rn(lapp, x);
+        }
     }
     res.lapp = lapp;
     res.le = le;
