@@ -98,26 +98,87 @@ struct SgBackwardArgs {
     sg_order_meta meta;
 };
 
-template <int NW>
+#define SG_BACK_WINDOW 2048   /* codewords of a launch that are ordered by length */
+#define SG_BACK_WARPS 24      /* of the backward kernel's CTAs, one per SM */
+
 struct SgBackSmem {
-    double gle[SG_CUBE]; /* d loss / d L_E of the phase being processed */
+    union {
+        double gle[SG_CUBE]; /* d loss / d L_E of the phase being processed */
+        struct { /* before it: the choice of the codeword */
+            uint8_t pick[SG_BACK_WINDOW];
+            int hist[SG_MAX_PHASES + 1];
+        };
+    };
     SgEtab<true> etab;
     alignas(16) double ltab[SG_LOG_TAB_LEN];
-    SgWarpScratch ws[NW];
+    SgWarpScratch ws[SG_BACK_WARPS];
     double ga;   /* d loss / d alpha of the phase */
     double lsum; /* loss of the codeword */
     int line_next;
 };
 
-/* MINB CTAs of NW warps per SM: 24 warps either way, the most with 80
- * registers.  The sums over the counted guesses take 34 of them; at 64
- * (32 warps) they spill.  The exp table is held in eight copies as in the
- * decoders: 1 024 codewords at 1.5 dB, Imax 10, 44.9 -> 42.3 ms. */
-template <int NW, int MINB>
-__global__ void __launch_bounds__(NW * 32, MINB) sg_backward_kernel(const __grid_constant__ SgBackwardArgs args)
+/* The codeword of block b: the last SG_BACK_WINDOW ones are taken in the
+ * order of falling phase counts, equal ones in index order.  Codewords differ
+ * in length by up to the number of phases, and a long one that starts last
+ * runs alone on its SM.  A block counts the window's phases for itself (a few
+ * microseconds of the millisecond a codeword takes), so nothing is shared
+ * between blocks.  1.5 dB, Imax 10: 1 024 codewords 32.8 -> 28.0 ms, 600 22.4
+ * -> 18.1. */
+__device__ __forceinline__ unsigned long long sg_back_pick(const SgBackwardArgs& args, unsigned long long b, uint8_t* ph,
+                                                           int* hist, int tid)
 {
-    constexpr int NT = NW * 32;
-    SgBackSmem<NW>& S = *reinterpret_cast<SgBackSmem<NW>*>(sg_smem_raw);
+    constexpr int NT = SG_BACK_WARPS * 32;
+    const unsigned long long n = args.n_cw, base = n > SG_BACK_WINDOW ? n - SG_BACK_WINDOW : 0;
+    if (b < base)
+        return b;
+    const int m = (int)(n - base);
+    int k = (int)(b - base); /* the k-th of m */
+    for (int i = tid; i <= SG_MAX_PHASES; i += NT)
+        hist[i] = 0;
+    __syncthreads();
+    for (int i = tid; i < m; i += NT) {
+        const int p = min(max(args.stats[base + i].phases, 0), SG_MAX_PHASES);
+        ph[i] = (uint8_t)p;
+        atomicAdd(&hist[p], 1);
+    }
+    __syncthreads();
+    if (tid < 32) {
+        int v = SG_MAX_PHASES;
+        for (; k >= hist[v]; v--)
+            k -= hist[v];
+        int i = tid;
+        for (;; i += 32) {
+            const uint32_t same = __ballot_sync(SG_FULL, i < m && ph[i] == v);
+            const int c = __popc(same);
+            if (k < c) {
+                if (i < m && ph[i] == v && __popc(same & ((1u << tid) - 1u)) == k)
+                    hist[0] = i;
+                break;
+            }
+            k -= c;
+        }
+    }
+    __syncthreads();
+    const int i = hist[0];
+    __syncthreads();
+    return base + (unsigned long long)i;
+}
+
+/* One codeword at a time on an SM's 24 warps, the most with 80 registers.
+ * The sums over the counted guesses take 34 of them: with 28 and 32 warps
+ * they spill (1 024 codewords at 1.5 dB, Imax 10: 26.8 ms, 28 warps 27.5, 32
+ * 28.7).  Two CTAs of 12 warps, each with a codeword of its own, hide the end
+ * of each other's phases but take twice as long over the longest codeword:
+ * 28.0 ms, and for 160 codewords 11.5 against 7.2.
+ * Bound by issue slots and, at 24 warps, latency: a guess costs its 17
+ * predicated additions besides the forward's work.  Per line, whatever the
+ * decode has worked out is used again, sums over a phase are kept per lane,
+ * and no logarithm is taken where the loss does not need L_APP (42.3 -> 32.8
+ * ms); the exp table in eight copies, as in the decoders (44.9 -> 42.3). */
+__global__ void __launch_bounds__(SG_BACK_WARPS * 32, 1) sg_backward_kernel(const __grid_constant__ SgBackwardArgs args)
+{
+    constexpr int NT = SG_BACK_WARPS * 32;
+    SgBackSmem& S = *reinterpret_cast<SgBackSmem*>(sg_smem_raw);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     sg_etab_fill<false, true>(S.etab, g_etab, tid, NT);
     for (int i = tid; i < SG_LOG_TAB_LEN; i += NT)
@@ -128,7 +189,8 @@ __global__ void __launch_bounds__(NW * 32, MINB) sg_backward_kernel(const __grid
     lp.thres = args.thres;
     const SgTab etab = sg_etab_of<false, true>(S.etab, args.k.v), ltab{S.ltab, args.k.v};
     __syncthreads();
-    for (unsigned long long cw = blockIdx.x; cw < args.n_cw; cw += gridDim.x) {
+    for (unsigned long long b = blockIdx.x; b < args.n_cw; b += gridDim.x) {
+        const unsigned long long cw = sg_back_pick(args, b, S.pick, S.hist, tid);
         const int P = args.stats[cw].phases;
         const double* g = args.llr + cw * SG_CUBE;
         for (int i = tid; i < SG_CUBE; i += NT) {

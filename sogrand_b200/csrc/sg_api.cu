@@ -501,10 +501,8 @@ sg_status get_ctx(DevCtx** out)
                 SG_CUDA(cudaFuncSetAttribute(bitso_fn(v, cr), cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              (int)k_bvariants[v].smem));
         SG_CUDA(cudaFuncSetAttribute(sg_gen_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SgGenSmem)));
-        SG_CUDA(cudaFuncSetAttribute(sg_backward_kernel<12, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)sizeof(SgBackSmem<12>)));
-        SG_CUDA(cudaFuncSetAttribute(sg_backward_kernel<24, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)sizeof(SgBackSmem<24>)));
+        SG_CUDA(cudaFuncSetAttribute(sg_backward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)sizeof(SgBackSmem)));
         SG_CUDA(cudaDeviceGetAttribute(&c.sms, cudaDevAttrMultiProcessorCount, dev));
         c.ready = true;
     }
@@ -1664,12 +1662,8 @@ sg_status sg_backward_device(const double* d_llr, size_t n_cw, const sg_params* 
     memcpy(a.alpha, p->alpha, sizeof a.alpha);
     a.k = k_consts;
     void* kargs[] = {(void*)&a};
-    /* one codeword per CTA: all of an SM's warps on it when there are no more
-     * codewords than SMs */
-    const bool few = n_cw <= (size_t)c->sms;
-    SG_CUDA(cudaLaunchKernel(few ? (const void*)sg_backward_kernel<24, 1> : (const void*)sg_backward_kernel<12, 2>,
-                             dim3(grid_for(n_cw, 1 << 30)), dim3(few ? 768 : 384), kargs,
-                             few ? sizeof(SgBackSmem<24>) : sizeof(SgBackSmem<12>), (cudaStream_t)stream));
+    SG_CUDA(cudaLaunchKernel((const void*)sg_backward_kernel, dim3(grid_for(n_cw, 1 << 30)),
+                             dim3(SG_BACK_WARPS * 32), kargs, sizeof(SgBackSmem), (cudaStream_t)stream));
     return SG_OK;
 }
 

@@ -1,7 +1,7 @@
 """Dispatch lines of the line and backward kernels: results must not depend on how many lines or
 codewords a call holds.  Lines: up to 256 on host buffers, one warp per line, one line per CTA below
-two CTAs per SM, a persistent grid above the resident warps (4 736 on 148 SMs).  Backward: one CTA
-of 24 warps per SM up to one codeword per SM, two of 12 beyond."""
+two CTAs per SM, a persistent grid above the resident warps (4 736 on 148 SMs).  Backward: a call's
+last 2 048 codewords are taken in the order of falling phase counts."""
 import ctypes as C
 
 import numpy as np
@@ -56,25 +56,24 @@ def test_line_routes(cuda, sg, mode):
             same(sg.bitso(v[:n], L=L, Tmax=tmax), [w[:n] for w in want])
 
 
-@pytest.mark.parametrize("loss_mode", [0, 1])
-def test_backward_routes(cuda, sg, loss_mode):
-    """A codeword's loss and gradients in a call beyond one codeword per SM (two CTAs of 12 warps)
-    against calls of few codewords (one of 24).  The warps of a CTA add into a codeword's sums in an
-    order of their own, so the bound is that of the adjoint's own tests, 1e-9 of the largest entry;
+@pytest.mark.parametrize("n,chunk,loss_mode", [(150, 50, 0), (150, 50, 1), (2047, 90, 1), (2048, 700, 0),
+                                               (2049, 700, 0), (2200, 700, 0)])
+def test_backward_order(cuda, sg, n, chunk, loss_mode):
+    """A codeword's loss and gradients in one call against smaller calls.  The warps of a CTA add
+    into a codeword's sums in an order of their own, so the bound is that of the adjoint's own tests, 1e-9 of the largest entry;
     the losses are sums of 4 096 positive terms in another grouping: 1e-12."""
     torch = cuda
     from sogrand_b200 import diff
 
-    n = torch.cuda.get_device_properties(0).multi_processor_count + 1
-    info, llr = sg.gen_llr(31, 0, n, ebn0_db=2.0, device="cuda")
+    info, llr = sg.gen_llr(31, 0, n, ebn0_range=(1.5, 3.0), device="cuda")
     llr[3, 9] = float("nan")
     cb = diff.code_bits_for(info, "cuda")
     p = sg.params(Imax=3)
     _, st, _, ck = diff.forward_raw(llr, p)
     whole = diff.backward_raw(llr, cb, p, st, ck, want_llr=True, loss_mode=loss_mode)
-    part = [torch.cat(t) for t in zip(*(diff.backward_raw(llr[a : a + 50], cb[a : a + 50], p, st[a : a + 50],
-                                                          ck[a : a + 50], want_llr=True, loss_mode=loss_mode)
-                                        for a in range(0, n, 50)))]
+    part = [torch.cat(t) for t in zip(*(diff.backward_raw(llr[a : a + chunk], cb[a : a + chunk], p, st[a : a + chunk],
+                                                          ck[a : a + chunk], want_llr=True, loss_mode=loss_mode)
+                                        for a in range(0, n, chunk)))]
     for w, q, tol in zip(whole, part, (1e-12, 1e-9, 1e-9)):
         w, q = w.cpu().numpy(), q.cpu().numpy()
         assert np.array_equal(np.isnan(w), np.isnan(q))
