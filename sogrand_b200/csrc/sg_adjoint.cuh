@@ -38,7 +38,7 @@ __device__ __forceinline__ double sg_sum16(double v)
 /* Gradient with respect to the line input x of g . L_APP, g the upstream
  * gradient of L_APP; lanes p and p + 16 hold position p alike.  The soft
  * output's exp, reciprocal and sums come from the decode. */
-__device__ __forceinline__ double sg_line_vjp(double x, double g, const SgAdjOut& a, int lane)
+__device__ __forceinline__ double sg_line_vjp(double x, double g, const SgAdjOut& a, SgTab etab, int lane)
 {
     if (a.curl == 0)
         return g; /* L_APP = x */
@@ -60,8 +60,8 @@ __device__ __forceinline__ double sg_line_vjp(double x, double g, const SgAdjOut
     if (pp1r > eps)
         gx -= a1 * p_nl * dsig;
     const double sgn = x > 0.0 ? 1.0 : (x < 0.0 ? -1.0 : 0.0);
-    /* sigma(-|x|): 1/(1 + e^x) for x > 0, e^x/(1 + e^x) otherwise */
-    const double sm = fabs(x) <= 50.0 ? (x > 0.0 ? pp1r : a.ex * pp1r) : 0.0;
+    const double ax = fabs(x);
+    const double sm = ax <= 50.0 ? (x > 0.0 ? pp1r : 1.0 / (1.0 + sg_exp(ax, etab))) : 0.0; /* sigma(-|x|) */
     for (int j = 0; j < a.curl; j++) {
         const double pj = __shfl_sync(SG_FULL, a.my_e, j);
         const uint32_t cm = __shfl_sync(SG_FULL, a.my_cm, j);
@@ -73,7 +73,7 @@ __device__ __forceinline__ double sg_line_vjp(double x, double g, const SgAdjOut
     }
     if (pnl_live) {
         const double gpnl = sg_sum16(a0 * pp0 + a1 * pp1);
-        const double ei = __shfl_sync(SG_FULL, a.esort, a.myrank);
+        const double ei = __shfl_sync(SG_FULL, a.esort, 2 * a.myrank);
         gx += gpnl * 0x1p-8 * sgn * (ei - sm * a.etot);
     }
     return gx;
@@ -122,8 +122,8 @@ struct SgBackSmem {
  * in length by up to the number of phases, and a long one that starts last
  * runs alone on its SM.  A block counts the window's phases for itself (a few
  * microseconds of the millisecond a codeword takes), so nothing is shared
- * between blocks.  1.5 dB, Imax 10: 1 024 codewords 32.8 -> 28.0 ms, 600 22.4
- * -> 18.1. */
+ * between blocks.  1.5 dB, Imax 10: 1 024 codewords 32.8 -> 26.8 ms, 600 22.4
+ * -> 17.4. */
 __device__ __forceinline__ unsigned long long sg_back_pick(const SgBackwardArgs& args, unsigned long long b, uint8_t* ph,
                                                            int* hist, int tid)
 {
@@ -166,14 +166,14 @@ __device__ __forceinline__ unsigned long long sg_back_pick(const SgBackwardArgs&
 
 /* One codeword at a time on an SM's 24 warps, the most with 80 registers.
  * The sums over the counted guesses take 34 of them: with 28 and 32 warps
- * they spill (1 024 codewords at 1.5 dB, Imax 10: 26.8 ms, 28 warps 27.5, 32
- * 28.7).  Two CTAs of 12 warps, each with a codeword of its own, hide the end
- * of each other's phases but take twice as long over the longest codeword:
- * 28.0 ms, and for 160 codewords 11.5 against 7.2.
+ * they spill (1 024 codewords at 1.5 dB, Imax 10: 27.5 ms, 28 warps 2.5 %
+ * more, 32 7 %).  Two CTAs of 12 warps, each with a codeword of its own, hide the end
+ * of each other's phases but take twice as long over the longest codeword: 4 %
+ * more, and 11.5 against 7.3 ms for 160 codewords.
  * Bound by issue slots and, at 24 warps, latency: a guess costs its 17
  * predicated additions besides the forward's work.  Per line, whatever the
  * decode has worked out is used again, sums over a phase are kept per lane,
- * and no logarithm is taken where the loss does not need L_APP (42.3 -> 32.8
+ * and no logarithm is taken where the loss does not need L_APP (42.3 -> 33
  * ms); the exp table in eight copies, as in the decoders (44.9 -> 42.3). */
 __global__ void __launch_bounds__(SG_BACK_WARPS * 32, 1) sg_backward_kernel(const __grid_constant__ SgBackwardArgs args)
 {
@@ -232,11 +232,11 @@ __global__ void __launch_bounds__(SG_BACK_WARPS * 32, 1) sg_backward_kernel(cons
                 if (scored) {
                     const double lapp = __shfl_sync(SG_FULL, r.lapp, lane & 15);
                     const double s = args.code_bits[cw * SG_CUBE + pos] ? 1.0 : -1.0;
-                    const double z = s * lapp, t = exp(-fabs(z));
-                    ls += (z > 0.0 ? z : 0.0) + log1p(t);            /* softplus */
-                    gL = s * (z > 0.0 ? 1.0 : t) / (1.0 + t);         /* s * sigmoid(z) */
+                    const double z = s * lapp;
+                    ls += (z > 0.0 ? z : 0.0) + log1p(exp(-fabs(z))); /* softplus */
+                    gL = s / (1.0 + exp(-z));                          /* s * sigmoid(z) */
                 }
-                const double gx = sg_line_vjp(x, gL + gE, a, lane) - gE;
+                const double gx = sg_line_vjp(x, gL + gE, a, etab, lane) - gE;
                 __syncwarp(); /* gle read by both halves */
                 if (lane < 16) {
                     S.gle[pos] = alpha * gx;

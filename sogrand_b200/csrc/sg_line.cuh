@@ -424,15 +424,15 @@ __device__ __forceinline__ bool sg_sum_hits(double e, uint32_t ent, uint32_t hit
  * Valid for decodes that stop at a list insertion (Tmax >= 65536). */
 struct SgAdjOut {
     double etot;    /* uniform: sum of exp(-PM) over the counted guesses */
-    double esort;   /* lanes r and r + 16: the same sum over guesses whose pattern holds sorted position r */
+    double esort;   /* lanes 2 r and 2 r + 1: the same sum over guesses whose pattern holds sorted position r */
     double pnl;     /* uniform: pNL of the last list insertion (before the 1e-40 clamp) */
     double my_e;    /* lane k < curl: exp(-PM) of list entry k */
     uint32_t my_cm; /* lane k < curl: bits of list entry k */
     uint32_t hdm;   /* hard decision, bit i = position i */
     int32_t curl;
     int32_t myrank; /* lanes i and i + 16: sorted rank of position i */
-    /* lanes i and i + 16, when curl > 0: e^{x_i}, 1/(1 + e^{x_i}), p0_i and p1_i of the soft output */
-    double ex, q1, p0, p1;
+    /* lanes i and i + 16, when curl > 0: 1/(1 + e^{x_i}), p0_i and p1_i of the soft output */
+    double q1, p0, p1;
     bool want_app; /* in: L_APP is needed (otherwise left out) */
 };
 
@@ -789,21 +789,21 @@ __device__ __forceinline__ SgLineResult sg_decode_line(double llr, const SgLineP
         idx += 32u;
     }
     if (ADJ) {
-        /* sums over the warp: halving exchanges, after which lanes r and
-         * r + 16 hold those of sorted position r (15 exchanges and one more
-         * instead of 16 full reductions) */
+        /* sums over the warp: halving exchanges, which leave lanes 2 r and
+         * 2 r + 1 with sorted position r's (15 exchanges and an addition
+         * instead of 16 full reductions, in the same order) */
         for (int off = 16; off > 0; off >>= 1)
             adj_tot += __shfl_xor_sync(SG_FULL, adj_tot, off);
 #pragma unroll
         for (int h = ADJ ? 8 : 0; h > 0; h >>= 1) {
-            const bool up = (lane & h) != 0;
+            const bool up = (lane & (2 * h)) != 0;
 #pragma unroll
             for (int r = 0; r < h; r++) {
                 const double give = up ? adj_r[r] : adj_r[r + h], keep = up ? adj_r[r + h] : adj_r[r];
-                adj_r[r] = keep + __shfl_xor_sync(SG_FULL, give, h);
+                adj_r[r] = keep + __shfl_xor_sync(SG_FULL, give, 2 * h);
             }
         }
-        const double mine_r = adj_r[0] + __shfl_xor_sync(SG_FULL, adj_r[0], 16);
+        const double mine_r = adj_r[0] + __shfl_xor_sync(SG_FULL, adj_r[0], 1);
         adj->etot = adj_tot;
         adj->esort = mine_r;
         const int curl = ws->curl;
@@ -854,7 +854,6 @@ __device__ __forceinline__ SgLineResult sg_decode_line(double llr, const SgLineP
         p0 = __dadd_rn(p0, __dmul_rn(pnlc, pp0));
         p1 = __dadd_rn(p1, __dmul_rn(pnlc, pp1));
         if (ADJ) {
-            adj->ex = ws->ex[pos];
             adj->q1 = q1;
             adj->p0 = p0;
             adj->p1 = p1;
