@@ -112,6 +112,7 @@ struct SgBackSmem {
     SgEtab<true> etab;
     alignas(16) double ltab[SG_LOG_TAB_LEN];
     SgWarpScratch ws[SG_BACK_WARPS];
+    double bins[SG_BACK_WARPS][9 * 32]; /* high positions' guess sums, per lane */
     double ga;   /* d loss / d alpha of the phase */
     double lsum; /* loss of the codeword */
     int line_next;
@@ -164,17 +165,19 @@ __device__ __forceinline__ unsigned long long sg_back_pick(const SgBackwardArgs&
     return base + (unsigned long long)i;
 }
 
-/* One codeword at a time on an SM's 24 warps, the most with 80 registers.
- * The sums over the counted guesses take 34 of them: with 28 and 32 warps
- * they spill (1 024 codewords at 1.5 dB, Imax 10: 27.5 ms, 28 warps 2.5 %
- * more, 32 7 %).  Two CTAs of 12 warps, each with a codeword of its own, hide the end
- * of each other's phases but take twice as long over the longest codeword: 4 %
- * more, and 11.5 against 7.3 ms for 160 codewords.
- * Bound by issue slots and, at 24 warps, latency: a guess costs its 17
- * predicated additions besides the forward's work.  Per line, whatever the
- * decode has worked out is used again, sums over a phase are kept per lane,
- * and no logarithm is taken where the loss does not need L_APP (42.3 -> 33
- * ms); the exp table in eight copies, as in the decoders (44.9 -> 42.3). */
+/* One codeword at a time on an SM's 24 warps of 80 registers; 28 warps take
+ * as long, 30 spill and take 2 % more.  Two CTAs of 12 warps, each with a
+ * codeword of its own, hide the end of each other's phases but take twice as
+ * long over the longest codeword: 4 % more for 1 024 codewords at 1.5 dB, Imax
+ * 10, and 11.5 against 7.3 ms for 160.
+ * Bound by issue slots (71 % used) and latency.  A guess costs nine predicated
+ * additions and two shared-memory sums besides the forward's work: with all 16
+ * positions' sums in registers 27.5 ms and spills, with the high ones' in
+ * shared memory, of which the forward's work leaves half idle, 25.7 ms.  Per
+ * line, whatever the decode has worked out is used again, sums over a phase
+ * are kept per lane, and no logarithm is taken where the loss does not need
+ * L_APP (42.3 -> 33 ms); the exp table in eight copies, as in the decoders
+ * (44.9 -> 42.3). */
 __global__ void __launch_bounds__(SG_BACK_WARPS * 32, 1) sg_backward_kernel(const __grid_constant__ SgBackwardArgs args)
 {
     constexpr int NT = SG_BACK_WARPS * 32;
@@ -226,6 +229,7 @@ __global__ void __launch_bounds__(SG_BACK_WARPS * 32, 1) sg_backward_kernel(cons
                 const double x = __dadd_rn(g[pos], __dmul_rn(alpha, lep));
                 SgAdjOut a;
                 a.want_app = scored;
+                a.bins = S.bins[warp];
                 const SgLineResult r = sg_decode_line<true, false, true>(x, lp, args.enum_tabs, etab, ltab, &S.ws[warp], &a);
                 const double gE = S.gle[pos];
                 double gL = 0.0;

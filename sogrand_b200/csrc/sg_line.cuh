@@ -434,6 +434,7 @@ struct SgAdjOut {
     /* lanes i and i + 16, when curl > 0: 1/(1 + e^{x_i}), p0_i and p1_i of the soft output */
     double q1, p0, p1;
     bool want_app; /* in: L_APP is needed (otherwise left out) */
+    double* bins;  /* in: shared, [9][32]; a lane's sums over guesses holding high position j in row 1 + j */
 };
 
 /* Decode one line.  llr: the input LLR of position lane & 15 (all lanes).  enum_tabs: SG_ENUM_NTAB tables of SG_ENUM_LEN entries.
@@ -633,15 +634,33 @@ __device__ __forceinline__ SgLineResult sg_decode_line(double llr, const SgLineP
     uint32_t T = 0;
     double adj_tot = 0.0, adj_r[ADJ ? 16 : 1];
 #pragma unroll
-    for (int r = 0; r < (ADJ ? 16 : 1); r++)
+    for (int r = 0; r < (ADJ ? 8 : 1); r++)
         adj_r[r] = 0.0;
-    auto adj_add = [&](double e, uint32_t ent) { /* a guess that entered P_notGuess */
-        adj_tot += e;
-        const uint32_t m = sg_ent_pattern(ent);
+    if (ADJ)
 #pragma unroll
-        for (int r = 0; r < (ADJ ? 16 : 1); r++)
+        for (int r = 1; r < 9; r++)
+            adj->bins[32 * r + lane] = 0.0;
+    /* A guess that entered P_notGuess.  The sums of the low positions stay in
+     * registers, a pattern holding any of them; of the high ones it holds at
+     * most two but for special steps, so theirs are in shared memory, picked
+     * by the entry's offsets (row 0: none). */
+    auto adj_add = [&](double e, uint32_t ent, bool general) {
+        adj_tot += e;
+        const uint32_t m = sg_swz(ent & 0xffu);
+#pragma unroll
+        for (int r = 0; r < (ADJ ? 8 : 1); r++)
             if ((m >> r) & 1u)
                 adj_r[r] += e;
+        double* bin = adj->bins + lane;
+        bin[((ent >> 16) & 0xffu) * 4u] += e;
+        bin[(ent >> 24) * 4u] += e;
+        if (general) {
+            uint32_t rest = (ent >> 8) & 0xffu;
+            rest &= rest - 1u;
+            rest &= rest - 1u;
+            for (; rest; rest &= rest - 1u)
+                bin[32 * __ffs(rest)] += e;
+        }
     };
     /* path metric (up to two high positions) and syndrome of an entry: the
      * high positions in ascending order, from the entry's offsets (offset 0
@@ -702,7 +721,7 @@ __device__ __forceinline__ SgLineResult sg_decode_line(double llr, const SgLineP
                     break;
                 }
                 if (ADJ)
-                    adj_add(ea_, enta);
+                    adj_add(ea_, enta, false);
                 idx += 32u;
                 Pb = pb;
                 if ((int32_t)(pb >> 32) <= __double2hiint(g.b1)) {
@@ -717,7 +736,7 @@ __device__ __forceinline__ SgLineResult sg_decode_line(double llr, const SgLineP
                     break;
                 }
                 if (ADJ)
-                    adj_add(eb_, entb);
+                    adj_add(eb_, entb, false);
                 idx += 32u;
             }
         }
@@ -735,7 +754,7 @@ __device__ __forceinline__ SgLineResult sg_decode_line(double llr, const SgLineP
                 break;
             }
             if (ADJ)
-                adj_add(e, ent);
+                adj_add(e, ent, false);
             idx += 32u;
         }
         if (!out) {
@@ -760,7 +779,7 @@ __device__ __forceinline__ SgLineResult sg_decode_line(double llr, const SgLineP
             Pb -= tot;
             if ((int32_t)(Pb >> 32) > __double2hiint(g.b1)) {
                 if (ADJ)
-                    adj_add(e, ent);
+                    adj_add(e, ent, true);
                 idx += 32u;
                 continue;
             }
@@ -783,7 +802,7 @@ __device__ __forceinline__ SgLineResult sg_decode_line(double llr, const SgLineP
             g = sg_grid(Pb);
         }
         if (ADJ && (!done || (idx & (SG_ENUM_LEN - 1u)) < T))
-            adj_add(e, ent);
+            adj_add(e, ent, true);
         if (done)
             break;
         idx += 32u;
@@ -794,6 +813,9 @@ __device__ __forceinline__ SgLineResult sg_decode_line(double llr, const SgLineP
          * instead of 16 full reductions, in the same order) */
         for (int off = 16; off > 0; off >>= 1)
             adj_tot += __shfl_xor_sync(SG_FULL, adj_tot, off);
+#pragma unroll
+        for (int r = 8; r < (ADJ ? 16 : 8); r++)
+            adj_r[r] = adj->bins[32 * (r - 7) + lane];
 #pragma unroll
         for (int h = ADJ ? 8 : 0; h > 0; h >>= 1) {
             const bool up = (lane & (2 * h)) != 0;
