@@ -338,9 +338,10 @@ std::mutex g_mu;
 std::atomic<long long> g_wait_limit{SG_WAIT_LIMIT_DEFAULT};
 std::atomic<int> g_math_mode{0}; /* 0: table-driven exp/log, 1: correctly rounded */
 /* Selected kernel variants, one per math mode (sogrand_b200.autotune
- * measures them).  B200, 12 000 codewords at 2 dB, table math: p32x3 122.0
- * ms, p28x3 124.2, p24x3 127.1; w16-gmem 124.8, w8-gmem 139.1, w12-smem
- * 140.7, w8-smem 169.1. */
+ * measures them).  B200, 12 000 codewords at 2 dB, table math: p32x3 112.6
+ * ms, p28x3 117.3, p24x3 121.6; w16-gmem 115.3, w8-gmem 134.0, w12-smem
+ * 137.0, w8-smem 162.7; correctly rounded, 6 000: p32x3 86.5, p28x3 89.2,
+ * p24x3 93.2; w16-gmem 87.7, w8-gmem 93.5. */
 int g_pvariant_by_mode[2] = {SG_PVARIANT_AUTO, SG_PVARIANT_AUTO};
 int g_variant_by_mode[2] = {SG_VARIANT_AUTO, SG_VARIANT_AUTO};
 #define g_pvariant (g_pvariant_by_mode[g_math_mode.load()])
@@ -429,7 +430,7 @@ cudaError_t cluster_setup(int dev, ClusterInfo* info)
 /* The cluster configuration for a batch of n codewords, -1 when it is large
  * enough for one CTA per codeword: the most CTAs per codeword with which all
  * clusters run at the same time; with two, also up to 7/4 codewords per SM.
- * B200, one call at 2 dB: n = 1 plain 2.29 ms, 16 CTAs 0.43, 8 CTAs 0.52;
+ * B200, one call at 2 dB, when the rule was set: n = 1 plain 2.29 ms, 16 CTAs 0.43, 8 CTAs 0.52;
  * n = 9: 8 CTAs 0.58, 16 (the ninth cluster waits) 0.66; n = 18: 4 CTAs 1.02,
  * 8 1.18; n = 33: 4 CTAs 1.02, 2 1.57; n = 37 (one too many): 4 CTAs 1.66, 2
  * 1.74; n = 100: 2 CTAs 2.00, plain 3.81; n = 220: 3.92, 4.46; n = 296: 4.35,
@@ -646,7 +647,9 @@ sg_status sg_bitso_device(const double* d_llr, size_t n_lines, int32_t L, uint64
     sg_order_meta meta;
     order_meta(tmax_eff(Tmax), &meta);
     /* few lines: one per warp, spread over the SMs; more than the warps two
-     * CTAs of 16 keep resident: those, each with an equal share */
+     * CTAs of 16 keep resident: those, each with an equal share.  Beyond that
+     * line the resident grid fills its tables once: 65 537 lines at 2 dB 294 us,
+     * one per warp in CTAs of their own 342. */
     const unsigned long long full = 2ull * c->sms;
     const int bv = n_lines > 16 * full ? 1 : 0;
     const SgBVariant& v = k_bvariants[bv];
@@ -664,7 +667,7 @@ namespace {
 /* Pinned staging of a thread's small line calls, mapped into the devices'
  * address spaces; freed when the thread ends. */
 struct LineStage {
-    static constexpr size_t MAX = 256; /* lines: 100 KB */
+    static constexpr size_t MAX = 256; /* lines: 100 KB per thread */
     unsigned char* p = nullptr;
     ~LineStage()
     {
@@ -675,8 +678,9 @@ struct LineStage {
 
 /* sg_bitso_host for few lines: the kernel reads the LLRs from pinned host
  * memory and writes its results there, so a call is one launch and one wait,
- * on the thread's own stream.  16 lines: 108 us with five allocations, six
- * copies and five frees per call.  *done = false: not possible here (no
+ * on the thread's own stream.  16 lines: 41 us, with five allocations, six
+ * copies and five frees per call 116; 256 lines: 60 us, 158.  The line at 256
+ * bounds what a thread keeps pinned.  *done = false: not possible here (no
  * pinned memory), nothing happened. */
 sg_status bitso_host_small(const double* llr, size_t n, int32_t L, uint64_t Tmax, double thres, double* lapp, double* le,
                            int32_t* nguess, int32_t* ncw, bool* done)

@@ -16,6 +16,10 @@
  * Words and maxima of a phase alternate between two buffers, since a CTA may
  * be one phase ahead.  Per codeword, the line decodes and their order of
  * phases are those of sg_decode_kernel, and so are the outputs, bit for bit.
+ *
+ * Bound by the latency of a line decode and of the phase ends (issue slots
+ * 64 % used with 70 codewords on pairs).  2 dB: one codeword 2.33 -> 0.39 ms
+ * (16 CTAs), 100 codewords 3.38 -> 1.95 ms (2 CTAs each).
  */
 #pragma once
 

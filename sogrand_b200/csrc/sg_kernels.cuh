@@ -1,8 +1,8 @@
 /* sg_kernels.cuh -- the decoder kernels, instantiated by sg_api.cu with the
- * table-driven exp/log and by sg_cr.cu with the correctly rounded ones.  The
- * two are separate translation units because the compiler's register
- * allocation of one set moved with the other's code (the table-driven
- * decoders by up to 13 %).
+ * table-driven exp/log and by sg_cr.cu with the correctly rounded ones: two
+ * translation units, since the correctly rounded routines take their
+ * constants as launch arguments and the table-driven ones as literals, and
+ * built side by side.
  *
  *   sg_decode_kernel   the whole iterative decode of a codeword per CTA
  *                      (SOGRAND_C/cubic_decoder_final.c:119-289): the

@@ -33,18 +33,20 @@
  *           running P_notGuess at each, so T and the list match exactly.
  *  output   soft output of :536-577 on lanes 0..15.
  *
- * What bounds it: issue slots and shared-memory cycles, about evenly (of
+ * What bounds it: issue slots (81 % used) and shared-memory cycles (75 %), of
  * 23 steps per line decode at 2 dB, 15 end in the sum, 2 hold codewords, 6
- * are replayed).  Per line decode at 2 dB, B200 counters: 4 720 warp
- * instructions and 1 010 shared-memory cycles with the former loop of two
+ * are replayed.  Per line decode at 2 dB, B200 counters: 4 740 warp
+ * instructions and 1 280 shared-memory cycles with the former loop of two
  * patterns per lane (steps of 64, of which half had to be replayed, term
- * rounding tested by difference, an exp from one table copy); 3 300 and 780
- * with this one.  20 000 codewords at 2 dB, batched form: 245.8 -> 202.1 ms;
- * 8 000, plain form: 101.2 -> 84.0 ms; 2 000 at 1 dB under Tmax 1000: 146.5
- * -> 97.5 ms; correctly rounded math, 4 000 at 2 dB: 68.3 -> 60.0 ms.
- * Steps of 64 patterns were slower once the sum was cheap (229 ms): a step
- * twice as long is summed half as often, and has to be looked at again by
- * halves.
+ * rounding tested by difference, an exp from one table copy); 3 510 and 810
+ * now.  20 000 codewords at 2 dB, batched form: 245.8 ms, 202.1 with this
+ * loop, 193.0 with the shorter set-up and soft output, 186.2 with the exp
+ * constants in constant memory; 8 000, plain form: 101.2 -> 78.1 ms; 2 000 at
+ * 1 dB under Tmax 1000: 146 -> 91 ms; correctly rounded math, 4 000 at 2 dB:
+ * 68.3 -> 58.4 ms.
+ * Steps of 64 patterns were slower once the sum was cheap (229 against 202
+ * ms): a step twice as long is summed half as often, and has to be looked at
+ * again by halves.
  * The file is built with -fmad=false: every floating-point operation the
  * reference performs is a separately rounded IEEE operation here.
  */
