@@ -430,11 +430,11 @@ cudaError_t cluster_setup(int dev, ClusterInfo* info)
 /* The cluster configuration for a batch of n codewords, -1 when it is large
  * enough for one CTA per codeword: the most CTAs per codeword with which all
  * clusters run at the same time; with two, also up to 7/4 codewords per SM.
- * B200, one call at 2 dB, when the rule was set: n = 1 plain 2.29 ms, 16 CTAs 0.43, 8 CTAs 0.52;
- * n = 9: 8 CTAs 0.58, 16 (the ninth cluster waits) 0.66; n = 18: 4 CTAs 1.02,
- * 8 1.18; n = 33: 4 CTAs 1.02, 2 1.57; n = 37 (one too many): 4 CTAs 1.66, 2
- * 1.74; n = 100: 2 CTAs 2.00, plain 3.81; n = 220: 3.92, 4.46; n = 296: 4.35,
- * 4.63 but 4.51 in the batched form; n = 600: 8.7, 8.5. */
+ * B200, one call at 2 dB, when the rule was set: n = 1 plain 2.29 ms, 16 CTAs
+ * 0.43, 8 CTAs 0.52; n = 9: 8 CTAs 0.58, 16 (the ninth cluster waits) 0.66;
+ * n = 18: 4 CTAs 1.02, 8 1.18; n = 33: 4 CTAs 1.02, 2 1.57; n = 37 (one too
+ * many): 4 CTAs 1.66, 2 1.74; n = 100: 2 CTAs 2.00, plain 3.81; n = 220: 3.92,
+ * 4.46; n = 296: 4.35, 4.63 but 4.51 in the batched form; n = 600: 8.7, 8.5. */
 int cluster_for(unsigned long long n, const ClusterInfo& info)
 {
     for (int v = 0; v < SG_NCVARIANTS; v++)
