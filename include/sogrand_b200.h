@@ -172,8 +172,8 @@ typedef struct {
 /* Decode and reduce on the device: bits (nullable: not returned) and one
  * sg_decode_summary at d_summary (device memory, overwritten).  d_ref_info
  * (nullable): the transmitted info bits, 64 packed bytes per codeword, for
- * the bit and block error counts.  Per-codeword statistics are held in
- * stream-ordered scratch (cudaMallocAsync) for the duration of the call. */
+ * the bit and block error counts.  The decode adds each codeword to the
+ * totals as it finishes. */
 sg_status sg_decode_summary_device(const double* d_llr, size_t n_cw, const sg_params* p,
                                    const uint8_t* d_ref_info, uint8_t* d_bits,
                                    sg_decode_summary* d_summary, void* stream);
@@ -184,17 +184,15 @@ sg_status sg_decode_summary_device(const double* d_llr, size_t n_cw, const sg_pa
  * while another component owns the device allocator (a framework's caching
  * pool, a real-time process that forbids allocation after start-up), or
  * code whose every device buffer is budgeted up front.  The regular entry
- * point takes stream-ordered scratch per call and its first call on a device
- * allocates the 15 MB error-pattern order table; this one uses only memory
- * that the library declares statically:
- *   - scratch for at most SG_NOALLOC_MAX_CW codewords (statistics and bits,
- *     1.5 MB in all), held by every GPU that loads the library until exit;
+ * point's first call on a device allocates the 15 MB error-pattern order
+ * table; this one uses only memory that the library declares statically:
+ *   - the call's error flag;
  *   - its own copy of the pattern-order table (15 MB, also static), built on
  *     the device by a kernel during the first call on each device.
  * That first call also resolves the device addresses of these arrays and
  * sets up the device; make it before any stream capture.  n_cw above
  * SG_NOALLOC_MAX_CW is rejected with SG_ERR_ARG.  All calls share the one
- * scratch array: calls that overlap on the GPU (other streams, other host
+ * error flag: calls that overlap on the GPU (other streams, other host
  * threads) race and must be serialised by the caller.  Results equal those
  * of sg_decode_summary_device.  This entry point has no counterpart in the
  * reference, which is a single-process file pipeline. */

@@ -143,25 +143,28 @@ __global__ void __launch_bounds__(NW * 32, 1) sg_cluster_kernel(const __grid_con
     }
     if (rank != 0)
         return;
+    ng_p = __shfl_sync(SG_FULL, ng_p, 0); /* of warp 0; the others leave */
+    if (warp != 0)
+        return;
     /* hard_decision (:393-415) and packing (:272-280) as in sg_decode_kernel */
     const uint16_t* hdw = S.hdw[(phase - 1) & 1];
-    if (tid < SG_INFO_BYTES) {
-        uint32_t byte = 0;
+    uint32_t byte[2];
+#pragma unroll 1
+    for (int h = 0; h < 2; h++) {
+        uint32_t v = 0;
         for (int q = 0; q < 8; q++) {
-            const int b = tid * 8 + q;
+            const int b = (lane + 32 * h) * 8 + q;
             const int p = (b >> 6) * 256 + ((b >> 3) & 7) * 16 + (b & 7);
             const int l = sg_line_of(axis, p), bit = axis == 0 ? p & 15 : (axis == 1 ? (p >> 4) & 15 : p >> 8);
-            byte = (byte << 1) | ((hdw[l] >> bit) & 1u);
+            v = (v << 1) | ((hdw[l] >> bit) & 1u);
         }
-        args.bits[cw * SG_INFO_BYTES + tid] = (uint8_t)byte;
+        (h ? byte[1] : byte[0]) = v;
     }
-    if (tid == 0 && args.stats) {
-        sg_cw_stats st;
-        st.iterations = 0.5 * phase;
-        st.ng = S.ng;
-        st.ng_p = ng_p;
-        st.converged = conv ? 1 : 0;
-        st.phases = phase;
-        args.stats[cw] = st;
-    }
+    sg_cw_stats st;
+    st.iterations = 0.5 * phase;
+    st.ng = S.ng;
+    st.ng_p = ng_p;
+    st.converged = conv ? 1 : 0;
+    st.phases = phase;
+    sg_cw_output(args, cw, byte[0], byte[1], st, lane);
 }

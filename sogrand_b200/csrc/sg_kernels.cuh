@@ -53,6 +53,8 @@ struct SgDecodeArgs {
     const uint32_t* enum_tabs;
     unsigned int* err;
     double* ckpt; /* nullable: [n_cw][3*imax][4096], L_E entering each phase */
+    sg_decode_summary* sum; /* nullable: totals, added to by every codeword */
+    const uint8_t* ref;     /* nullable: info bits to compare with, for sum */
     unsigned long long n_cw;
     long long wait_limit; /* polls or idle rounds before a bounded wait gives up */
     int32_t L;
@@ -80,21 +82,65 @@ __device__ __forceinline__ uint32_t sg_mbar_wait(uint32_t mbar, uint32_t parity,
     return ok;
 }
 
+/* Outputs of a codeword, by one warp: bytes `lane` and `lane + 32` of its info
+ * bits (b0, b1), its statistics, and its share of the totals.  Iterations are
+ * multiples of 0.5, their total below 2^52, so that the atomic double
+ * additions are exact and their order does not matter.  Totals kept here
+ * need neither the per-codeword statistics in memory nor a kernel that reads
+ * them. */
+__device__ __forceinline__ void sg_cw_output(const SgDecodeArgs& args, unsigned long long cw, uint32_t b0, uint32_t b1,
+                                             const sg_cw_stats& st, int lane)
+{
+    if (args.bits) {
+        args.bits[cw * SG_INFO_BYTES + lane] = (uint8_t)b0;
+        args.bits[cw * SG_INFO_BYTES + 32 + lane] = (uint8_t)b1;
+    }
+    if (lane == 0 && args.stats)
+        args.stats[cw] = st;
+    if (args.sum) {
+        uint32_t e = 0;
+        if (args.ref) {
+            const uint8_t* r = args.ref + cw * SG_INFO_BYTES + lane;
+            e = __popc(b0 ^ r[0]) + __popc(b1 ^ r[32]);
+        }
+        e = __reduce_add_sync(SG_FULL, e);
+        if (lane == 0) {
+            typedef unsigned long long u64;
+            sg_decode_summary* s = args.sum;
+            atomicAdd((u64*)&s->blocks, 1ull);
+            uint64_t* what = st.converged == 1 ? &s->converged
+                                               : (st.converged == -1 ? &s->nonfinite
+                                                                     : (st.converged == -2 ? &s->timeouts : nullptr));
+            if (what)
+                atomicAdd((u64*)what, 1ull);
+            atomicAdd((u64*)&s->total_ng, (u64)st.ng);
+            atomicAdd((u64*)&s->total_ng_p, (u64)st.ng_p);
+            atomicAdd(&s->total_iterations, st.iterations);
+            if (args.ref) {
+                atomicAdd((u64*)&s->bits_compared, (u64)SG_INFO_BITS);
+                atomicAdd((u64*)&s->bit_errors, (u64)e);
+                atomicAdd((u64*)&s->block_errors, e ? 1ull : 0ull);
+            }
+            const unsigned int err = *(volatile const unsigned int*)args.err;
+            if (err)
+                atomicOr(&s->device_error, err);
+        }
+    }
+}
+
 /* Outputs of a codeword that is not decoded: zero bits and statistics with
  * the given converged code (-1 non-finite input, -2 a wait gave up).
  * Called by the whole CTA. */
 __device__ __forceinline__ void sg_cw_not_decoded(const SgDecodeArgs& args, unsigned long long cw, int code)
 {
-    if (threadIdx.x < SG_INFO_BYTES)
-        args.bits[cw * SG_INFO_BYTES + threadIdx.x] = 0;
-    if (threadIdx.x == 0 && args.stats) {
+    if (threadIdx.x < 32) {
         sg_cw_stats st;
         st.iterations = 0;
         st.ng = 0;
         st.ng_p = 0;
         st.converged = code;
         st.phases = 0;
-        args.stats[cw] = st;
+        sg_cw_output(args, cw, 0u, 0u, st, (int)threadIdx.x);
     }
 }
 
@@ -332,34 +378,36 @@ __global__ void __launch_bounds__(NW * 32, MINB) sg_decode_kernel(const __grid_c
 
         /* hard_decision (:393-415): info bit b = s*64 + r*8 + c is the sign of
          * L_APP at cube index s*256 + r*16 + c; packed MSB first (:272-280) */
-        if (tid < SG_INFO_BYTES) {
-            uint32_t byte = 0;
-            for (int q = 0; q < 8; q++) {
-                const int b = tid * 8 + q;
-                const int p = (b >> 6) * 256 + ((b >> 3) & 7) * 16 + (b & 7);
-                int l, bit;
-                if (axis_last == 0) {
-                    l = (p >> 8) * 16 + ((p >> 4) & 15);
-                    bit = p & 15;
-                } else if (axis_last == 1) {
-                    l = (p >> 8) * 16 + (p & 15);
-                    bit = (p >> 4) & 15;
-                } else {
-                    l = ((p >> 4) & 15) * 16 + (p & 15);
-                    bit = p >> 8;
+        if (warp == 0) {
+            uint32_t byte[2];
+#pragma unroll 1
+            for (int h = 0; h < 2; h++) {
+                uint32_t v = 0;
+                for (int q = 0; q < 8; q++) {
+                    const int b = (lane + 32 * h) * 8 + q;
+                    const int p = (b >> 6) * 256 + ((b >> 3) & 7) * 16 + (b & 7);
+                    int l, bit;
+                    if (axis_last == 0) {
+                        l = (p >> 8) * 16 + ((p >> 4) & 15);
+                        bit = p & 15;
+                    } else if (axis_last == 1) {
+                        l = (p >> 8) * 16 + (p & 15);
+                        bit = (p >> 4) & 15;
+                    } else {
+                        l = ((p >> 4) & 15) * 16 + (p & 15);
+                        bit = p >> 8;
+                    }
+                    v = (v << 1) | ((S.hdw[l] >> bit) & 1u);
                 }
-                byte = (byte << 1) | ((S.hdw[l] >> bit) & 1u);
+                (h ? byte[1] : byte[0]) = v;
             }
-            args.bits[cw * SG_INFO_BYTES + tid] = (uint8_t)byte;
-        }
-        if (tid == 0 && args.stats) {
             sg_cw_stats st;
             st.iterations = 0.5 * phases;
             st.ng = S.ng;
             st.ng_p = ng_p;
             st.converged = conv ? 1 : 0;
             st.phases = phases;
-            args.stats[cw] = st;
+            sg_cw_output(args, cw, byte[0], byte[1], st, lane);
         }
         __syncthreads();
     }

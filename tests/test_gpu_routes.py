@@ -82,3 +82,34 @@ def test_backward_order(cuda, sg, n, chunk, loss_mode):
             d, ref = d.max(axis=1), np.maximum(1.0, ref.max(axis=1))
         ok = ~np.isnan(d)
         assert ok.sum() >= n - 1 and (d[ok] <= tol * ref[ok]).all()
+
+
+@pytest.mark.parametrize("n", [1, 8, 37, 74, 148, 259, 260, 700])
+@pytest.mark.parametrize("want_bits", [False, True])
+def test_summary_totals(cuda, sg, mode, n, want_bits):
+    """Totals that the decode kernels keep, for every cluster size and the plain form, against those
+    of the per-codeword outputs: whole numbers and multiples of 0.5, equal."""
+    torch = cuda
+    from sogrand_b200 import _lib
+
+    info, llr = sg.gen_llr(500 + n, 0, n, ebn0_range=(0.5, 2.5), device="cuda")
+    if n > 5:
+        llr[4, 100] = float("inf")
+    p = sg.params(Imax=3)
+    bits, raw, _ = sg.decode(llr, p)
+    st = sg.stats_from_device(raw)
+    wrong = np.unpackbits((bits ^ info).cpu().numpy(), axis=1).sum(axis=1)
+    want = dict(blocks=n, converged=(st["converged"] == 1).sum(), nonfinite=(st["converged"] == -1).sum(),
+                total_ng=st["ng"].sum(), total_ng_p=st["ng_p"].sum(), bits_compared=512 * n, bit_errors=wrong.sum(),
+                block_errors=(wrong > 0).sum(), total_iterations=st["iterations"].sum(), timeouts=0, device_error=0)
+    got, b = sg.decode_summary(llr, p, ref_info=info, want_bits=want_bits)
+    assert {k: got[k] for k in want} == want
+    if want_bits:
+        assert torch.equal(b, bits)
+    summ = torch.zeros(sg.SUMMARY_DTYPE.itemsize, dtype=torch.uint8, device="cuda")
+    _lib.check(_lib.load().sg_decode_summary_device_noalloc(
+        llr.data_ptr(), n, C.byref(p), None, b.data_ptr() if want_bits else None, summ.data_ptr(),
+        torch.cuda.current_stream().cuda_stream))
+    rec = np.frombuffer(summ.cpu().numpy().tobytes(), dtype=sg.SUMMARY_DTYPE)[0]
+    want.update(bits_compared=0, bit_errors=0, block_errors=0)
+    assert {k: rec[k].item() for k in want} == want
