@@ -460,12 +460,13 @@ __device__ __forceinline__ SgLineResult sg_decode_line(double llr, const SgLineP
     const uint32_t hdm = __ballot_sync(SG_FULL, !(llr > 0.0)) & 0xffffu;
     /* JacLog(xj) = xj if xj > 50, 0 if xj < -50, else log(1 + e^xj) (:762):
      * lanes 0..15 take -|L| (getPM_HD, :617, :764), lanes 16..31 +|L| (the PM
-     * increments) */
+     * increments).  A NaN, which weights that are 0 or large can make of
+     * finite LLRs, stays one; sg_dec_log_pos takes positive numbers only. */
     const double xj = act ? -a : a;
     double ex = CR ? sg_exp_cr(xj, etab) : sg_exp_mid(xj, etab);
     if (!CR && !(a < 700.0))
         ex = sg_exp(xj, etab);
-    const double jl = xj > 50 ? xj : (xj < -50 ? 0.0 : sg_dec_log_pos<CR>(1.0 + ex, ltab));
+    const double jl = !(xj <= 50) ? xj : (xj < -50 ? 0.0 : sg_dec_log_pos<CR>(1.0 + ex, ltab));
     /* the soft output's exp(LLR) is this exp of lane p + 16 when the LLR is
      * positive, of lane p otherwise (a NaN LLR is its own exp) */
     if (act ? !(llr > 0.0) : (llr > 0.0))
