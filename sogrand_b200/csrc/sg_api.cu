@@ -702,12 +702,16 @@ sg_status sg_bitso_device(const double* d_llr, size_t n_lines, int32_t L, uint64
         return s;
     sg_order_meta meta;
     order_meta(tmax_eff(Tmax), &meta);
-    /* few lines: one per warp, spread over the SMs; more than the warps two
-     * CTAs of 16 keep resident: those, each with an equal share.  Beyond that
-     * line the resident grid fills its tables once: 65 537 lines at 2 dB 294 us,
-     * one per warp in CTAs of their own 342. */
+    /* up to 16 lines per SM: one per warp, in CTAs spread over the SMs; more:
+     * two CTAs of 16 warps on every SM, each with an equal share, which fill
+     * their tables once.  The line is where the two meet.  148 SMs, 1 / 2 / 3
+     * dB, us, one per warp against resident: 2 000 lines 33 / 35 / 39 and 35 /
+     * 35 / 39, 2 368 equal, 4 000 38 / 45 / 51 and 37 / 38 / 42, 4 736 51 / 54
+     * / 59 and 41 / 44 / 48, 65 537 327 / 338 / 354 and 232 / 236 / 242;
+     * correctly rounded, 2 dB: 1 000 39 and 43, 2 368 41 and 43, 3 552 57 and
+     * 46. */
     const unsigned long long full = 2ull * c->sms;
-    const int bv = n_lines > 16 * full ? 1 : 0;
+    const int bv = n_lines > 8 * full ? 1 : 0;
     const SgBVariant& v = k_bvariants[bv];
     unsigned long long n = n_lines, per = bv ? (n + full - 1) / full : (n < full ? 1 : v.nw);
     const uint32_t* tabs = c->enum_tabs;
