@@ -305,9 +305,11 @@ int32_t sg_get_math_mode(void);
  * staged by a bulk asynchronous copy, or global memory through L2), and in
  * lines per warp (one line on 32 lanes, or two lines on 16 lanes each, with 2
  * or 4 error patterns per lane per step: the "-l2-" variants); all give
- * identical results.  The default one hands batches of up to about 1.75
- * codewords per SM, those in flight on other streams included, to a kernel
- * that decodes a codeword on a cluster of CTAs: sooner, for more SM time.
+ * identical results.  A one-line kernel has two names: X decodes every batch
+ * with it, X-g2 (the default among them, as of the batched variants) hands
+ * batches of up to about 1.75 codewords per SM, those in flight on other
+ * streams included, to a kernel that decodes a codeword on a cluster of CTAs:
+ * sooner, for more SM time.
  * sogrand_b200.autotune() measures them.  The selection is kept per math
  * mode: the setters change the current mode's. */
 int sg_decoder_variant_count(void);

@@ -277,8 +277,8 @@ std::atomic<int> g_math_mode{0}; /* 0: table-driven exp/log, 1: correctly rounde
  * ms, p28x3 117.3, p24x3 121.6; w16-gmem 115.3, w8-gmem 134.0, w12-smem
  * 137.0, w8-smem 162.7; correctly rounded, 6 000: p32x3 86.5, p28x3 89.2,
  * p24x3 93.2; w16-gmem 87.7, w8-gmem 93.5. */
-int g_pvariant_by_mode[2] = {SG_PVARIANT_AUTO, SG_PVARIANT_AUTO};
-int g_variant_by_mode[2] = {SG_VARIANT_AUTO, SG_VARIANT_AUTO};
+int g_pvariant_by_mode[2] = {SG_PVARIANT_DEFAULT, SG_PVARIANT_DEFAULT};
+int g_variant_by_mode[2] = {SG_VARIANT_DEFAULT, SG_VARIANT_DEFAULT};
 #define g_pvariant (g_pvariant_by_mode[g_math_mode.load()])
 #define g_variant (g_variant_by_mode[g_math_mode.load()])
 std::vector<uint32_t> g_enum_host;
@@ -503,7 +503,9 @@ cudaError_t launch_decode(const SgDecodeArgs& a, const ClusterInfo& info, Flight
         return cudaLaunchKernel(decode_fn(vi, mode == 1), dim3((unsigned)std::min<unsigned long long>(a.n_cw, 1 << 30)),
                                 dim3(v.nw * 32), kargs, v.smem, st);
     };
-    return vi == SG_VARIANT_AUTO ? launch_small_or(a.n_cw, info, fl, st, launch) : launch(-1);
+    /* as in the batched form, a lowered wait limit keeps a kernel that waits */
+    const bool cl = k_variants[vi].clusters && (!k_variants[vi].lch_smem || a.wait_limit == SG_WAIT_LIMIT_DEFAULT);
+    return cl ? launch_small_or(a.n_cw, info, fl, st, launch) : launch(-1);
 }
 
 sg_status get_ctx(DevCtx** out)
@@ -1170,7 +1172,7 @@ sg_status batch_enqueue(sg_batch b, const double* d_llr, size_t n_cw, const sg_p
     /* a small batch goes to clusters; under a lowered wait limit it keeps the
      * kernel whose waits that limit bounds (clusters only meet at hardware
      * barriers) */
-    if (vi == SG_PVARIANT_AUTO && a.wait_limit == SG_WAIT_LIMIT_DEFAULT)
+    if (k_pvariants[vi].clusters && a.wait_limit == SG_WAIT_LIMIT_DEFAULT)
         SG_CUDA(launch_small_or(n_cw, c->clusters, &c->flights, st, launch));
     else
         SG_CUDA(launch(-1));

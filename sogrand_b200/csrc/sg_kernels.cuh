@@ -488,62 +488,66 @@ __global__ void __launch_bounds__(NW * 32, NW == 16 ? 2 : 1)
  * shared memory (bulk copy) or read from global memory, minimum resident
  * CTAs per SM for the register budget, and lines per warp (1: 32 lanes per
  * line, sg_line.cuh; 2: 16 lanes per line and G patterns per lane,
- * sg_line16.cuh).  The "-g2" names of one-line configurations date from a
- * guess loop with two patterns per lane; they are the same kernels, and
- * w16-gmem-g2 and p32x3-g2, the defaults, hand small batches to the cluster
- * configurations below. */
+ * sg_line16.cuh).  A one-line kernel has two names: X decodes every batch
+ * with it, X-g2 hands small batches to the cluster configurations below. */
 struct SgVariant {
     const char* name;
     int nw;
     bool lch_smem;
+    bool clusters; /* small batches go to clusters */
     size_t smem;
     const void* fn;
 };
 
-#define SG_VARIANT(NW, L, M, NAME) \
-    { NAME, NW, L, sizeof(SgCwSmem<NW, L>), (const void*)sg_decode_kernel<NW, L, M, 1, SG_TU_CR> }
+#define SG_VARIANT(NW, L, M, CL, NAME) \
+    { NAME, NW, L, CL, sizeof(SgCwSmem<NW, L>), (const void*)sg_decode_kernel<NW, L, M, 1, SG_TU_CR> }
 #define SG_VARIANT_L2(NW, M, G, NAME) \
-    { NAME, NW, false, sizeof(SgCwSmem<NW, false, 2>), (const void*)sg_decode_kernel<NW, false, M, G, SG_TU_CR, 2> }
+    { NAME, NW, false, false, sizeof(SgCwSmem<NW, false, 2>), \
+      (const void*)sg_decode_kernel<NW, false, M, G, SG_TU_CR, 2> }
 static const SgVariant k_variants[] = {
-    SG_VARIANT(8, false, 3, "w8-gmem"),
-    SG_VARIANT(8, true, 2, "w8-smem"),
-    SG_VARIANT(12, true, 2, "w12-smem"),
-    SG_VARIANT(16, false, 2, "w16-gmem"),
-    SG_VARIANT(16, false, 2, "w16-gmem-g2"),
-    SG_VARIANT(8, false, 3, "w8-gmem-g2"),
-    SG_VARIANT(12, true, 2, "w12-smem-g2"),
+    SG_VARIANT(8, false, 3, false, "w8-gmem"),
+    SG_VARIANT(8, true, 2, false, "w8-smem"),
+    SG_VARIANT(12, true, 2, false, "w12-smem"),
+    SG_VARIANT(16, false, 2, false, "w16-gmem"),
+    SG_VARIANT(16, false, 2, true, "w16-gmem-g2"),
+    SG_VARIANT(8, false, 3, true, "w8-gmem-g2"),
+    SG_VARIANT(12, true, 2, true, "w12-smem-g2"),
     SG_VARIANT_L2(8, 2, 2, "w8-l2-g2"),
     SG_VARIANT_L2(8, 2, 4, "w8-l2-g4"),
     SG_VARIANT_L2(10, 1, 2, "w10-l2-g2"),
     SG_VARIANT_L2(16, 1, 2, "w16-l2-g2"),
+    SG_VARIANT(8, true, 2, true, "w8-smem-g2"),
 };
 #define SG_NVARIANTS ((int)(sizeof(k_variants) / sizeof(k_variants[0])))
 
-#define SG_VARIANT_AUTO 4 /* w16-gmem-g2 */
+#define SG_VARIANT_DEFAULT 4 /* w16-gmem-g2 */
 
 /* Batched persistent decoder configurations: warps per CTA (one CTA per
- * SM), codeword slots per CTA. */
+ * SM), codeword slots per CTA; names as above. */
 struct SgPVariant {
     const char* name;
     int nw;
     int slots;
+    bool clusters;
     size_t smem;
     const void* fn;
 };
-#define SG_PVARIANT(NW, C, NAME) \
-    { NAME, NW, C, sizeof(SgPersistSmem<NW, C>), (const void*)sg_persist_kernel<NW, C, SG_TU_CR> }
+#define SG_PVARIANT(NW, C, CL, NAME) \
+    { NAME, NW, C, CL, sizeof(SgPersistSmem<NW, C>), (const void*)sg_persist_kernel<NW, C, SG_TU_CR> }
 static const SgPVariant k_pvariants[] = {
-    SG_PVARIANT(24, 3, "p24x3"),
-    SG_PVARIANT(28, 3, "p28x3"),
-    SG_PVARIANT(16, 3, "p16x3"),
-    SG_PVARIANT(20, 4, "p20x4"),
-    SG_PVARIANT(32, 3, "p32x3"),
-    SG_PVARIANT(32, 3, "p32x3-g2"),
-    SG_PVARIANT(24, 3, "p24x3-g2"),
-    SG_PVARIANT(28, 3, "p28x3-g2"),
+    SG_PVARIANT(24, 3, false, "p24x3"),
+    SG_PVARIANT(28, 3, false, "p28x3"),
+    SG_PVARIANT(16, 3, false, "p16x3"),
+    SG_PVARIANT(20, 4, false, "p20x4"),
+    SG_PVARIANT(32, 3, false, "p32x3"),
+    SG_PVARIANT(32, 3, true, "p32x3-g2"),
+    SG_PVARIANT(24, 3, true, "p24x3-g2"),
+    SG_PVARIANT(28, 3, true, "p28x3-g2"),
+    SG_PVARIANT(16, 3, true, "p16x3-g2"),
+    SG_PVARIANT(20, 4, true, "p20x4-g2"),
 };
 #define SG_NPVARIANTS ((int)(sizeof(k_pvariants) / sizeof(k_pvariants[0])))
-#define SG_PVARIANT_AUTO 5 /* p32x3-g2 */
+#define SG_PVARIANT_DEFAULT 5 /* p32x3-g2 */
 
 /* Cluster configurations (sg_cluster.cuh): warps per CTA and CTAs per
  * codeword, the latter descending. */
