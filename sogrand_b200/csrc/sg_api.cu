@@ -167,39 +167,34 @@ __global__ void __launch_bounds__(SG_THREADS, 3) sg_gen_kernel(uint64_t seed, ui
     }
 }
 
-/* 16-byte alignment of the shared tables (double2 loads) and of the bulk
- * copy destination, for every configuration built. */
-template <class T>
-constexpr bool sg_tables_aligned()
+/* A configuration's shared memory: tables on 16-byte boundaries (double2
+ * loads), warp records on 256-byte ones (the guess loop puts table bytes into
+ * the low byte of a record's address), and room for the CTAs per SM that it
+ * is built for (228 KB per SM, 1 KB of it reserved per CTA; 227 KB per CTA). */
+template <class T, int CTAS>
+constexpr bool sg_smem_ok()
 {
-    return offsetof(T, etab) % 16 == 0 && offsetof(T, ltab) % 16 == 0;
+    return offsetof(T, etab) % 16 == 0 && offsetof(T, ltab) % 16 == 0 && offsetof(T, ws) % 256 == 0 &&
+           alignof(T) <= 1024 && sizeof(T) <= 227 * 1024 && CTAS * (sizeof(T) + 1024) <= 228 * 1024;
 }
-static_assert(sg_tables_aligned<SgPersistSmem<24, 3>>() && sg_tables_aligned<SgPersistSmem<28, 3>>() &&
-                  sg_tables_aligned<SgPersistSmem<16, 3>>() && sg_tables_aligned<SgPersistSmem<20, 4>>() && sg_tables_aligned<SgPersistSmem<32, 3>>() &&
-                  sg_tables_aligned<SgCwSmem<8, false>>() && sg_tables_aligned<SgCwSmem<8, true>>() &&
-                  sg_tables_aligned<SgCwSmem<12, true>>() && sg_tables_aligned<SgCwSmem<16, false>>() &&
-                  sg_tables_aligned<SgCwSmem<8, false, 2>>() && sg_tables_aligned<SgCwSmem<10, false, 2>>() &&
-                  sg_tables_aligned<SgCwSmem<16, false, 2>>() && sg_tables_aligned<SgLineSmem<4, false>>() &&
-                  sg_tables_aligned<SgLineSmem<16, true>>(),
-              "shared table alignment");
+static_assert(sg_smem_ok<SgPersistSmem<16, 3>, 1>() && sg_smem_ok<SgPersistSmem<20, 4>, 1>() &&
+                  sg_smem_ok<SgPersistSmem<24, 3>, 1>() && sg_smem_ok<SgPersistSmem<28, 3>, 1>() &&
+                  sg_smem_ok<SgPersistSmem<32, 3>, 1>(),
+              "batched configurations");
+static_assert(sg_smem_ok<SgCwSmem<8, false>, 3>() && sg_smem_ok<SgCwSmem<8, true>, 2>() &&
+                  sg_smem_ok<SgCwSmem<12, true>, 2>() && sg_smem_ok<SgCwSmem<16, false>, 2>() &&
+                  sg_smem_ok<SgCwSmem<8, false, 2>, 2>() && sg_smem_ok<SgCwSmem<10, false, 2>, 1>() &&
+                  sg_smem_ok<SgCwSmem<16, false, 2>, 1>(),
+              "plain configurations");
+static_assert(sg_smem_ok<SgClusterSmem<16>, 1>() && sg_smem_ok<SgClusterSmem<32>, 1>(), "cluster configurations");
+static_assert(sg_smem_ok<SgLineSmem<4, false>, 1>() && sg_smem_ok<SgLineSmem<16, true>, 2>(), "line kernels");
+static_assert(sg_smem_ok<SgBackSmem, 1>(), "backward kernel");
 template <class T>
 constexpr bool sg_bulk_aligned()
 {
     return offsetof(T, lch) == 0 && offsetof(T, mbar) % 8 == 0;
 }
 static_assert(sg_bulk_aligned<SgCwSmem<8, true>>() && sg_bulk_aligned<SgCwSmem<12, true>>(), "bulk copy");
-/* every configuration fits the 227 KB of shared memory a CTA may have */
-static_assert(sizeof(SgPersistSmem<32, 3>) <= 227 * 1024 && sizeof(SgPersistSmem<28, 3>) <= 227 * 1024 &&
-                  sizeof(SgPersistSmem<24, 3>) <= 227 * 1024 && sizeof(SgPersistSmem<20, 4>) <= 227 * 1024 &&
-                  sizeof(SgPersistSmem<16, 3>) <= 227 * 1024 && sizeof(SgCwSmem<8, true>) <= 227 * 1024 &&
-                  sizeof(SgCwSmem<16, false>) <= 227 * 1024 && sizeof(SgCwSmem<12, true>) <= 227 * 1024 &&
-                  sizeof(SgCwSmem<16, false, 2>) <= 227 * 1024,
-              "shared memory per CTA");
-/* the configurations built for two CTAs per SM fit them (228 KB per SM, 1 KB
- * of it reserved per CTA) */
-static_assert(2 * (sizeof(SgCwSmem<8, false, 2>) + 1024) <= 228 * 1024 &&
-                  2 * (sizeof(SgCwSmem<16, false>) + 1024) <= 228 * 1024,
-              "two CTAs per SM");
 
 /* Static device memory of the allocation-free entry point: the error flag
  * (word 0; while the tables are built, each one's completion flag) and a

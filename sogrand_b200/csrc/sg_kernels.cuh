@@ -151,7 +151,9 @@ template <int NW, bool LCH_SMEM, int LPW = 1> /* LPW: lines decoded per warp at 
 struct SgCwSmem {
     alignas(16) double lch[LCH_SMEM ? SG_CUBE : 2]; /* bulk-copy destination */
     double le[SG_CUBE];
-    /* eight copies where the configuration's CTAs per SM still fit */
+    /* eight copies where the CTAs per SM that this costs are outweighed:
+     * w10-l2-g2 falls from two CTAs to one, and 12 000 codewords at 2 dB from
+     * 507 to 406 ms */
     static constexpr bool T8 = NW * LPW >= 16 && !LCH_SMEM;
     SgEtab<T8> etab;
     alignas(16) double ltab[SG_LOG_TAB_LEN];
