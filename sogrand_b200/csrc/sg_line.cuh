@@ -337,21 +337,21 @@ __device__ __forceinline__ bool sg_list_hit(SgWarpScratch* ws, const SgLineParam
  * P - e does by adding it to 2^E (s1) and to 2^E + u (s2).  The two start
  * with different parity, so an exact tie (a term whose units end in 1/2,
  * rounded to even) leaves them something else than one unit apart.
- * SgGrid: the two addends of P's binade.  A P below 2^-970, not positive or
- * not finite has no such grid: NaNs, whose sums never differ by one unit and
- * whose high word no P exceeds, send every step to the replay. */
+ * SgGrid: the two addends of P's binade.  A P below 2^-970 or not positive
+ * has no such grid: NaNs, whose sums never differ by one unit and whose high
+ * word no P exceeds, send every step to the replay.  (A NaN P stays one in
+ * either.) */
 struct SgGrid {
     double b1, b2;
 };
 
 __device__ __forceinline__ SgGrid sg_grid(uint64_t Pb)
 {
-    const uint32_t ph = (uint32_t)(Pb >> 32);
-    const bool grid = ph - 0x03500000u < 0x7ff00000u - 0x03500000u;
-    const int32_t hi = grid ? (int32_t)(ph & 0xfff00000u) : 0x7fffffff;
+    const int32_t ph = (int32_t)(Pb >> 32);
+    const int32_t hi = ph >= 0x03500000 ? (int32_t)(ph & 0xfff00000) : 0x7fffffff;
     SgGrid g;
     g.b1 = __hiloint2double(hi, 0);
-    g.b2 = __hiloint2double(hi, grid ? 1 : 0);
+    g.b2 = __hiloint2double(hi, ph >= 0x03500000 ? 1 : 0);
     return g;
 }
 
