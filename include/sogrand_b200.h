@@ -172,8 +172,8 @@ typedef struct {
 /* Decode and reduce on the device: bits (nullable: not returned) and one
  * sg_decode_summary at d_summary (device memory, overwritten).  d_ref_info
  * (nullable): the transmitted info bits, 64 packed bytes per codeword, for
- * the bit and block error counts.  The decode adds each codeword to the
- * totals as it finishes. */
+ * the bit and block error counts.  d_ref_info and d_bits must be 16-byte
+ * aligned.  The decode adds each codeword to the totals as it finishes. */
 sg_status sg_decode_summary_device(const double* d_llr, size_t n_cw, const sg_params* p,
                                    const uint8_t* d_ref_info, uint8_t* d_bits,
                                    sg_decode_summary* d_summary, void* stream);
@@ -191,7 +191,8 @@ sg_status sg_decode_summary_device(const double* d_llr, size_t n_cw, const sg_pa
  *     the device by a kernel during the first call on each device.
  * That first call also resolves the device addresses of these arrays and
  * sets up the device; make it before any stream capture.  n_cw above
- * SG_NOALLOC_MAX_CW is rejected with SG_ERR_ARG.  All calls share the one
+ * SG_NOALLOC_MAX_CW is rejected with SG_ERR_ARG (a limit of this entry
+ * point's contract; nothing in it grows with n_cw).  All calls share the one
  * error flag: calls that overlap on the GPU (other streams, other host
  * threads) race and must be serialised by the caller.  Results equal those
  * of sg_decode_summary_device.  This entry point has no counterpart in the
@@ -228,7 +229,7 @@ sg_status sg_encode_host(const uint8_t* info, size_t n_cw, uint8_t* code_bits);
  * sigma <= 0 draws each codeword's Eb/N0 uniformly from
  * [ebn0_lo_db, ebn0_hi_db] with the decoder's own exp.  The device form
  * writes the same values on the device (asynchronously on `stream`); its
- * llr must be 8-byte aligned (16-byte aligned output is stored faster). */
+ * llr must be 8-byte aligned. */
 sg_status sg_gen_llr_host(uint64_t seed, uint64_t cw0, size_t n_cw, double sigma,
                           double ebn0_lo_db, double ebn0_hi_db, uint8_t* info, double* llr);
 sg_status sg_gen_llr_device(uint64_t seed, uint64_t cw0, size_t n_cw, double sigma,
@@ -317,13 +318,18 @@ const char* sg_decoder_variant_name(int v);
 sg_status sg_decoder_set_variant(int v);
 int sg_decoder_get_variant(void);
 
-/* ---- device-side waits.  Every wait in the library's kernels is bounded.
+/* ---- device-side waits.  Every polling wait in the library's kernels is
+ * bounded; the CTAs of a codeword on a cluster meet at hardware barriers, one
+ * per phase, which every warp reaches.
  * A bulk-copy wait that gives up marks its CTA's remaining codewords
  * converged = -2 and sets the device's error flag; a persistent-decoder warp
  * that finds no work for too long exits and sets its batch's flag
  * (sg_batch_check; the other warps finish the batch).  The limit applies to
  * launches made after the call, process-wide: polls of a bulk-copy wait,
- * idle rounds of a persistent warp.  The default, and the largest value
+ * idle rounds (about a microsecond each) of a persistent warp.  Below the
+ * default, small batches of the batched form, and of plain variants that
+ * stage the cube by a bulk copy, are not handed to clusters, so that the
+ * limit's waits are the ones that run.  The default, and the largest value
  * accepted (larger values are clamped), is 2^22.  A limit of 0 makes every
  * wait that is not already complete give up; it exists so that tests can
  * exercise the error paths without a faulty GPU. */

@@ -170,14 +170,14 @@ __device__ __forceinline__ unsigned long long sg_back_pick(const SgBackwardArgs&
  * codeword of its own, hide the end of each other's phases but take twice as
  * long over the longest codeword: 4 % more for 1 024 codewords at 1.5 dB, Imax
  * 10, and 11.5 against 7.3 ms for 160.
- * Bound by issue slots (71 % used) and latency.  A guess costs nine predicated
- * additions and two shared-memory sums besides the forward's work: with all 16
- * positions' sums in registers 27.5 ms and spills, with the high ones' in
- * shared memory, of which the forward's work leaves half idle, 25.7 ms.  Per
- * line, whatever the decode has worked out is used again, sums over a phase
- * are kept per lane, and no logarithm is taken where the loss does not need
- * L_APP (42.3 -> 33 ms); the exp table in eight copies, as in the decoders
- * (44.9 -> 42.3). */
+ * Bound by issue slots (71 % used) and latency; 25.9 ms for those 1 024.  A
+ * guess costs nine predicated additions and two shared-memory sums besides the
+ * forward's work: with all 16 positions' sums in registers there are spills
+ * and 7 % more, since the forward's work leaves half of the shared-memory
+ * cycles idle.  Per line, whatever the decode has worked out is used again,
+ * sums over a phase are kept per lane, and no logarithm is taken where the
+ * loss does not need L_APP (a fifth less in all); the exp table in eight
+ * copies, as in the decoders, takes 6 %. */
 __global__ void __launch_bounds__(SG_BACK_WARPS * 32, 1) sg_backward_kernel(const __grid_constant__ SgBackwardArgs args)
 {
     constexpr int NT = SG_BACK_WARPS * 32;

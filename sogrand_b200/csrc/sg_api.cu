@@ -71,7 +71,7 @@ __device__ __forceinline__ double sg_sym_unit_bits(uint64_t r)
  * its first accepted attempt (after SG_POLAR_TRIES rejections, 0), as
  * sg_normal does.  Bound by issue slots: one attempt is two 64-bit hashes;
  * keyed per attempt once per CTA, not per sample, and with unit and quotient
- * from bits and remainders, 20 000 codewords take 0.88 ms (1.37 ms with one
+ * from bits and remainders, 20 000 codewords take 0.86 ms (1.36 ms with one
  * pass, four hashes per attempt and three library divisions per sample). */
 __global__ void __launch_bounds__(SG_THREADS, 3) sg_gen_kernel(uint64_t seed, uint64_t cw0, unsigned long long n_cw,
                                                                double sigma, double lo, double hi, uint8_t* info,
@@ -435,8 +435,8 @@ cudaError_t cluster_setup(int dev, ClusterInfo* info)
     return e;
 }
 
-/* The cluster configuration for a batch of n codewords, -1 when it is large
- * enough for one CTA per codeword: the most CTAs per codeword with which all
+/* The cluster configuration when n codewords share the device, -1 when they
+ * are enough for one CTA per codeword: the most CTAs per codeword with which all
  * clusters run at the same time; with two, also up to 7/4 codewords per SM.
  * B200, one call at 2 dB, when the rule was set: n = 1 plain 2.29 ms, 16 CTAs
  * 0.43, 8 CTAs 0.52; n = 9: 8 CTAs 0.58, 16 (the ninth cluster waits) 0.66;

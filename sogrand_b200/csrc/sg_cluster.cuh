@@ -18,8 +18,9 @@
  * phases are those of sg_decode_kernel, and so are the outputs, bit for bit.
  *
  * Bound by the latency of a line decode and of the phase ends (issue slots
- * 64 % used with 70 codewords on pairs).  2 dB: one codeword 2.33 -> 0.39 ms
- * (16 CTAs), 100 codewords 3.38 -> 1.95 ms (2 CTAs each).
+ * 64 % used with 70 codewords on pairs).  2 dB, one CTA per codeword against
+ * clusters: one codeword 2.4 and 0.31 to 0.45 ms (16 CTAs, by its noise), 100
+ * codewords 3.2 and 2.0 ms (2 CTAs each).
  */
 #pragma once
 

@@ -33,20 +33,15 @@
  *           running P_notGuess at each, so T and the list match exactly.
  *  output   soft output of :536-577 on lanes 0..15.
  *
- * What bounds it: issue slots (81 % used) and shared-memory cycles (75 %), of
- * 23 steps per line decode at 2 dB, 15 end in the sum, 2 hold codewords, 6
- * are replayed.  Per line decode at 2 dB, B200 counters: 4 740 warp
- * instructions and 1 280 shared-memory cycles with the former loop of two
- * patterns per lane (steps of 64, of which half had to be replayed, term
- * rounding tested by difference, an exp from one table copy); 3 510 and 810
- * now.  20 000 codewords at 2 dB, batched form: 245.8 ms, 202.1 with this
- * loop, 193.0 with the shorter set-up and soft output, 186.2 with the exp
- * constants in constant memory; 8 000, plain form: 101.2 -> 78.1 ms; 2 000 at
- * 1 dB under Tmax 1000: 146 -> 91 ms; correctly rounded math, 4 000 at 2 dB:
- * 68.3 -> 58.4 ms.
- * Steps of 64 patterns were slower once the sum was cheap (229 against 202
- * ms): a step twice as long is summed half as often, and has to be looked at
- * again by halves.
+ * What bounds it: issue slots (81 % used) and shared-memory cycles (75 %).
+ * Per line decode at 2 dB 3 510 warp instructions and 810 shared-memory
+ * cycles; of its 23 steps 15 end in the sum, 2 hold codewords, 6 are
+ * replayed.  Why 32 patterns a step and not 64, two per lane: the longer step
+ * is summed half as often but has to be looked at again by halves, and half
+ * of such steps are replayed (4 740 instructions, 1 280 cycles; 20 000
+ * codewords at 2 dB, batched form, 229 against 202 ms).  The shorter set-up
+ * and soft output take that to 193, exp constants read from constant memory
+ * to 186 ms; with correctly rounded math 60 ms for 4 096.
  * The file is built with -fmad=false: every floating-point operation the
  * reference performs is a separately rounded IEEE operation here.
  */
