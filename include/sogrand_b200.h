@@ -308,9 +308,9 @@ int32_t sg_get_math_mode(void);
  * or 4 error patterns per lane per step: the "-l2-" variants); all give
  * identical results.  A one-line kernel has two names: X decodes every batch
  * with it, X-g2 (the default among them, as of the batched variants) hands
- * batches of up to about 1.75 codewords per SM, those in flight on other
- * streams included, to a kernel that decodes a codeword on a cluster of CTAs:
- * sooner, for more SM time.
+ * batches of up to about 1.75 codewords per SM to a kernel that decodes a
+ * codeword on a cluster of CTAs: sooner, for more SM time, so the clusters
+ * are the smaller the more codewords are in flight on other streams.
  * sogrand_b200.autotune() measures them.  The selection is kept per math
  * mode: the setters change the current mode's. */
 int sg_decoder_variant_count(void);

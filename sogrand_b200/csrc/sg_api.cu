@@ -318,8 +318,8 @@ struct ClusterInfo {
  * after its latest decode; earlier ones on that stream run before it, not
  * beside it.  At most MAX events, kept for later calls; streams beyond them
  * are not counted.  A wrong count costs time, never results.  2 dB, 4
- * codewords per call: 64 streams 13.0 -> 3.5 ms, one CTA per codeword 5.8; 16
- * streams 3.2 -> 1.3; 20 per call, 64 streams 23.1 -> 12.7; one stream pays
+ * codewords per call: 64 streams 13.0 -> 3.7 ms, one CTA per codeword 5.8; 16
+ * streams 3.2 -> 1.3; 20 per call, 64 streams 23.1 -> 15.9; one stream pays
  * 1 us of host time. */
 class Flights {
     static constexpr int MAX = 128, LOOK = 8;
@@ -435,20 +435,31 @@ cudaError_t cluster_setup(int dev, ClusterInfo* info)
     return e;
 }
 
-/* The cluster configuration when n codewords share the device, -1 when they
- * are enough for one CTA per codeword: the most CTAs per codeword with which all
+/* The cluster configuration for a batch of n codewords, -1 when it is large
+ * enough for one CTA per codeword: the most CTAs per codeword with which all
  * clusters run at the same time; with two, also up to 7/4 codewords per SM.
  * B200, one call at 2 dB, when the rule was set: n = 1 plain 2.29 ms, 16 CTAs
  * 0.43, 8 CTAs 0.52; n = 9: 8 CTAs 0.58, 16 (the ninth cluster waits) 0.66;
  * n = 18: 4 CTAs 1.02, 8 1.18; n = 33: 4 CTAs 1.02, 2 1.57; n = 37 (one too
  * many): 4 CTAs 1.66, 2 1.74; n = 100: 2 CTAs 2.00, plain 3.81; n = 220: 3.92,
- * 4.46; n = 296: 4.35, 4.63 but 4.51 in the batched form; n = 600: 8.7, 8.5. */
-int cluster_for(unsigned long long n, const ClusterInfo& info)
+ * 4.46; n = 296: 4.35, 4.63 but 4.51 in the batched form; n = 600: 8.7, 8.5.
+ * With `others` in flight on other streams, at most three times the clusters
+ * that run at the same time: their codewords end at different times and let
+ * waiting clusters in, until the SM time that large clusters cost decides.
+ * 2 dB, several streams of n codewords, ms a round, as if alone / at most
+ * once / twice / three times: 16 of 1 0.83 / 0.69 / 0.67 / 0.84; 64 of 4 13.0
+ * / 3.5 / 3.7 / 3.8; 1 dB, 4 of 3 2.7 / 3.5 / 2.7 / 2.7; 6 of 3 3.2 / - / 3.5
+ * / 3.2: only with three is nothing slower than as if alone.  Two CTAs per
+ * codeword cost a tenth more SM time than one, so these take any number. */
+int cluster_for(unsigned long long n, unsigned long long others, const ClusterInfo& info)
 {
-    for (int v = 0; v < SG_NCVARIANTS; v++)
-        if (n <= (unsigned long long)info.fit[v])
+    constexpr int last = SG_NCVARIANTS - 1;
+    for (int v = 0; v < SG_NCVARIANTS; v++) {
+        const unsigned long long fit = (unsigned long long)info.fit[v];
+        if (n <= fit && (v == last || n + others <= 3 * fit))
             return v;
-    return info.fit[SG_NCVARIANTS - 1] > 0 && 4 * n <= 7ull * info.sms ? SG_NCVARIANTS - 1 : -1;
+    }
+    return info.fit[last] > 0 && 4 * n <= 7ull * info.sms ? last : -1;
 }
 
 cudaError_t launch_cluster(const SgDecodeArgs& a, int v, int mode, cudaStream_t st)
@@ -470,11 +481,11 @@ cudaError_t launch_small_or(unsigned long long n, const ClusterInfo& info, Fligh
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     if (!fl || cudaStreamIsCapturing(st, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone ||
         cudaStreamGetId(st, &id) != cudaSuccess)
-        return launch(cluster_for(n, info));
+        return launch(cluster_for(n, 0, info));
     /* event calls are legal here whatever other streams are capturing */
     cudaStreamCaptureMode was = cudaStreamCaptureModeRelaxed;
     cudaThreadExchangeStreamCaptureMode(&was);
-    const int v = cluster_for(n, info) >= 0 ? cluster_for(n + fl->others(id), info) : -1;
+    const int v = cluster_for(n, 0, info) >= 0 ? cluster_for(n, fl->others(id), info) : -1;
     cudaThreadExchangeStreamCaptureMode(&was);
     const cudaError_t e = launch(v);
     if (e == cudaSuccess) {
